@@ -1,6 +1,6 @@
 """In-tree build of the CUDA library glia_gb300/_build/libglia_rd.so (sm_103a only).
 
-The three translation units compile in parallel with nvcc and link against cuFFT. Nothing is
+The translation units compile in parallel with nvcc and link against cuFFT. Nothing is
 installed outside the repository.
 """
 from __future__ import annotations
@@ -15,9 +15,11 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT_DIR, "libglia_rd.so")
-UNITS = ["capi.cu", "engine_f32.cu", "engine_f64.cu", "noalloc.cu"]
+UNITS = ["capi.cu", "engine_f32.cu", "engine_f64.cu", "noalloc.cu", "plane_f32.cu",
+         "plane_f64.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall"]
+FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
+         "-Xcompiler", "-Wno-unknown-pragmas"]
 
 
 def nvcc() -> str:

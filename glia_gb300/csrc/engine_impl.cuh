@@ -26,6 +26,8 @@
 #include "zpass2.cuh"
 #include "zpass.cuh"
 #include "ownfft.cuh"
+#include "fx.cuh"
+#include "plane.hpp"
 
 #define GLIA_TIMED(slot, bytes, ...)             \
   do {                                           \
@@ -321,24 +323,108 @@ class Engine final : public EngineBase {
   // which: 0 state, 1 adjoint, 2 other (set-up, recomputation) for the iteration counters.
   // The fused engine does not wait for the solve: its outcome is folded into device counters
   // that sync_sweep() reads once per sweep.
-  void solve(R* c, double dts, R* chat_slot, const R* cx, double kdot_w, int which = 2) {
+  // pre: a reaction step taken on c first (fused engine with a plane kernel only).
+  struct Pre {
+    int mode = 0;  // PlaneArgs::pre
+    const R* lin = nullptr;
+    R* half = nullptr;
+  };
+  void solve(R* c, double dts, R* chat_slot, const R* cx, double kdot_w, int which = 2,
+             Pre pre = {}) {
     ctx_dt_ = dts;
     if (pc_dt_mode_ == GLIA_PC_DT_MATCHED) prec_factor_dt(2.0 * dts);
     st_.total_diffusion_solves++;
     if (k_scale_ == 0) {
       ksp_itr_ = 0;
-      if (chat_slot) r2c(r2c1_, c, chat_slot);
+      if (chat_slot) spectrum(c, chat_slot);
       return;
     }
     if (ref_) {
       ref_solve(c, dts);
       if (which < 2) (which == 0 ? st_.diff_ksp_itr_state : st_.diff_ksp_itr_adj) += ksp_itr_;
     } else {
-      fused_solve(c, dts, chat_slot ? chat_slot : chat_, cx, kdot_w, which);
+      fused_solve(c, dts, chat_slot ? chat_slot : chat_, cx, kdot_w, which, pre);
     }
   }
 
-  void fused_solve(R* c, double dts, R* chat, const R* cx, double kdot_w, int which) {
+  // Arguments and launch of the grid's plane kernel (plane.cuh), all CTAs resident at once.
+  PlaneArgs<R> plane_args(int prog, const R* in, R* out, R* chat) {
+    using C = typename CT<R>::C;
+    PlaneArgs<R> a{};
+    a.prog = prog;
+    a.in = in;
+    a.out = out;
+    a.k = kxx_;
+    a.chat = reinterpret_cast<C*>(chat);
+    a.xhat = reinterpret_cast<C*>(xhat_);
+    a.rhat = reinterpret_cast<C*>(rhat_);
+    a.phat = reinterpret_cast<C*>(phat_);
+    a.G = reinterpret_cast<C*>(g3r_);
+    a.M = reinterpret_cast<C*>(g3s_);
+    a.W = reinterpret_cast<C*>(plane_w_);
+    a.sc = sc_;
+    a.part = plane_part_;
+    a.bar = plane_bar_;
+    a.tw = plane_tw_;
+    a.pf = plane_pf_;
+    return a;
+  }
+  void plane_launch(PlaneArgs<R>& a, double bytes) {
+    void* args[] = {&a};
+    const int grid = std::min({plane_.items, plane_res_, red_blocks_});
+    GLIA_TIMED(KS_PLANE, bytes,
+               GLIA_CUDA(cudaLaunchCooperativeKernel(plane_.fn, dim3(grid), dim3(plane_.threads),
+                                                     args, plane_.smem, stream_)));
+  }
+  bool plane() const { return plane_.fn != nullptr; }
+  // Whether the plane kernel also takes a solve's two ends (real field <-> spectrum): in FP64. The
+  // mixed engine keeps cuFFT there: each FP32 round trip c -> spectrum -> c loses a little of the
+  // field (2.2e-7 of a smooth one at 64^3 with cuFFT, 0.7e-7 with the plane kernel), the same way
+  // every time, and hundreds of solves add up to 1e-5 and more, so the ends decide which answer
+  // within the path's accuracy a simulation gives. Users' answers stay where they were.
+  bool plane_ends() const { return std::is_same<R, double>::value; }
+  // spectrum of a real field
+  void spectrum(const R* in, R* out) {
+    if (!plane() || !plane_ends()) {
+      r2c(r2c1_, in, out);
+      return;
+    }
+    PlaneArgs<R> a = plane_args(PP_SPEC, in, nullptr, out);
+    plane_launch(a, FB() + SB());
+    st_.total_fft_execs += 1;
+  }
+
+  void fused_solve(R* c, double dts, R* chat, const R* cx, double kdot_w, int which, Pre pre) {
+    if (plane()) {
+      if (!plane_ends()) r2c(r2c1_, c, chat);
+      PlaneArgs<R> a = plane_args(plane_ends() ? PP_SOLVE : PP_SOLVE_SPEC, c, c, chat);
+      a.which = which;
+      a.pre = pre.mode;
+      a.rho = rho_;
+      a.lin = pre.lin;
+      a.half = pre.half;
+      a.dt = (R)dt_;
+      a.cx = reinterpret_cast<const typename CT<R>::C*>(cx);
+      a.a_cn = 0.5 * dts;
+      a.pc_c = 0.25 * pc_dt_ * pc_kbar_;
+      if (plane_pf_ && plane_pc_ != a.pc_c) {
+        k_pc_field<R><<<pw_blocks_, kThreads, 0, stream_>>>(g_, plane_pf_, a.pc_c);
+        GLIA_LAUNCH_CHECK();
+        plane_pc_ = a.pc_c;
+      }
+      a.rtol = rtol_;
+      a.abstol = abstol_;
+      a.divtol = divtol_;
+      a.maxit = maxit_;
+      a.kdot_weight = kdot_w;
+      plane_launch(a, 3 * FB());  // c in and out, k
+      graph_solves_ = true;
+      if (plane_ends())
+        st_.total_fft_execs += 2;
+      else
+        c2r(c2r1_, xhat_, c);
+      return;
+    }
     k_solve_config<<<1, 1, 0, stream_>>>(sc_, 0.5 * dts, 0.25 * pc_dt_ * pc_kbar_, rtol_, abstol_,
                                          divtol_, maxit_, kdot_w);
     GLIA_LAUNCH_CHECK();
@@ -727,8 +813,9 @@ class Engine final : public EngineBase {
   // a kernel's bounded wait ran out (its CTA stopped early): the results are invalid
   [[noreturn]] void raise_device_fault() {
     GLIA_CUDA(cudaMemsetAsync(&sc_->dev_fault, 0, sizeof(int), stream_));
+    if (plane_bar_) GLIA_CUDA(cudaMemsetAsync(plane_bar_, 0, 2 * sizeof(unsigned), stream_));
     GLIA_CUDA(cudaStreamSynchronize(stream_));
-    throw Error(GLIA_ERR_CUDA, "a device-side copy did not complete within its time limit");
+    throw Error(GLIA_ERR_CUDA, "a device-side wait did not complete within its time limit");
   }
   void check_device_fault() {
     if (ref_) return;
@@ -915,6 +1002,12 @@ class Engine final : public EngineBase {
       ref_applyD(dc, c);
       return;
     }
+    if (plane()) {
+      PlaneArgs<R> a = plane_args(PP_APPLY, c, dc, chat_);
+      plane_launch(a, 3 * FB());
+      st_.total_fft_execs += 2;
+      return;
+    }
     r2c(r2c1_, c, chat_);
     d_front<false>(chat_, nullptr);
     d_back<EPI_APPLYD>(nullptr, nullptr, xhat_, nullptr, (R)g_.invN);
@@ -983,6 +1076,13 @@ class Engine final : public EngineBase {
       return;
     }
     const R* K = smoother_kernel(sigma);
+    if (plane()) {
+      PlaneArgs<R> a = plane_args(PP_SMOOTH, in, out, chat_);
+      a.mulk = reinterpret_cast<const typename CT<R>::C*>(K);
+      plane_launch(a, 2 * FB() + SB());
+      st_.total_fft_execs += 2;
+      return;
+    }
     r2c(r2c1_, in, chat_);
     k_spec_mul<R><<<pw_blocks_, kThreads, 0, stream_>>>(Ns_, 1, chat_, K);
     GLIA_LAUNCH_CHECK();
@@ -1433,12 +1533,23 @@ class Engine final : public EngineBase {
   void step(R* c, R* chat_slot, R* half_out, int which = 0) {
     if (order_ == 2) {
       solve(c, dt_ / 2.0, chat_slot, nullptr, 0.0, which);
-      reaction(c, half_out);
-      solve(c, dt_ / 2.0, nullptr, nullptr, 0.0, which);
+      const Pre pre = react(c, 1, nullptr, half_out);
+      solve(c, dt_ / 2.0, nullptr, nullptr, 0.0, which, pre);
     } else {
       solve(c, dt_, chat_slot, nullptr, 0.0, which);
       reaction(c, half_out);
     }
+  }
+  // The reaction step between two diffusion half steps (mode 1: logistic, storing the field in
+  // half; 2: linearised at lin): a plane kernel takes it as it reads the field of the next solve,
+  // otherwise it runs here.
+  Pre react(R* c, int mode, const R* lin, R* half) {
+    if (plane() && plane_ends() && k_scale_ != 0) return Pre{mode, lin, half};
+    if (mode == 1)
+      reaction(c, half);
+    else
+      reaction_linearized(c, lin);
+    return Pre{};
   }
   void reaction(R* c, R* half_out) {
     GLIA_TIMED(KS_REACTION, FB() * (half_out ? 4 : 3),
@@ -1467,7 +1578,7 @@ class Engine final : public EngineBase {
         step(ct_, (!ref_ && trick) ? chat_hist_[i] : nullptr, half);
         vcopy(c_hist_[i + 1], ct_);
       }
-      if (!ref_ && trick) r2c(r2c1_, ct_, chat_hist_[nt_]);
+      if (!ref_ && trick) spectrum(ct_, chat_hist_[nt_]);
     } else {
       // the last segment is written straight into the segment buffers, so the backward sweep
       // starts without recomputing it
@@ -1482,7 +1593,7 @@ class Engine final : public EngineBase {
         }
       }
       vcopy(seg_c_[nt_ - last0], ct_);
-      if (trick) r2c(r2c1_, ct_, seg_chat_[nt_ - last0]);
+      if (trick) spectrum(ct_, seg_chat_[nt_ - last0]);
       last_seg_resident_ = true;
       vcopy(cfin(), ct_);  // c_[nt] for the Hessian's kappa rows
     }
@@ -1529,8 +1640,8 @@ class Engine final : public EngineBase {
       if (mode == 2) source(ci, cj, 1);
       if (order_ == 2) {
         solve(ct_, dt_ / 2.0, nullptr, nullptr, 0.0, 0);
-        reaction_linearized(ct_, ci);
-        solve(ct_, dt_ / 2.0, nullptr, nullptr, 0.0, 0);
+        const Pre pre = react(ct_, 2, ci, nullptr);
+        solve(ct_, dt_ / 2.0, nullptr, nullptr, 0.0, 0, pre);
         if (mode == 2) source(ci, cj, 2);
       } else {
         solve(ct_, dt_, nullptr, nullptr, 0.0, 0);
@@ -1572,18 +1683,14 @@ class Engine final : public EngineBase {
     const R* cxx = accumulate ? cx : nullptr;
     if (order_ == 2) {
       solve(p0_, dt_ / 2.0, nullptr, cxx, w * dt_, 1);
-      reaction_adjoint(chalf);
-      solve(p0_, dt_ / 2.0, nullptr, nullptr, 0.0, 1);
+      const Pre pre = react(p0_, 2, chalf, nullptr);
+      solve(p0_, dt_ / 2.0, nullptr, nullptr, 0.0, 1, pre);
     } else {
       solve(p0_, dt_, nullptr, cxx, w * dt_, 1);
       reaction_adjoint(chalf);
     }
   }
-  void reaction_adjoint(const R* chalf) {
-    GLIA_TIMED(KS_REACTION_LIN, FB() * 4,
-               k_reaction_lin<R><<<pw_blocks_, kThreads, 0, stream_>>>(N_, p0_, rho_, chalf,
-                                                                        (R)dt_));
-  }
+  void reaction_adjoint(const R* chalf) { reaction_linearized(p0_, chalf); }
   // reactionAdjoint without stored half steps (src/pde/PdeOperators.cpp:331-344)
   const R* recompute_half(const R* ci) {
     vcopy(tmp_, ci);
@@ -1650,8 +1757,8 @@ class Engine final : public EngineBase {
           solve(p0_, dt_ / 2.0, nullptr, kdot ? chat_hist_[i + 1] : nullptr,
                 ((i + 1 == nt_) ? 0.5 : 1.0) * dt_, 1);
           if (!chalf) chalf = recompute_half(c_hist_[i]);
-          reaction_adjoint(chalf);
-          solve(p0_, dt_ / 2.0, nullptr, nullptr, 0.0, 1);
+          const Pre pre = react(p0_, 2, chalf, nullptr);
+          solve(p0_, dt_ / 2.0, nullptr, nullptr, 0.0, 1, pre);
         } else {
           solve(p0_, dt_, nullptr, kdot ? chat_hist_[i + 1] : nullptr,
                 ((i + 1 == nt_) ? 0.5 : 1.0) * dt_, 1);
@@ -1677,7 +1784,7 @@ class Engine final : public EngineBase {
             step(tmp2(), trick ? seg_chat_[i - i0] : nullptr, seg_half_[i - i0], 2);
             vcopy(seg_c_[i - i0 + 1], tmp2());
           }
-          if (trick) r2c(r2c1_, tmp2(), seg_chat_[i1 - i0]);
+          if (trick) spectrum(tmp2(), seg_chat_[i1 - i0]);
         }
         for (int i = i1 - 1; i >= i0; i--) {
           adjoint_step(i, seg_half_[i - i0], trick ? seg_chat_[i - i0 + 1] : nullptr,
@@ -1710,6 +1817,14 @@ class Engine final : public EngineBase {
   }
   // acc[6] += w <c_0, D alpha_0>: a D apply on alpha_0 whose spectral epilogue takes the dot
   void kappa_dot_at(const R* chat0, double w) {
+    if (plane()) {
+      PlaneArgs<R> a = plane_args(PP_DOT, p0_, nullptr, xhat_);
+      a.cx = reinterpret_cast<const typename CT<R>::C*>(chat0);
+      a.kdot_weight = w;
+      plane_launch(a, 2 * FB() + SB());
+      st_.total_fft_execs += 1;
+      return;
+    }
     k_solve_config<<<1, 1, 0, stream_>>>(sc_, 0.0, 0.0, rtol_, abstol_, divtol_, maxit_, w);
     GLIA_LAUNCH_CHECK();
     R* spec_a = xhat_;
@@ -1804,7 +1919,7 @@ class Engine final : public EngineBase {
           if (full())
             chat_n = chat_hist_[nt_];
           else
-            r2c(r2c1_, cn, chat_);
+            spectrum(cn, chat_);
           kappa_dot_at(chat_n, 0.5 * dt_);
         } else {
           grad_point(nt_, cn, true);
@@ -2219,6 +2334,10 @@ class Engine final : public EngineBase {
     xpass_ = std::is_same<R, float>::value && (n == 64 || n == 128 || n == 256) && !zpass_ &&
              !ref_ && !(xenv && xenv[0] == '0');
     own_ = xpass_ && !(xenv && std::strcmp(xenv, "2d") == 0);
+    // Grids with a plane kernel run every solve as one launch, in either precision.
+    if (!ref_ && !zpass_ && !(xenv && (xenv[0] == '0' || std::strcmp(xenv, "2d") == 0)))
+      init_plane();
+    if (plane()) xpass_ = own_ = false;
     size_t w2[2] = {0, 0};
     if (xpass_ && !own_) {
       int dims[2] = {n, n};
@@ -2254,6 +2373,36 @@ class Engine final : public EngineBase {
     if (zpass_) GLIA_CUFFT(cufftSetWorkArea(p2d_, fft_ws_));
     if (xpass_ && !own_)
       for (cufftHandle p : {r2c2d3_, c2r2d3_}) GLIA_CUFFT(cufftSetWorkArea(p, fft_ws_));
+  }
+  void init_plane() {
+    using C = typename CT<R>::C;
+    const PlaneKernel k = plane_kernel<R>(g_.n);
+    if (!k.fn) return;
+    GLIA_CUDA(cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem));
+    int b = 0;
+    GLIA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k.fn, k.threads, k.smem));
+    if (b < 1) return;
+    plane_ = k;
+    plane_res_ = sms_ * b;
+    plane_part_ = dalloc<double>((int64_t)kPlanePartials * plane_res_);
+    plane_bar_ = dalloc<unsigned>(2);
+    // exp(2 pi i j / n): float2, or cos and sin in 64-bit fixed point
+    using Tw = std::conditional_t<std::is_same<R, float>::value, float2, FxTw>;
+    std::vector<Tw> tw(g_.n);
+    for (int j = 0; j < g_.n; j++) {
+      const long double a = 2.0L * 3.14159265358979323846264338327950288L * j / g_.n;
+      if constexpr (std::is_same<R, float>::value)
+        tw[j] = make_float2((float)std::cos(a), (float)std::sin(a));
+      else
+        tw[j] = FxTw{fx_from(std::cos(a)), fx_from(std::sin(a))};
+    }
+    plane_tw_ = dalloc<C>(g_.n);
+    if (k.split) plane_w_ = dalloc<R>(3 * N_);
+    if constexpr (std::is_same<R, double>::value) plane_pf_ = dalloc<R>(Ns_);
+    GLIA_CUDA(cudaMemsetAsync(plane_bar_, 0, 2 * sizeof(unsigned), stream_));
+    GLIA_CUDA(cudaMemcpyAsync(plane_tw_, tw.data(), g_.n * sizeof(Tw), cudaMemcpyHostToDevice,
+                              stream_));
+    GLIA_CUDA(cudaStreamSynchronize(stream_));
   }
   void c2c2d(R* data, int dir) {
     cudaEvent_t ev = tm_.begin(stream_);
@@ -2451,6 +2600,15 @@ class Engine final : public EngineBase {
   int64_t cap_solves_ = 0, cap_total_solves_ = 0;
   double cap_reg_ = 0;
   std::vector<double> cap_x_;
+  // plane kernel (plane.cuh) of this grid size: resident CTAs, partial sums, barrier, twiddles
+  PlaneKernel plane_{nullptr, 0, 0, 0, false};
+  R* plane_w_ = nullptr;
+  int plane_res_ = 0;
+  double* plane_part_ = nullptr;
+  unsigned* plane_bar_ = nullptr;
+  typename CT<R>::C* plane_tw_ = nullptr;
+  R* plane_pf_ = nullptr;  // FP64: preconditioner field for pc_c = plane_pc_
+  double plane_pc_ = -1;
   float2* tw_ = nullptr;
   char* fft_ws_ = nullptr;
   char* batch_ws_ = nullptr;

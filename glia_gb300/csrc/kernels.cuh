@@ -555,6 +555,14 @@ __global__ void k_precfactor(Geo g, R* __restrict__ P, double dt, double kbar) {
     P[e] = (v == (R)0) ? factor : factor / v;
   }
 }
+// pc_mult per spectrum element
+template <typename R>
+__global__ void k_pc_field(Geo g, R* __restrict__ P, double pcc) {
+  GRID_STRIDE(e, g.Ns) {
+    SpecIdx s = spec_index((uint32_t)e, g);
+    P[e] = pc_mult<R>((R)pcc, s.wx, s.wy, s.wz);
+  }
+}
 // hadamardComplexProduct (complex x real, src/cuda/UtilsCuda.cu:14-19)
 template <typename R>
 __global__ void k_hadamard_real(int64_t Ns, R* __restrict__ f, const R* __restrict__ P) {

@@ -1,0 +1,1116 @@
+// plane.cuh — a whole diffusion solve (or D apply, smoother, transform) as one persistent kernel.
+//
+// Grids whose (y, z) plane fits in shared memory. A three-dimensional transform is split by
+// direction into two kinds of phase, separated by grid-wide barriers:
+//  - plane phase, one work item per x plane (and gradient component): the y and z transforms of
+//    the plane in shared memory. Between the inverse and the forward z transform the lines are
+//    in real space, where the diffusivity multiplies, the reaction acts and fields are loaded
+//    and stored.
+//  - column phase, one work item per tile of T (ky, kz) columns: the x transforms, forward then
+//    inverse, with the PCG vector updates between them.
+// One PCG iteration is three phases:
+//    columns  p = P r + b p; G_x = F_x^-1(i w_x p)/N, G_0 = F_x^-1(p)/N; sum |p|^2
+//    planes   per component j: grad_j p, times k, sum k (grad_j p)^2, back -> M_j
+//             (j = y: i w_y before; j = z: i w_z before and after)
+//    columns  D p = i w_x F_x M_x + F_x (i w_y M_y + M_z); <p, A p> = sum p^2 + a sum k |grad p|^2
+//             (the derivatives are skew-symmetric), so alpha is known here and x, r are updated
+//             in the same pass; ||P r||, <P r, r>
+// The scalars live in every CTA: after each barrier all CTAs add the same per-CTA partial sums in
+// the same order and take the same decision.
+//
+// Why. Up to 128^3 every array stays in L2 and a solve is bound by latency: as separate launches it
+// took 7 kernels and a conditional graph node an iteration and a graph launch a solve, 35 to 60 us
+// an iteration whatever the size. A barrier costs 1.0 us, a phase at 64^3 4 to 10 us (float).
+// In FP64 the arithmetic is the bound, see fx.cuh. Measured on GB300, before -> after:
+//   mixed  gradient  32^3, 16 steps   14.5 -> 6.8 ms      64^3, 40 steps   41.6 -> 24.9 ms
+//          forward   96^3, 20 steps   13.9 -> 6.2 ms
+//          gradient 128^3, 40 steps   88.0 -> 84.0 ms
+//   FP64   forward   64^3, 100 steps   151 -> 57 ms
+//          gradient 128^3, 6 steps     168 -> 48 ms
+//          solve    256^3               45 -> 15 ms
+//
+// N = R1 R2 (R2 a power of two, so that a group of R2 threads is part of a warp). Inverse
+// transforms read index R2 a + b (R1-point DFTs over a, twiddle w^(b k1), R2-point DFTs over b) and
+// leave index k1 + R1 k2 at place k1 R2 + k2; forward transforms take that order and mirror the
+// steps (R2-point DFTs over k2, twiddle, R1-point DFTs over k1), so nothing is reordered between
+// them and every exchange is in place.
+//
+// A plane holds N / 2 packed complex per line (slot 0: the kz = 0 and kz = N/2 values, both real
+// after the y transform, as re / im). Two neighbouring lines a, b of the place order form one
+// complex line Z = A + i B. Column c of the first sits in slot c of the pair, column c of the
+// second in slot N - c (c = 0: slot N/2), so the thread that has both lines' values at c writes
+// Z[c] and Z[N - c] in their places.
+#pragma once
+
+#include "dft.cuh"
+#include "fx.cuh"
+#include "plane.hpp"
+#include "reduce.cuh"
+
+namespace glia {
+
+__host__ __device__ constexpr int plane_r2(int n) { return n <= 56 ? 4 : (n < 144 ? 8 : 16); }
+
+template <typename R, int NN>
+struct PlaneGeo {
+  using C = typename CT<R>::C;
+  static constexpr int N = NN, R2 = plane_r2(NN), R1 = NN / R2;
+  static constexpr int NQ = N / 2, NH = N / 2 + 1;
+  static constexpr int PL = N * NH;       // complex per x plane of a half spectrum
+  // complex per pair of lines: groups of R2 < 16 lanes that share a wavefront meet different banks
+  // (float), or one slot after every R2 (double, where exchanges in place have no swizzle)
+  static constexpr int GAP = sizeof(R) == 8 ? 1 : 0;
+  static constexpr int PS2 =
+      GAP ? N + R1 : N + (R2 == 4 ? 4 : (R2 == 8 && N % 16 == 0) ? 8 : 0);
+  static __host__ __device__ constexpr int slot(int k) { return GAP ? k + k / R2 : k; }
+  // double planes above 200 KB: y and z in phases of their own (column blocks, lines), see k_plane
+  static constexpr bool SPLIT = GAP && NQ * PS2 * 16 > 200 * 1024;
+  static constexpr int TC = NQ % 16 == 0 ? 16 : 8;  // SPLIT: columns per block
+  static constexpr int PLANE = SPLIT ? 0 : NQ * PS2;
+  // columns per tile: about one tile per resident CTA
+  static constexpr int T = N <= 32 ? 4 : N <= 64 ? 8 : N < 112 ? 16 : SPLIT ? 8 : sizeof(R) == 4 ? 28 : 32;
+  static constexpr int XT = (PL + T - 1) / T;
+  static constexpr int TILE = N * T;
+  static constexpr int RED = 5 * 512 * 8 / (int)sizeof(C);  // partial sums of a phase
+  static constexpr int LINES = SPLIT ? 16 * PS2 : 0;  // one pair of lines per group of R2 lanes
+  static constexpr int BUF0 = 2 * TILE > RED ? 2 * TILE : RED;
+  static constexpr int BUF1 = PLANE > LINES ? PLANE : LINES, BUF = BUF0 > BUF1 ? BUF0 : BUF1;
+  static constexpr int SMEM = (BUF + 4 * N) * (int)sizeof(C);  // + twiddles twice, kz' = 0 twice
+  static constexpr int MINB = SMEM > 110 * 1024 ? 1 : 2;
+  static constexpr int NT = N <= 32 ? 128 : (MINB == 2 ? 256 : 512);
+  static constexpr int NW = NT / 32, GPW = 32 / R2, NG = NW * GPW;
+  static_assert(R1 * R2 == N && N % 2 == 0, "decomposition");
+  static_assert(R1 <= 16, "register DFT");
+  static_assert(!SPLIT || (NG == 16 && N * TC <= BUF), "column block and lines fit the buffer");
+};
+
+// Barrier of all CTAs of a cooperative launch: cnt counts arrivals and is set back to zero by the
+// last CTA that leaves the kernel. The wait is bounded by the SM clock (about one second).
+struct GridBarrier {
+  unsigned* cnt;
+  unsigned target;
+  __device__ __forceinline__ bool sync(int* fault) {
+    __syncthreads();
+    bool late = false;
+    if (threadIdx.x == 0) {
+      target += gridDim.x;
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(cnt) : "memory");
+      const long long t0 = clock64();
+      unsigned v;
+      for (;;) {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(cnt) : "memory");
+        if ((int)(v - target) >= 0) break;
+        if (clock64() - t0 > (1LL << 31)) {
+          late = true;
+          atomicExch(fault, 2);
+          break;
+        }
+      }
+    }
+    return !__syncthreads_or(late);
+  }
+  __device__ __forceinline__ void leave() {
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(cnt + 1, 1u) == gridDim.x - 1) {
+      cnt[0] = 0;
+      cnt[1] = 0;
+    }
+  }
+};
+
+// The DFT tasks of the phases, in registers: float data as they are, doubles in block fixed point
+// (fx.cuh). tw(k) is the table's factor of result k.
+template <class C>
+struct Task;
+template <>
+struct Task<float2> {
+  using Tw = float2;
+  template <int R, int S, bool CONJ, class F>
+  static __device__ __forceinline__ void dft_tw(float2 (&v)[R], F&& tw) {
+    reg_dft<R, S>(v);
+#pragma unroll
+    for (int k = 0; k < R; k++) v[k] = CONJ ? cmulc(v[k], tw(k)) : cmul2(v[k], tw(k));
+  }
+  template <int R, int S>
+  static __device__ __forceinline__ void dft(float2 (&v)[R]) {
+    reg_dft<R, S>(v);
+  }
+  // inputs times i w(a)
+  template <int R, int S, class W, class F>
+  static __device__ __forceinline__ void dft_iw_tw(float2 (&v)[R], W&& w, F&& tw) {
+#pragma unroll
+    for (int a = 0; a < R; a++) v[a] = cimul<float2>((float)w(a), v[a]);
+    dft_tw<R, S, false>(v, tw);
+  }
+  // inputs i w u(a) + v(a), loaded here
+  template <int R, int S, class U, class V, class F>
+  static __device__ __forceinline__ void dft_sum_tw(float2 (&q)[R], U&& u, V&& v, int w, F&& tw) {
+    float2 x[R];
+#pragma unroll
+    for (int a = 0; a < R; a++) q[a] = v(a);
+#pragma unroll
+    for (int a = 0; a < R; a++) x[a] = u(a);
+#pragma unroll
+    for (int a = 0; a < R; a++) q[a] = cadd(q[a], cimul<float2>((float)w, x[a]));
+    dft_tw<R, S, true>(q, tw);
+  }
+  // results (times i w when dz) in pairs a, h -> Z[c] = a + i h, Z[N - c] = conj a + i conj h;
+  // c = 0: re / im hold the two packed real values of each
+  template <int R>
+  static __device__ __forceinline__ void dft_pair(float2 (&v)[R], int c, bool dz) {
+    reg_dft<R, +1>(v);
+#pragma unroll
+    for (int i = 0; i < R / 2; i++) {
+      float2 a = v[2 * i], h = v[2 * i + 1];
+      if (dz) {
+        a = cimul<float2>((float)c, a);
+        h = cimul<float2>((float)c, h);
+      }
+      v[2 * i] = c == 0 ? make_float2(a.x, h.x) : make_float2(a.x - h.y, a.y + h.x);
+      v[2 * i + 1] = c == 0 ? make_float2(a.y, h.y) : make_float2(a.x + h.y, h.x - a.y);
+    }
+  }
+  // the way back: pairs Z[c], Z[N - c] -> a, h (times i w when dz), DFT
+  template <int R, class F>
+  static __device__ __forceinline__ void split_dft_tw(float2 (&v)[R], int c, bool dz, F&& tw) {
+#pragma unroll
+    for (int i = 0; i < R / 2; i++) {
+      const float2 z = v[2 * i], zq = v[2 * i + 1];
+      float2 a = make_float2(0.5f * (z.x + zq.x), 0.5f * (z.y - zq.y));
+      float2 h = make_float2(0.5f * (z.y + zq.y), -0.5f * (z.x - zq.x));
+      if (c == 0) {
+        a = make_float2(z.x, zq.x);
+        h = make_float2(z.y, zq.y);
+      }
+      v[2 * i] = dz ? cimul<float2>((float)c, a) : a;
+      v[2 * i + 1] = dz ? cimul<float2>((float)c, h) : h;
+    }
+    dft_tw<R, -1, true>(v, tw);
+  }
+};
+// Doubles: block fixed point (fx.cuh). One body per radix for every use, called, not inlined: the
+// integer code of a 16-point task is about 3000 instructions, and inlined at each use it ran out
+// of the instruction cache (measured: 5.6 stalled warps waiting for instructions per issue).
+enum FxMode {
+  FX_FWD = 1,    // forward transform (real and imaginary parts swapped around an inverse one)
+  FX_IW = 2,     // inputs times i w(a), w(a) the wave number of w0 + wl a
+  FX_IC = 4,     // inputs times i w0
+  FX_PAIR = 8,   // results in pairs a, h -> Z[c] = a + i h, Z[N - c] = conj a + i conj h
+  FX_SPLIT = 16, // inputs in pairs Z[c], Z[N - c] -> a, h
+  FX_C0 = 32,    // of c = 0: re / im hold the two packed real values of each line
+  FX_SUM = 64    // inputs i w0 src(a) + src2(a)
+};
+template <int R, int N, class AtS, class AtD>
+__device__ __forceinline__ void fx_task_body(const double2* src, const double2* src2, double2* dst,
+                                             AtS&& at_s, AtD&& at_d, const FxTw* tw, int twl,
+                                             int mode, int w0, int wl) {
+  constexpr int B = 61 - fx_log2(R);
+  double2 v[R];
+#pragma unroll
+  for (int a = 0; a < R; a++) v[a] = src[at_s(a)];
+  fx2 q[R];
+  int E;
+  if (mode & (FX_IW | FX_IC)) {
+    auto w = [&](int a) { return (mode & FX_IC) ? w0 : wavenum(w0 + wl * a, N); };
+    E = 0;
+#pragma unroll
+    for (int a = 0; a < R; a++) E = max(E, fx_exp_w<B>(v[a], w(a)));
+#pragma unroll
+    for (int a = 0; a < R; a++) q[a] = fx_in2_iw<B>(v[a], E, w(a));
+    if (mode & FX_SUM) {  // src on its own exponent first: one of the two in registers as doubles
+      const int Eu = E;
+#pragma unroll
+      for (int a = 0; a < R; a++) v[a] = src2[at_s(a)];
+      E = max(E, fx_block(v));
+      const int sh = min(E - Eu, 63);
+#pragma unroll
+      for (int a = 0; a < R; a++)
+        q[a] = cadd(cmk<fx2>(q[a].x >> sh, q[a].y >> sh), fx_in2<B>(v[a], E));
+    }
+  } else {
+    E = fx_block(v);
+#pragma unroll
+    for (int a = 0; a < R; a++) q[a] = fx_in2<B>(v[a], E);
+  }
+  int adj = 0;
+  if (R % 2 == 0 && (mode & FX_SPLIT)) {  // twice a and h
+    adj = -1;
+    if (mode & FX_C0) {
+#pragma unroll
+      for (int i = 0; i < R / 2; i++) {
+        const fx2 z = q[2 * i], zq = q[2 * i + 1];
+        q[2 * i] = cmk<fx2>(2 * z.x, 2 * zq.x);
+        q[2 * i + 1] = cmk<fx2>(2 * z.y, 2 * zq.y);
+      }
+    } else {
+      // conj of an input that was multiplied by i c is minus i c times the conjugate
+      const int64_t s = (mode & FX_IC) ? -1 : 0;
+#pragma unroll
+      for (int i = 0; i < R / 2; i++) {
+        const fx2 z = q[2 * i];
+        const fx2 zq = cmk<fx2>((q[2 * i + 1].x ^ s) - s, (q[2 * i + 1].y ^ s) - s);
+        q[2 * i] = cmk<fx2>(z.x + zq.x, z.y - zq.y);
+        q[2 * i + 1] = cmk<fx2>(z.y + zq.y, zq.x - z.x);
+      }
+    }
+  }
+  const bool swap = mode & FX_FWD;
+#pragma unroll
+  for (int a = 0; a < R; a++)
+    q[a] = cmk<fx2>(swap ? q[a].y : q[a].x, swap ? q[a].x : q[a].y);
+  reg_dft<R, +1>(q);
+  if (tw) {
+    adj += 1;
+#pragma unroll
+    for (int k = 0; k < R; k++) q[k] = fx_tw(q[k], tw[k * twl]);
+  }
+#pragma unroll
+  for (int a = 0; a < R; a++)
+    q[a] = cmk<fx2>(swap ? q[a].y : q[a].x, swap ? q[a].x : q[a].y);
+  if (R % 2 == 0 && (mode & FX_PAIR)) {
+    const bool c0 = mode & FX_C0;
+#pragma unroll
+    for (int i = 0; i < R / 2; i++) {
+      const fx2 a = q[2 * i], h = q[2 * i + 1];
+      q[2 * i] = c0 ? cmk<fx2>(a.x, h.x) : cmk<fx2>(a.x - h.y, a.y + h.x);
+      q[2 * i + 1] = c0 ? cmk<fx2>(a.y, h.y) : cmk<fx2>(a.x + h.y, h.x - a.y);
+    }
+  }
+  fx_store<R, B>(q, v, E, adj);
+#pragma unroll
+  for (int a = 0; a < R; a++) dst[at_d(a)] = v[a];
+}
+// values at src[a ls], results at dst[a ld]
+template <int R, int N>
+__device__ __noinline__ void fx_task1(const double2* src, const double2* src2, int ls,
+                                      double2* dst, int ld, const FxTw* tw, int twl, int mode,
+                                      int w0, int wl) {
+  fx_task_body<R, N>(src, src2, dst, [&](int a) { return a * ls; }, [&](int a) { return a * ld; },
+                     tw, twl, mode, w0, wl);
+}
+// values at src[(a >> 1) s2 + (a & 1) s1], results at dst[(a >> 1) d2 + (a & 1) d1]
+template <int R, int N>
+__device__ __noinline__ void fx_task2(const double2* src, int s1, int s2, double2* dst, int d1,
+                                      int d2, const FxTw* tw, int twl, int mode, int w0, int wl) {
+  fx_task_body<R, N>(src, nullptr, dst, [&](int a) { return (a >> 1) * s2 + (a & 1) * s1; },
+                     [&](int a) { return (a >> 1) * d2 + (a & 1) * d1; }, tw, twl, mode, w0, wl);
+}
+template <>
+struct Task<double2> {
+  using Tw = FxTw;
+};
+
+enum PlaneStep {
+  PS_FWD = 0,   // planes: real field -> y, z forward
+  PS_GRAD,      // planes: G -> gradient, times k, -> M
+  PS_BACK,      // planes: G_0 -> real field
+  PS_YINV,      // SPLIT: columns of planes, y inverse, G -> W (Z pairs)
+  PS_LINE,      // SPLIT: line pairs in W, z inverse, k, z forward (GRAD; FWD: z forward only;
+                //        BACK: z inverse only)
+  PS_YFWD,      // SPLIT: columns of planes, y forward, W -> M
+  PS_SPEC,      // columns: M_0 -> spectrum (stored)
+  PS_ENTER,     // columns: M_0 -> spectrum (stored) -> G_x, G_0
+  PS_OPEN,      // columns: given spectrum -> G_x, G_0
+  PS_SMOOTH,    // columns: M_0 -> spectrum times mulk -> G_0
+  PS_SETUP,     // columns: M -> D c, solve set-up, first direction -> G_x, G_0
+  PS_UPDATE,    // columns: M -> D p, x and r
+  PS_DIR,       // columns: next direction -> G_x, G_0
+  PS_LEAVE,     // columns: x -> G_0
+  PS_APPLY,     // columns: M -> D u -> G_0
+  PS_DOT        // columns: M -> <cx, D u>
+};
+
+template <typename R, int NN>
+__global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
+    k_plane(const __grid_constant__ PlaneArgs<R> A) {
+  using Geo_ = PlaneGeo<R, NN>;
+  using C = typename Geo_::C;
+  constexpr int N = NN, R1 = Geo_::R1, R2 = Geo_::R2, NQ = Geo_::NQ, NH = Geo_::NH, PL = Geo_::PL,
+                T = Geo_::T, NT = Geo_::NT, PS2 = Geo_::PS2, TILE = Geo_::TILE;
+  constexpr int S = N * PL;
+  constexpr bool FX = sizeof(R) == 8;
+  extern __shared__ double2 plane_dyn[];
+  C* buf = reinterpret_cast<C*>(plane_dyn);
+  using K = Task<C>;
+  using Tw = typename K::Tw;
+  static_assert(sizeof(Tw) == sizeof(C), "table entry");
+  Tw* twA = reinterpret_cast<Tw*>(buf + Geo_::BUF);  // [k1 R2 + b] exp(+2 pi i b k1 / N)
+  Tw* twB = twA + N;                                 // [b R1 + k1], the same
+  C* zcol = reinterpret_cast<C*>(twB + N);           // column kz' = 0 of a plane, forward
+  C* zin = zcol + N;                                 // and inverse
+  __shared__ double tot[5];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < N; i += NT) {
+    const int k1 = i / R2, b = i - k1 * R2;
+    const Tw w = reinterpret_cast<const Tw*>(A.tw)[b * k1];  // b k1 < N
+    twA[i] = w;
+    twB[b * R1 + k1] = w;
+  }
+  __syncthreads();
+  const R invN = (R)(1.0 / ((double)N * N * N));
+  const double dinvN = 1.0 / ((double)N * N * N);
+  const R a_cn = (R)A.a_cn, pcc = (R)A.pc_c;
+  GridBarrier bar{A.bar, 0};
+  // PCG scalars, the same in every CTA (thread 0 updates them)
+  __shared__ struct {
+    double beta, beta_old, dpi, dpi_old, alpha, bcoef;
+    double dp, rnorm0, ttol, pp;  // squares
+    int it, iter, status, step;
+  } cg;
+  if (tid == 0) {
+    cg.dpi = cg.dp = cg.alpha = cg.bcoef = 0.0;
+    cg.it = cg.iter = cg.status = 0;
+  }
+  C* __restrict__ const Gp = A.G;
+  C* __restrict__ const Mp = A.M;
+  C* __restrict__ const xh = A.xhat;
+  C* __restrict__ const rh = A.rhat;
+  C* __restrict__ const ph = A.phat;
+  C* __restrict__ const ch = A.chat;
+  const R* __restrict__ const kf = A.k;
+
+  // per-CTA partial sums of slots s0 ... s0 + Q - 1, and their totals after the next barrier
+  // (few FP64 operations: all threads' values go to shared memory and one warp adds each sum)
+  auto partials = [&](const double* v, int q_n, int s0) {
+    double* all = reinterpret_cast<double*>(buf);
+    __syncthreads();
+    for (int q = 0; q < q_n; q++) all[q * NT + tid] = v[q];
+    __syncthreads();
+    for (int q = warp; q < q_n; q += Geo_::NW) {
+      double x = 0;
+#pragma unroll
+      for (int w = 0; w < Geo_::NW; w++) x += all[q * NT + 32 * w + lane];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+      if (lane == 0) A.part[(s0 + q) * gridDim.x + blockIdx.x] = x;
+    }
+  };
+  auto totals = [&](int q_n, int s0) {
+    for (int q = warp; q < q_n; q += Geo_::NW) {
+      double x = 0;
+      for (int b = lane; b < (int)gridDim.x; b += 32) x += __ldcg(&A.part[(s0 + q) * gridDim.x + b]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+      if (lane == 0) tot[q] = x;
+    }
+    __syncthreads();
+  };
+  // PETSc's default test (conv_test of the other engines), on the squares of the norms
+  auto converged = [&](double rn) {
+    if (isnan(rn) || isinf(rn)) return -9;
+    if (rn <= cg.ttol) return 1;
+    if (rn >= A.divtol * A.divtol * cg.rnorm0) return -4;
+    return 0;
+  };
+
+  // the reaction step on two voxels as their field is read
+  auto reacted = [&](C v, int64_t i0, int64_t i1) {
+    const R e0 = exp(A.rho[i0] * A.dt), e1 = exp(A.rho[i1] * A.dt);
+    if (A.pre == 1) {  // logistic (k_reaction_fwd)
+      if (A.half) {
+        A.half[i0] = v.x;
+        A.half[i1] = v.y;
+      }
+      const R c0 = v.x * e0, c1 = v.y * e1;
+      return cmk<C>(c0 / (c0 + (R)1 - v.x), c1 / (c1 + (R)1 - v.y));
+    }
+    // linearised at lin (k_reaction_lin)
+    const R c0 = A.lin[i0], c1 = A.lin[i1];
+    const R q0 = c0 * e0 + (R)1 - c0, q1 = c1 * e1 + (R)1 - c1;
+    return cmk<C>(v.x * e0 / (q0 * q0), v.y * e1 / (q1 * q1));
+  };
+
+  Acc<R> acc[5];
+  // Double: row k1 of a line pair in real space (places k2, z = k1 + R1 k2 of lines l0 and l1)
+  auto line_middle = [&](int kind, C* row, int64_t l0, int64_t l1, int k1) {
+    if constexpr (FX) {
+      if (kind == PS_FWD) {
+#pragma unroll 2
+        for (int k2 = 0; k2 < R2; k2++) {
+          const int m = k1 + R1 * k2;
+          row[k2] = cmk<C>(A.in[l0 + m], A.in[l1 + m]);
+          if (A.pre) row[k2] = reacted(row[k2], l0 + m, l1 + m);
+        }
+      } else {
+        fx_task2<R2, N>(row, 1, 2, row, 1, 2, nullptr, 0, 0, 0, 0);
+        if (kind == PS_GRAD) {
+#pragma unroll 4
+          for (int k2 = 0; k2 < R2; k2++) {
+            const int m = k1 + R1 * k2;
+            const C z = row[k2];
+            const R sx = z.x * kf[l0 + m], sy = z.y * kf[l1 + m];
+            acc[0].add(sx * z.x + sy * z.y);
+            row[k2] = cmk<C>(sx, sy);
+          }
+        } else {
+#pragma unroll 4
+          for (int k2 = 0; k2 < R2; k2++) {
+            const int m = k1 + R1 * k2;
+            A.out[l0 + m] = row[k2].x;
+            A.out[l1 + m] = row[k2].y;
+          }
+        }
+      }
+      if (kind != PS_BACK)
+        fx_task2<R2, N>(row, 1, 2, row, 1, 2, twA + k1 * R2, 1, FX_FWD, 0, 0);
+    }
+  };
+
+  // slots of column c in the first and the second line of a pair
+  auto even = [](int c) { return Geo_::slot(c); };
+  auto odd = [](int c) { return Geo_::slot(c == 0 ? NQ : N - c); };
+
+  int step = A.prog == PP_SOLVE_SPEC ? PS_OPEN : Geo_::SPLIT ? PS_LINE : PS_FWD;
+  bool started = false;  // the solve's set-up is done
+  int kind = PS_FWD;  // SPLIT: the plane phase that the current y and line phases are part of
+  for (;;) {
+#pragma unroll
+    for (int q = 0; q < 5; q++) acc[q] = Acc<R>{};
+    if constexpr (Geo_::SPLIT) {
+      if (step == PS_YINV || step == PS_YFWD) {
+        // ------------------------------------------------------ SPLIT: column blocks of planes
+        constexpr int TC = Geo_::TC, CB = NQ / TC;
+        const int nj = kind == PS_GRAD ? 3 : 1;
+        for (int item = blockIdx.x; item < nj * N * CB; item += gridDim.x) {
+          const int cb = item % CB, xj = item / CB, x = xj / nj, j = xj - nj * x;
+          C* const W = A.W + ((int64_t)j * N + x) * NQ * N + cb * TC;
+          if (step == PS_YINV) {
+            const C* G = (kind == PS_GRAD && j == 0 ? Gp : Gp + S) + x * PL + cb * TC;
+            if (cb == 0)
+              for (int ky = tid; ky < N; ky += NT) {
+                const C z = G[ky * NH], w = G[ky * NH + NQ];
+                zin[ky] = cmk<C>(z.x - w.y, z.y + w.x);
+              }
+            __syncthreads();
+            for (int task = tid; task < TC * R2; task += NT) {
+              const int b = task / TC, c = task - b * TC;
+              const bool c0 = cb == 0 && c == 0;
+              const int ld = c0 ? 1 : NH;
+              fx_task1<R1, N>((c0 ? zin : G + c) + b * ld, nullptr, R2 * ld, buf + b * TC + c,
+                              R2 * TC, twA + b, R2, j == 1 ? FX_IW : 0, b, R2);
+            }
+            __syncthreads();
+            for (int task = tid; task < TC * R1; task += NT) {
+              const int k1 = task / TC, c = task - k1 * TC, cc = cb * TC + c;
+              fx_task2<R2, N>(buf + k1 * R2 * TC + c, TC, 2 * TC, W + k1 * (R2 / 2) * N + c,
+                              (cc == 0 ? NQ : N - cc) - cc, N, nullptr, 0,
+                              FX_PAIR | (j == 2 ? FX_IC : 0) | (cc == 0 ? FX_C0 : 0), cc, 0);
+            }
+          } else {
+            for (int task = tid; task < TC * R1; task += NT) {
+              const int k1 = task / TC, c = task - k1 * TC, cc = cb * TC + c;
+              fx_task2<R2, N>(W + k1 * (R2 / 2) * N + c, (cc == 0 ? NQ : N - cc) - cc, N,
+                              buf + k1 * R2 * TC + c, TC, 2 * TC, twA + k1 * R2, 1,
+                              FX_FWD | FX_SPLIT | (j == 2 ? FX_IC : 0) | (cc == 0 ? FX_C0 : 0),
+                              cc, 0);
+            }
+            __syncthreads();
+            C* M = Mp + j * S + x * PL;
+            for (int task = tid; task < TC * R2; task += NT) {
+              const int b = task / TC, c = task - b * TC;
+              const bool c0 = cb == 0 && c == 0;
+              const int ld = c0 ? 1 : NH;
+              fx_task1<R1, N>(buf + b * TC + c, nullptr, R2 * TC,
+                              (c0 ? zcol : M + cb * TC + c) + b * ld, R2 * ld, nullptr, 0, FX_FWD,
+                              0, 0);
+            }
+            __syncthreads();
+            if (cb == 0)
+              for (int ky = tid; ky < N; ky += NT) {
+                const C z = zcol[ky], zm = zcol[ky == 0 ? 0 : N - ky];
+                M[ky * NH] = cmk<C>((R)0.5 * (z.x + zm.x), (R)0.5 * (z.y - zm.y));
+                M[ky * NH + NQ] = cmk<C>((R)0.5 * (z.y + zm.y), (R)-0.5 * (z.x - zm.x));
+              }
+          }
+          __syncthreads();
+        }
+      } else if (step == PS_LINE) {
+        // ----------------------------------------------------- SPLIT: line pairs of all planes
+        const int nj = kind == PS_GRAD ? 3 : 1;
+        const int g = lane / R2, t = lane % R2;
+        C* const E = buf + (warp * Geo_::GPW + g) * PS2;
+        C* const col = E + t;
+        const int pairs = nj * N * NQ, per = gridDim.x * Geo_::NG;
+        for (int base = blockIdx.x * Geo_::NG + warp * Geo_::GPW; base < pairs; base += per) {
+          // pair pr of plane x, component j fastest (the three share k)
+          const int id = base + g, j = id % nj, px = id / nj, x = px / NQ, pr = px - x * NQ;
+          const int p0 = 2 * pr, y0 = p0 / R2 + R1 * (p0 % R2);
+          const int64_t l0 = ((int64_t)x * N + y0) * N, l1 = l0 + (int64_t)R1 * N;
+          C* const W = A.W + (((int64_t)j * N + x) * NQ + pr) * N + t;
+          const bool on = id < pairs;
+          if (kind != PS_FWD) {
+            if (on) fx_task1<R1, N>(W, nullptr, R2, col, R2 + 1, twA + t, R2, 0, 0, 0);
+            __syncwarp();
+          }
+          if (on) {
+            for (int k1 = t; k1 < R1; k1 += R2)
+              line_middle(kind, E + k1 * (R2 + 1), l0, l1, k1);
+          }
+          if (kind != PS_BACK) {
+            __syncwarp();
+            if (on) fx_task1<R1, N>(col, nullptr, R2 + 1, W, R2, nullptr, 0, FX_FWD, 0, 0);
+          }
+          __syncwarp();
+        }
+        if (kind == PS_GRAD) {
+          const double v[1] = {acc[0].value()};
+          partials(v, 1, 1);
+        }
+      }
+    }
+    if (step <= PS_BACK && !Geo_::SPLIT) {
+      // ------------------------------------------------------------------------------ planes
+      const int items = step == PS_GRAD ? 3 * N : N;
+      for (int item = blockIdx.x; item < items; item += gridDim.x) {
+        const int x = step == PS_GRAD ? item / 3 : item;
+        const int j = step == PS_GRAD ? item - 3 * x : 0;
+        if (step != PS_FWD) {
+          // y inverse: the kz = 0 and kz = N/2 columns as one, then rows ky = R2 a + b of column c
+          const C* G = (step == PS_GRAD && j == 0 ? Gp : Gp + S) + x * PL;
+          for (int ky = tid; ky < N; ky += NT) {
+            const C z = G[ky * NH], w = G[ky * NH + NQ];
+            zin[ky] = cmk<C>(z.x - w.y, z.y + w.x);
+          }
+          __syncthreads();
+          for (int task = tid; task < NQ * R2; task += NT) {
+            const int b = task / NQ, c = task - b * NQ;
+            const C* src = c == 0 ? zin : G + c;
+            const int ld = c == 0 ? 1 : NH;
+            if constexpr (FX) {
+              fx_task1<R1, N>(src + b * ld, nullptr, R2 * ld,
+                              buf + (b >> 1) * PS2 + ((b & 1) ? odd(c) : even(c)), R2 / 2 * PS2,
+                              twA + b, R2, j == 1 ? FX_IW : 0, b, R2);
+            } else {
+            C u[R1];
+#pragma unroll
+            for (int a = 0; a < R1; a++) u[a] = src[(R2 * a + b) * ld];
+            auto tw = [&](int k1) { return twA[k1 * R2 + b]; };
+            if (j == 1)
+              K::template dft_iw_tw<R1, +1>(u, [&](int a) { return wavenum(R2 * a + b, N); }, tw);
+            else
+              K::template dft_tw<R1, +1, false>(u, tw);
+#pragma unroll
+            for (int k1 = 0; k1 < R1; k1++) {
+              buf[(k1 * (R2 / 2) + (b >> 1)) * PS2 + ((b & 1) ? odd(c) : even(c))] = u[k1];
+            }
+            }
+          }
+          __syncthreads();
+          for (int task = tid; task < NQ * R1; task += NT) {
+            const int k1 = task / NQ, c = task - k1 * NQ;
+            C* row = buf + k1 * (R2 / 2) * PS2 + even(c);
+            const int od = odd(c) - even(c);
+            if constexpr (FX) {
+              fx_task2<R2, N>(row, od, PS2, row, od, PS2, nullptr, 0,
+                              FX_PAIR | (j == 2 ? FX_IC : 0) | (c == 0 ? FX_C0 : 0), c, 0);
+            } else {
+            C v[R2];
+#pragma unroll
+            for (int b = 0; b < R2; b++) v[b] = row[(b >> 1) * PS2 + (b & 1) * od];
+            K::template dft_pair<R2>(v, c, j == 2);
+#pragma unroll
+            for (int b = 0; b < R2; b++) row[(b >> 1) * PS2 + (b & 1) * od] = v[b];
+            }
+          }
+          __syncthreads();
+        }
+        // z lines, two at a time: R2 lanes per pair
+        for (int base = warp * Geo_::GPW; base < NQ; base += Geo_::NG) {
+          const int g = lane / R2, t = lane % R2, pr = base + g;
+          const bool on = pr < NQ;
+          C* E = buf + (on ? pr : 0) * PS2;
+          const int p0 = 2 * pr, y0 = p0 / R2 + R1 * (p0 % R2), y1 = y0 + R1;
+          const int64_t l0 = ((int64_t)x * N + y0) * N, l1 = ((int64_t)x * N + y1) * N;
+          if constexpr (FX) {
+            // thread t: index R2 a + t in place, then rows k1 = t, t + R2, ... in place, and back
+            C* const col = E + t;
+            if (step != PS_FWD) {
+              if (on) fx_task1<R1, N>(col, nullptr, R2 + 1, col, R2 + 1, twA + t, R2, 0, 0, 0);
+              __syncwarp();
+            }
+            if (on) {
+              for (int k1 = t; k1 < R1; k1 += R2)
+                line_middle(step, E + k1 * (R2 + 1), l0, l1, k1);
+            }
+            if (step != PS_BACK) {
+              __syncwarp();
+              if (on) fx_task1<R1, N>(col, nullptr, R2 + 1, col, R2 + 1, nullptr, 0, FX_FWD, 0, 0);
+            }
+            continue;
+          } else {
+          auto ex = [&](int k1, int q) -> C& { return E[k1 * R2 + (q ^ (k1 & (R2 - 1)))]; };
+          if (step != PS_FWD) {
+            C u[R1];
+            if (on) {
+#pragma unroll
+              for (int a = 0; a < R1; a++) u[a] = E[R2 * a + t];
+              K::template dft_tw<R1, +1, false>(u, [&](int k1) { return twA[k1 * R2 + t]; });
+            }
+            __syncwarp();
+            if (on) {
+#pragma unroll
+              for (int k1 = 0; k1 < R1; k1++) ex(k1, t) = u[k1];
+            }
+            __syncwarp();
+          }
+          if (on) {
+#pragma unroll
+            for (int ii = 0; ii < (R1 + R2 - 1) / R2; ii++) {
+              const int k1 = t + R2 * ii;
+              if (R1 % R2 != 0 && k1 >= R1) continue;
+              C v[R2];
+              if (step == PS_FWD) {
+#pragma unroll
+                for (int k2 = 0; k2 < R2; k2++) {
+                  const int m = k1 + R1 * k2;
+                  v[k2] = cmk<C>(A.in[l0 + m], A.in[l1 + m]);
+                }
+                if (A.pre) {
+#pragma unroll
+                  for (int k2 = 0; k2 < R2; k2++)
+                    v[k2] = reacted(v[k2], l0 + k1 + R1 * k2, l1 + k1 + R1 * k2);
+                }
+              } else {
+                R ka[R2], kb[R2];
+                if (step == PS_GRAD) {
+#pragma unroll
+                  for (int k2 = 0; k2 < R2; k2++) {
+                    ka[k2] = kf[l0 + k1 + R1 * k2];
+                    kb[k2] = kf[l1 + k1 + R1 * k2];
+                  }
+                }
+#pragma unroll
+                for (int q = 0; q < R2; q++) v[q] = ex(k1, q);
+                K::template dft<R2, +1>(v);  // v[k2]: lines a, b at z = k1 + R1 k2
+                if (step == PS_GRAD) {
+#pragma unroll
+                  for (int k2 = 0; k2 < R2; k2++) {
+                    const R sx = v[k2].x * ka[k2], sy = v[k2].y * kb[k2];
+                    acc[0].add(sx * v[k2].x + sy * v[k2].y);
+                    v[k2] = cmk<C>(sx, sy);
+                  }
+                } else {
+#pragma unroll
+                  for (int k2 = 0; k2 < R2; k2++) {
+                    const int m = k1 + R1 * k2;
+                    A.out[l0 + m] = v[k2].x;
+                    A.out[l1 + m] = v[k2].y;
+                  }
+                }
+              }
+              if (step != PS_BACK) {
+                K::template dft_tw<R2, -1, true>(v, [&](int q) { return twB[q * R1 + k1]; });
+#pragma unroll
+                for (int q = 0; q < R2; q++) ex(k1, q) = v[q];
+              }
+            }
+          }
+          if (step != PS_BACK) {
+            __syncwarp();
+            C u[R1];
+            if (on) {
+#pragma unroll
+              for (int k1 = 0; k1 < R1; k1++) u[k1] = ex(k1, t);
+              K::template dft<R1, -1>(u);
+            }
+            __syncwarp();
+            if (on) {
+#pragma unroll
+              for (int a = 0; a < R1; a++) E[R2 * a + t] = u[a];
+            }
+          }
+          }
+        }
+        __syncthreads();
+        if (step != PS_BACK) {
+          // y forward: places k1 R2 + k2 of column c, split into the two lines of each pair
+          for (int task = tid; task < NQ * R1; task += NT) {
+            const int k1 = task / NQ, c = task - k1 * NQ;
+            C* row = buf + k1 * (R2 / 2) * PS2 + even(c);
+            const int od = odd(c) - even(c);
+            if constexpr (FX) {
+              fx_task2<R2, N>(row, od, PS2, row, od, PS2, twA + k1 * R2, 1,
+                              FX_FWD | FX_SPLIT | (j == 2 ? FX_IC : 0) | (c == 0 ? FX_C0 : 0), c,
+                              0);
+            } else {
+            C v[R2];
+#pragma unroll
+            for (int b = 0; b < R2; b++) v[b] = row[(b >> 1) * PS2 + (b & 1) * od];
+            K::template split_dft_tw<R2>(v, c, j == 2, [&](int b) { return twA[k1 * R2 + b]; });
+#pragma unroll
+            for (int b = 0; b < R2; b++) row[(b >> 1) * PS2 + (b & 1) * od] = v[b];
+            }
+          }
+          __syncthreads();
+          C* M = Mp + j * S + x * PL;
+          for (int task = tid; task < NQ * R2; task += NT) {
+            const int b = task / NQ, c = task - b * NQ;
+            C* dst = c == 0 ? zcol : M + c;
+            const int ld = c == 0 ? 1 : NH;
+            if constexpr (FX) {
+              fx_task1<R1, N>(buf + (b >> 1) * PS2 + ((b & 1) ? odd(c) : even(c)), nullptr,
+                              R2 / 2 * PS2, dst + b * ld, R2 * ld, nullptr, 0, FX_FWD, 0, 0);
+            } else {
+            C u[R1];
+#pragma unroll
+            for (int k1 = 0; k1 < R1; k1++) {
+              u[k1] = buf[(k1 * (R2 / 2) + (b >> 1)) * PS2 + ((b & 1) ? odd(c) : even(c))];
+            }
+            K::template dft<R1, -1>(u);
+#pragma unroll
+            for (int a = 0; a < R1; a++) dst[(b + R2 * a) * ld] = u[a];
+            }
+          }
+          __syncthreads();
+          for (int ky = tid; ky < N; ky += NT) {  // kz' = 0 into kz = 0 and kz = N/2
+            const C z = zcol[ky], zm = zcol[ky == 0 ? 0 : N - ky];
+            M[ky * NH] = cmk<C>((R)0.5 * (z.x + zm.x), (R)0.5 * (z.y - zm.y));
+            M[ky * NH + NQ] = cmk<C>((R)0.5 * (z.y + zm.y), (R)-0.5 * (z.x - zm.x));
+          }
+        }
+      }
+      if (step == PS_GRAD) {
+        const double v[1] = {acc[0].value()};
+        partials(v, 1, 1);
+      }
+    } else if (step >= PS_SPEC) {
+      // ----------------------------------------------------------------------------- columns
+      const int nin = step == PS_SPEC || step == PS_ENTER || step == PS_SMOOTH ? 1
+                      : step == PS_OPEN || step == PS_DIR || step == PS_LEAVE  ? 0
+                                                                               : 2;
+      const int nout = step == PS_SMOOTH || step == PS_LEAVE || step == PS_APPLY ? 1
+                       : step == PS_SPEC || step == PS_UPDATE || step == PS_DOT  ? 0
+                                                                                 : 2;
+      if (step == PS_UPDATE) {  // alpha
+        totals(2, 0);
+        if (tid == 0) {
+          if (cg.iter == 0) tot[0] = cg.pp;  // of the set-up's first direction
+          cg.dpi_old = cg.dpi;
+          cg.dpi = tot[0] * dinvN + A.a_cn * tot[1];
+          cg.beta_old = cg.beta;
+          cg.it = cg.iter + 1;
+          if (cg.dpi == 0.0 || (cg.iter > 0 && cg.dpi * cg.dpi_old <= 0.0))
+            cg.status = -8;
+          else if (isnan(cg.dpi) || isinf(cg.dpi))
+            cg.status = -9;
+          else
+            cg.alpha = cg.beta / cg.dpi;
+        }
+        __syncthreads();
+        if (cg.status != 0) {  // x and r stay as they are
+          if (A.prog == PP_SOLVE_SPEC) break;
+          step = PS_LEAVE;
+          continue;
+        }
+      }
+      const R al = (R)cg.alpha, alN = (R)(cg.alpha * dinvN), bc = (R)cg.bcoef;
+      for (int tile = blockIdx.x; tile < Geo_::XT; tile += gridDim.x) {
+        for (int i = 0; i < nin; i++) {  // forward, first part: rows x = R2 a + b
+          for (int task = tid; task < T * R2; task += NT) {
+            const int c = task % T, b = task / T, q = tile * T + c;
+            if (q >= PL) continue;
+            const C* src = Mp + i * S + q;
+            if constexpr (FX) {  // M_x, then i w_y M_y + M_z
+              fx_task1<R1, N>(src + b * PL, i == 1 ? src + S + b * PL : nullptr, R2 * PL,
+                              buf + i * TILE + b * T + c, R2 * T, twA + b, R2,
+                              i == 1 ? FX_FWD | FX_IC | FX_SUM : FX_FWD, wavenum(q / NH, N), 0);
+              continue;
+            } else {
+            C u[R1];
+            auto tw = [&](int k1) { return twA[k1 * R2 + b]; };
+            if (i == 1) {  // i w_y M_y + M_z
+              K::template dft_sum_tw<R1, -1>(
+                  u, [&](int a) { return src[(R2 * a + b) * PL]; },
+                  [&](int a) { return src[S + (R2 * a + b) * PL]; }, wavenum(q / NH, N), tw);
+            } else {
+#pragma unroll
+              for (int a = 0; a < R1; a++) u[a] = src[(R2 * a + b) * PL];
+              K::template dft_tw<R1, -1, true>(u, tw);
+            }
+#pragma unroll
+            for (int k1 = 0; k1 < R1; k1++) buf[i * TILE + (k1 * R2 + b) * T + c] = u[k1];
+            }
+          }
+        }
+        if (nin) __syncthreads();
+        for (int task = tid; task < T * R1; task += NT) {
+          const int c = task % T, k1 = task / T, q = tile * T + c;
+          if (q >= PL) continue;
+          const int ky = q / NH, kz = q - ky * NH;
+          const int wy = wavenum(ky, N), wz = wavenum(kz, N);
+          const R mult = (kz == 0 || kz == NQ) ? (R)1 : (R)2;
+          C* sl = buf + k1 * R2 * T + c;
+          auto at = [&](int k2) { return (k1 + R1 * k2) * PL + q; };
+          auto pm = [&](int k2) {
+            if constexpr (FX)
+              return A.pf[at(k2)];
+            else
+              return pc_mult<R>(pcc, wavenum(k1 + R1 * k2, N), wy, wz);
+          };
+          // what a step does at one spectrum element: d = the forward x transform's result (the
+          // divergence for two inputs); returns the value that is transformed back
+          auto element = [&](int k2, C d) -> C {
+            const int e = at(k2);
+            switch (step) {
+              case PS_SPEC:
+              case PS_ENTER:
+                ch[e] = d;
+                return cmk<C>(d.x * invN, d.y * invN);
+              case PS_OPEN: {
+                const C c = ch[e];
+                return cmk<C>(c.x * invN, c.y * invN);
+              }
+              case PS_SMOOTH:
+                return cmul2(d, A.mulk[e]);
+              case PS_SETUP: {
+                const C av = ch[e];
+                const R br = av.x + a_cn * d.x, bi = av.y + a_cn * d.y;
+                const R rr = (R)2 * a_cn * d.x, ri = (R)2 * a_cn * d.y;
+                const R P = pm(k2), r2 = rr * rr + ri * ri;
+                acc[0].add(mult * P * P * (br * br + bi * bi));
+                acc[1].add(mult * P * P * r2);
+                acc[2].add(mult * P * r2);
+                if (A.cx) {
+                  const C xv = A.cx[e];
+                  acc[3].add(mult * (xv.x * d.x + xv.y * d.y));
+                }
+                xh[e] = cmk<C>(av.x * invN, av.y * invN);
+                rh[e] = cmk<C>(rr, ri);
+                const C p = cmk<C>(rr * P, ri * P);  // the first direction
+                ph[e] = p;
+                acc[4].add(mult * (p.x * p.x + p.y * p.y));
+                return cmk<C>(p.x * invN, p.y * invN);
+              }
+              case PS_UPDATE: {
+                const C p = ph[e], xv = xh[e], rv = rh[e];
+                const R wr = p.x - a_cn * d.x, wi = p.y - a_cn * d.y;
+                const C rn = cmk<C>(rv.x - al * wr, rv.y - al * wi);
+                xh[e] = cmk<C>(xv.x + alN * p.x, xv.y + alN * p.y);
+                rh[e] = rn;
+                const R P = pm(k2), m2 = mult * (rn.x * rn.x + rn.y * rn.y);
+                acc[0].add(P * P * m2);
+                acc[1].add(P * m2);
+                return d;
+              }
+              case PS_DIR: {
+                const C rv = rh[e], po = ph[e];
+                const R P = pm(k2);
+                const C p = cmk<C>(rv.x * P + bc * po.x, rv.y * P + bc * po.y);
+                ph[e] = p;
+                acc[0].add(mult * (p.x * p.x + p.y * p.y));
+                return cmk<C>(p.x * invN, p.y * invN);
+              }
+              case PS_LEAVE:
+                return xh[e];
+              case PS_APPLY:
+                return cmk<C>(d.x * invN, d.y * invN);
+              default: {  // PS_DOT
+                const C xv = A.cx[e];
+                acc[0].add(mult * (xv.x * d.x + xv.y * d.y));
+                return d;
+              }
+            }
+          };
+          if constexpr (FX) {
+            if (nin) fx_task2<R2, N>(sl, T, 2 * T, sl, T, 2 * T, nullptr, 0, FX_FWD, 0, 0);
+            if (nin == 2)
+              fx_task2<R2, N>(sl + TILE, T, 2 * T, sl + TILE, T, 2 * T, nullptr, 0, FX_FWD,
+                              0, 0);
+#pragma unroll 2
+            for (int k2 = 0; k2 < R2; k2++) {
+              C d = sl[k2 * T];
+              if (nin == 2) d = cadd(cimul<C>((R)wavenum(k1 + R1 * k2, N), d), sl[TILE + k2 * T]);
+              sl[k2 * T] = element(k2, d);
+            }
+            if (nout == 2)
+              fx_task2<R2, N>(sl, T, 2 * T, sl + TILE, T, 2 * T, twA + k1 * R2, 1, FX_IW, k1, R1);
+            if (nout) fx_task2<R2, N>(sl, T, 2 * T, sl, T, 2 * T, twA + k1 * R2, 1, 0, 0, 0);
+            continue;
+          } else {
+          C d[R2];
+          if (nin) {
+#pragma unroll
+            for (int b = 0; b < R2; b++) d[b] = sl[b * T];
+            K::template dft<R2, -1>(d);  // x wave number k1 + R1 k2
+          }
+          if (nin == 2) {
+#pragma unroll
+            for (int k2 = 0; k2 < R2; k2++) d[k2] = cimul<C>((R)wavenum(k1 + R1 * k2, N), d[k2]);
+            C y[R2];
+#pragma unroll
+            for (int b = 0; b < R2; b++) y[b] = sl[TILE + b * T];
+            K::template dft<R2, -1>(y);
+#pragma unroll
+            for (int k2 = 0; k2 < R2; k2++) d[k2] = cadd(d[k2], y[k2]);
+          }
+#pragma unroll
+          for (int k2 = 0; k2 < R2; k2++) d[k2] = element(k2, d[k2]);
+          if (nout == 2) {
+            C g[R2];
+#pragma unroll
+            for (int k2 = 0; k2 < R2; k2++) g[k2] = d[k2];
+            K::template dft_iw_tw<R2, +1>(
+                g, [&](int k2) { return wavenum(k1 + R1 * k2, N); },
+                [&](int b) { return twA[k1 * R2 + b]; });
+#pragma unroll
+            for (int b = 0; b < R2; b++) sl[TILE + b * T] = g[b];
+          }
+          if (nout) {
+            K::template dft_tw<R2, +1, false>(d, [&](int b) { return twA[k1 * R2 + b]; });
+#pragma unroll
+            for (int b = 0; b < R2; b++) sl[b * T] = d[b];
+          }
+          }
+        }
+        __syncthreads();
+        for (int i = 0; i < nout; i++) {  // inverse, second part: rows x = b + R2 a
+          for (int task = tid; task < T * R2; task += NT) {
+            const int c = task % T, b = task / T, q = tile * T + c;
+            if (q >= PL) continue;
+            C* dst = Gp + (1 - i) * S + q;  // i = 0: G_0, i = 1: G_x
+            if constexpr (FX) {
+              fx_task1<R1, N>(buf + i * TILE + b * T + c, nullptr, R2 * T, dst + b * PL, R2 * PL,
+                              nullptr, 0, 0, 0, 0);
+            } else {
+            C u[R1];
+#pragma unroll
+            for (int k1 = 0; k1 < R1; k1++) u[k1] = buf[i * TILE + (k1 * R2 + b) * T + c];
+            K::template dft<R1, +1>(u);
+#pragma unroll
+            for (int a = 0; a < R1; a++) dst[(b + R2 * a) * PL] = u[a];
+            }
+          }
+        }
+        if (nout) __syncthreads();
+      }
+      if (step == PS_SETUP) {
+        const double v[5] = {acc[0].value(), acc[1].value(), acc[2].value(), acc[3].value(),
+                             acc[4].value()};
+        partials(v, 5, 1);
+      } else if (step == PS_UPDATE || step == PS_DOT) {
+        const double v[2] = {acc[0].value(), acc[1].value()};
+        partials(v, 2, 2);
+      } else if (step == PS_DIR) {
+        const double v[1] = {acc[0].value()};
+        partials(v, 1, 0);
+      }
+    }
+    if (step == PS_SPEC || (Geo_::SPLIT ? step == PS_LINE && kind == PS_BACK : step == PS_BACK))
+      break;
+    if (!bar.sync(&A.sc->dev_fault)) return;
+
+    // ---------------------------------------------------------------------- the next step
+    if constexpr (Geo_::SPLIT) {  // FWD: line, y; GRAD: y, line, y; BACK: y, line
+      if (step == PS_YINV) {
+        step = PS_LINE;
+        continue;
+      }
+      if (step == PS_LINE) {
+        step = PS_YFWD;
+        continue;
+      }
+      if (step == PS_YFWD) step = kind;
+    }
+    switch (step) {
+      case PS_FWD:
+        step = A.prog == PP_SPEC ? PS_SPEC : A.prog == PP_SMOOTH ? PS_SMOOTH : PS_ENTER;
+        break;
+      case PS_ENTER:
+      case PS_OPEN:
+        step = PS_GRAD;
+        break;
+      case PS_GRAD:
+        step = A.prog == PP_APPLY ? PS_APPLY
+               : A.prog == PP_DOT ? PS_DOT
+               : started          ? PS_UPDATE
+                                  : PS_SETUP;
+        break;
+      case PS_SETUP:
+        started = true;
+        totals(5, 1);
+        if (tid == 0) {
+          double snorm = tot[0] * dinvN;
+          cg.dp = tot[1] * dinvN;
+          if (snorm == 0.0) snorm = cg.dp;
+          cg.rnorm0 = snorm;
+          cg.ttol = fmax(A.rtol * A.rtol * snorm, A.abstol * A.abstol);
+          cg.beta = tot[2] * dinvN;
+          cg.pp = tot[4];
+          cg.status = converged(cg.dp);
+          if (cg.status == 0 && cg.beta == 0.0) {
+            cg.status = 2;
+            cg.it = 1;
+          }
+          if (A.cx && blockIdx.x == 0) A.sc->acc[6] += A.kdot_weight * tot[3] * dinvN;
+          cg.step = cg.status == 0 ? PS_GRAD : PS_LEAVE;
+        }
+        __syncthreads();
+        step = cg.step;
+        break;
+      case PS_UPDATE:
+        totals(2, 2);
+        if (tid == 0) {
+          cg.dp = tot[0] * dinvN;
+          cg.status = converged(cg.dp);
+          if (cg.status == 0) {
+            const double bnew = tot[1] * dinvN;
+            cg.beta = bnew;
+            cg.bcoef = bnew / cg.beta_old;
+            cg.iter++;
+            if (bnew == 0.0) {
+              cg.status = 2;
+              cg.it = cg.iter + 1;
+            } else if (cg.iter >= A.maxit) {
+              cg.status = -3;
+            }
+          }
+          cg.step = cg.status == 0 ? PS_DIR : PS_LEAVE;
+        }
+        __syncthreads();
+        step = cg.step;
+        break;
+      case PS_DIR:
+        step = PS_GRAD;
+        break;
+      case PS_DOT:
+        totals(1, 2);
+        if (blockIdx.x == 0 && tid == 0) A.sc->acc[6] += A.kdot_weight * tot[0] * dinvN;
+        bar.leave();
+        return;
+      default:  // PS_SMOOTH, PS_LEAVE, PS_APPLY
+        step = PS_BACK;
+    }
+    if (step == PS_LEAVE && A.prog == PP_SOLVE_SPEC) break;
+    if constexpr (Geo_::SPLIT) {
+      if (step <= PS_BACK) {
+        kind = step;
+        step = PS_YINV;
+      }
+    }
+  }
+  if ((A.prog == PP_SOLVE || A.prog == PP_SOLVE_SPEC) && blockIdx.x == 0 && tid == 0) {  // outcome and sweep statistics
+    DevScalars* s = A.sc;
+    s->it = cg.it;
+    s->iter = cg.iter;
+    s->dp = sqrt(cg.dp);
+    s->status = cg.status;
+    s->sum_its[A.which] += cg.it;
+    s->nsolves += 1;
+    if (cg.it > s->max_its) s->max_its = cg.it;
+    s->last_dp = s->dp;
+    if (cg.status < 0 && s->err_status == 0) {
+      s->err_status = cg.status;
+      s->err_its = cg.it;
+    }
+  }
+  bar.leave();
+}
+
+template <typename R, int N>
+PlaneKernel plane_entry() {
+  using P = PlaneGeo<R, N>;
+  return PlaneKernel{reinterpret_cast<const void*>(&k_plane<R, N>), P::NT, P::SMEM,
+                     P::XT > 3 * N ? P::XT : 3 * N, P::SPLIT};
+}
+
+}  // namespace glia
