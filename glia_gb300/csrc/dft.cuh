@@ -37,12 +37,34 @@ __host__ __device__ __forceinline__ C cmk(creal_t<C> x, creal_t<C> y) {
   c.y = y;
   return c;
 }
+// float2: one packed instruction (sm_100 and later) instead of two, the same roundings. The z pass at
+// 256^3, bound by instruction issue: 115 -> 108 us (with the sum of k |grad p|^2).
 template <class C>
 __host__ __device__ __forceinline__ C cadd(C a, C b) {
+#ifdef __CUDA_ARCH__
+  if constexpr (std::is_same<C, float2>::value) {
+    float2 r;
+    asm("{.reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n"
+        " add.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+  }
+#endif
   return cmk<C>(a.x + b.x, a.y + b.y);
 }
 template <class C>
 __host__ __device__ __forceinline__ C csub(C a, C b) {
+#ifdef __CUDA_ARCH__
+  if constexpr (std::is_same<C, float2>::value) {
+    float2 r;
+    asm("{.reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n"
+        " sub.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+  }
+#endif
   return cmk<C>(a.x - b.x, a.y - b.y);
 }
 template <class C>

@@ -460,9 +460,9 @@ class Engine final : public EngineBase {
   void d_front(const R* src, R* pdir) {
     if (own_) {  // no cuFFT: x, y, z passes of our own, k multiplied inside the z pass
       GLIA_TIMED(KS_XINV, SB() * (CGDIR ? 5 : 3), launch_xinv<CGDIR>(src, pdir));
-      GLIA_TIMED(KS_YINV, SB() * 2 + FB() * 3, launch_own(0));
-      GLIA_TIMED(KS_ZFUSED, FB() * 7, launch_own(1));
-      GLIA_TIMED(KS_YFWD, FB() * 3 + SB() * 2, launch_own(2));
+      GLIA_TIMED(KS_YINV, SB() * 2 + FB() * 3, launch_own(0, CGDIR));
+      GLIA_TIMED(KS_ZFUSED, FB() * 7, launch_own(1, CGDIR));
+      GLIA_TIMED(KS_YFWD, FB() * 3 + SB() * 2, launch_own(2, CGDIR));
       return;
     }
     if (xpass_) {
@@ -503,21 +503,16 @@ class Engine final : public EngineBase {
       constexpr int MODE = CGDIR ? 1 : 0;
       const int grid = std::min(xres_inv_, pw_blocks_);
       k_xinv<NN, MODE, OUT2><<<grid, 256, xinv_smem_bytes<NN, MODE>(), stream_>>>(
-          g_, src, pdir, G, sc_, tw256_);
+          g_, src, pdir, G, sc_, ws_, tw256_);
     }
   }
   template <bool CGDIR>
   void launch_xinv(const R* src, R* pdir) {
     const int n = g_.n;
-    if (own_) {
-      if (n == 256) xinv_n<256, CGDIR, true>(src, pdir, g3r_);
-      else if (n == 128) xinv_n<128, CGDIR, true>(src, pdir, g3r_);
-      else xinv_n<64, CGDIR, true>(src, pdir, g3r_);
-    } else {
-      if (n == 256) xinv_n<256, CGDIR, false>(src, pdir, g3s_);
-      else if (n == 128) xinv_n<128, CGDIR, false>(src, pdir, g3s_);
-      else xinv_n<64, CGDIR, false>(src, pdir, g3s_);
-    }
+    if (own_) xinv_n<256, CGDIR, true>(src, pdir, g3r_);
+    else if (n == 256) xinv_n<256, CGDIR, false>(src, pdir, g3s_);
+    else if (n == 128) xinv_n<128, CGDIR, false>(src, pdir, g3s_);
+    else xinv_n<64, CGDIR, false>(src, pdir, g3s_);
   }
   template <int NN, int EPI, bool IN2>
   void xfwd_n(const R* G, const R* aux_in, const R* cx, R* out, R* aux_out, R scale, int blocks) {
@@ -535,10 +530,8 @@ class Engine final : public EngineBase {
     const int n = g_.n;
     blocks = std::min(xres_fwd_, blocks);
     if (own_) {
-      if (n == 256) xfwd_n<256, EPI, true>(g3r_, aux_in, cx, out, aux_out, scale, blocks);
-      else if (n == 128) xfwd_n<128, EPI, true>(g3r_, aux_in, cx, out, aux_out, scale, blocks);
-      else xfwd_n<64, EPI, true>(g3r_, aux_in, cx, out, aux_out, scale, blocks);
-    } else {
+      xfwd_n<256, EPI, true>(g3r_, aux_in, cx, out, aux_out, scale, blocks);
+    } else if constexpr (EPI != EPI_CGU) {
       if (n == 256) xfwd_n<256, EPI, false>(g3s_, aux_in, cx, out, aux_out, scale, blocks);
       else if (n == 128) xfwd_n<128, EPI, false>(g3s_, aux_in, cx, out, aux_out, scale, blocks);
       else xfwd_n<64, EPI, false>(g3s_, aux_in, cx, out, aux_out, scale, blocks);
@@ -546,34 +539,28 @@ class Engine final : public EngineBase {
   }
   // own y / z passes: 0 = y inverse (g3r_ -> g3s_), 1 = z pass (g3s_ in place, k), 2 = k_yfwd
   // (g3s_ -> g3r_)
-  template <int NN>
-  void own_n(int which) {
+  // dot: the z pass also sets alpha (PCG iterations)
+  void launch_own(int which, bool dot) {
     if constexpr (std::is_same<R, float>::value) {
+      constexpr int NN = 256;
+      const int grid = std::min(own_res_[which], pw_blocks_);
       if (which == 0 && yinv_bulk_)
-        k_yinv_bulk<NN><<<std::min(own_res_[0], pw_blocks_), 256, yinv_bulk_smem_bytes<NN>(),
-                          stream_>>>(g3r_, g3s_, tw256_, sc_);
+        k_yinv_bulk<NN><<<grid, 256, yinv_bulk_smem_bytes<NN>(), stream_>>>(g3r_, g3s_, tw256_,
+                                                                             sc_);
       else if (which == 0)
-        k_yinv<NN><<<std::min(own_res_[0], pw_blocks_), 256, yinv_smem_bytes<NN>(), stream_>>>(
-            g3r_, g3s_, tw256_);
-      else if (which == 1 && zpass2_)
-        k_zpass2<NN><<<std::min(own_res_[1], pw_blocks_), 256, zpass2_smem_bytes<NN>(),
-                       stream_>>>(g3s_, kxx_, tw256_, zrev_);
+        k_yinv<NN><<<grid, 256, yinv_smem_bytes<NN>(), stream_>>>(g3r_, g3s_, tw256_);
+      else if (which == 1 && dot)
+        k_zpass2<NN, true><<<std::min(grid, red_blocks_), 256, zpass2_smem_bytes<NN>(), stream_>>>(
+            g3s_, kxx_, tw256_, zrev_, sc_, ws_, g_.invN);
       else if (which == 1)
-        k_zpass<NN><<<std::min(own_res_[1], pw_blocks_), 256, zpass_smem_bytes<NN>(), stream_>>>(
-            g3s_, kxx_, tw256_);
+        k_zpass2<NN, false><<<grid, 256, zpass2_smem_bytes<NN>(), stream_>>>(
+            g3s_, kxx_, tw256_, zrev_, sc_, ws_, g_.invN);
       else if (tma_)
-        k_yfwd_tma<NN><<<std::min(own_res_[2], pw_blocks_), 256, yfwd_tma_smem_bytes<NN>(),
-                         stream_>>>(kmap_, g3r_, tw256_, sc_);
+        k_yfwd_tma<NN><<<grid, 256, yfwd_tma_smem_bytes<NN>(), stream_>>>(kmap_, g3r_, tw256_,
+                                                                           sc_);
       else
-        k_yfwd<NN><<<std::min(own_res_[2], pw_blocks_), 256, yfwd_smem_bytes<NN>(), stream_>>>(
-            g3s_, g3r_, tw256_);
+        k_yfwd<NN><<<grid, 256, yfwd_smem_bytes<NN>(), stream_>>>(g3s_, g3r_, tw256_);
     }
-  }
-  void launch_own(int which) {
-    const int n = g_.n;
-    if (n == 256) own_n<256>(which);
-    else if (n == 128) own_n<128>(which);
-    else own_n<64>(which);
   }
   // resident CTAs of the x-pass and own-transform kernels on this device (persistent grids:
   // every CTA walks the same number of tiles to within one)
@@ -587,31 +574,27 @@ class Engine final : public EngineBase {
         GLIA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, 256, smem));
         return std::max(1, std::min(b, kMaxRedBlocksPerSm));
       };
-      if (own_) {
+      if constexpr (NN == 256) if (own_) {
         xres_inv_ = sms_ * std::min(per_sm(k_xinv<NN, 0, true>, xinv_smem_bytes<NN, 0>()),
                                     per_sm(k_xinv<NN, 1, true>, xinv_smem_bytes<NN, 1>()));
         constexpr int fs = xfwd_own_smem_bytes<NN>();
         xres_fwd_ = sms_ * std::min({per_sm(k_xfwd_own<NN, EPI_APPLYD>, fs),
                                      per_sm(k_xfwd_own<NN, EPI_SETUP>, fs),
-                                     per_sm(k_xfwd_own<NN, EPI_CGW>, fs)});
+                                     per_sm(k_xfwd_own<NN, EPI_CGU>, fs)});
         // y-inverse rows staged by bulk copies (default) or per-thread cp.async
         // (GLIA_YINV_BULK=0)
         const char* yb = std::getenv("GLIA_YINV_BULK");
         yinv_bulk_ = !(yb && yb[0] == '0');
         own_res_[0] = sms_ * (yinv_bulk_ ? per_sm(k_yinv_bulk<NN>, yinv_bulk_smem_bytes<NN>())
                                          : per_sm(k_yinv<NN>, yinv_smem_bytes<NN>()));
-        // z pass: two real lines per complex transform (k_zpass2) unless GLIA_ZPASS2=0 picks
-        // the even/odd half-length version (k_zpass)
-        const char* z2 = std::getenv("GLIA_ZPASS2");
-        zpass2_ = !(z2 && z2[0] == '0');
         // z pass over its line blocks in descending order (default; GLIA_ZREV=0 ascending): the
         // y-inverse pass before it writes the lines in ascending order, so the z pass starts on
         // the lines still in L2, and the y-forward pass after it (ascending) starts on the lines
         // the z pass wrote last
         const char* zr = std::getenv("GLIA_ZREV");
         zrev_ = !(zr && zr[0] == '0');
-        own_res_[1] = sms_ * (zpass2_ ? per_sm(k_zpass2<NN>, zpass2_smem_bytes<NN>())
-                                      : per_sm(k_zpass<NN>, zpass_smem_bytes<NN>()));
+        own_res_[1] = sms_ * std::min(per_sm(k_zpass2<NN, false>, zpass2_smem_bytes<NN>()),
+                                      per_sm(k_zpass2<NN, true>, zpass2_smem_bytes<NN>()));
         const char* te = std::getenv("GLIA_TMA");
         tma_ = te && te[0] == '1';
         own_res_[2] = sms_ * (tma_ ? per_sm(k_yfwd_tma<NN>, yfwd_tma_smem_bytes<NN>())
@@ -620,7 +603,9 @@ class Engine final : public EngineBase {
         // 2T floats x n rows (used by k_yfwd<TMA = true>, GLIA_TMA=1)
         if (tma_)
           kmap_ = make_tmap_f32_2d(g3s_, (uint64_t)NN, 3ull * NN * NN, 2 * YDecomp<NN>::T, NN);
-      } else {
+        return;
+      }
+      {
         xres_inv_ = sms_ * std::min(per_sm(k_xinv<NN, 0, false>, xinv_smem_bytes<NN, 0>()),
                                     per_sm(k_xinv<NN, 1, false>, xinv_smem_bytes<NN, 1>()));
         xres_fwd_ = sms_ * std::min({per_sm(k_xfwd<NN, EPI_APPLYD>, 0),
@@ -633,6 +618,11 @@ class Engine final : public EngineBase {
   // one PCG iteration of the fused engine (launched directly, or captured as the loop body)
   void cg_iteration() {
     d_front<true>(rhat_, phat_);  // p = P r + b p and the spectra of k grad p
+    if (own_) {  // alpha is known: w = A p and the update of x and r in one pass
+      GLIA_TIMED(KS_XFWD_CGU, SB() * 7,
+                 launch_xfwd<EPI_CGU>(phat_, rhat_, xhat_, rhat_, R(0), red_blocks_));
+      return;
+    }
     d_back<EPI_CGW>(phat_, nullptr, what_, nullptr, R(0));  // w = A p, <p, w>, alpha
     GLIA_TIMED(KS_CG_UPDATE, SB() * 6,
                k_cg_update<R><<<red_blocks_, kThreads, 0, stream_>>>(g_, xhat_, phat_, rhat_,
@@ -2590,7 +2580,6 @@ class Engine final : public EngineBase {
   CUtensorMap kmap_{};               // TMA map of the packed line arrays (k_yfwd)
   bool tma_ = false;                 // k_yfwd stages with TMA copies (GLIA_TMA=1)
   bool zrev_ = true;                 // k_zpass2 line blocks in descending order
-  bool zpass2_ = true;               // z pass with two real lines per complex transform
   bool yinv_bulk_ = true;            // y-inverse rows staged by bulk copies
   bool own_ = false;  // own y and z passes (x pass on): no cuFFT inside the D apply
   // graph-captured evaluations (eval_prepare / eval_capture / eval_finish)

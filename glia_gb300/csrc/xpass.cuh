@@ -152,12 +152,12 @@ __device__ __forceinline__ void xdft(float2* sm, const float2* twb, int c, int g
 // so two x transforms give the three components: G_x = F^-1(i w_x u) / N and
 // G_y, G_z = i w_y, i w_z F^-1(u) / N. The inputs of the CTA's next tile are staged into shared
 // memory (cp.async) while the current tile is transformed.
-// OUT2 (own y / z passes): two arrays out, [G_x, G_0] with G_0 = F^-1(u) / N; otherwise three,
+// OUT2 (own y / z passes): in MODE 1 also sum |p|^2 (DevScalars::pp); two arrays out, [G_x, G_0] with G_0 = F^-1(u) / N; otherwise three,
 // [G_x, G_y, G_z].
 template <int NN, int MODE, bool OUT2>
 __global__ void __launch_bounds__(256, 2)
     k_xinv(Geo g, const float* __restrict__ src, float* __restrict__ pdir, float* __restrict__ G3,
-           const DevScalars* __restrict__ sc, const float2* __restrict__ tw_g) {
+           DevScalars* __restrict__ sc, RedWs ws, const float2* __restrict__ tw_g) {
   using D = XDecomp<NN>;
   constexpr int R1 = D::R1, R2 = D::R2, T = D::T, GR = 256 / T;
   constexpr int NB1 = R2 / GR;
@@ -186,11 +186,13 @@ __global__ void __launch_bounds__(256, 2)
     cp_async_commit();
   };
   stage(blockIdx.x);
+  Acc<float> pp;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     cp_async_wait<0>();
     __syncthreads();
     const XCol col = xcol(g, tile * T + c);
     float2 v[NB1][R1];
+    float pl = 0.f;  // the tile's few positive terms, then compensated
 #pragma unroll
     for (int m = 0; m < NB1; m++) {
       const int b = gi + GR * m;
@@ -208,10 +210,12 @@ __global__ void __launch_bounds__(256, 2)
             val.y += bc * po.y;
           }
           P[kx * plane + col.q] = val;
+          if (OUT2) pl = fmaf(val.x, val.x, fmaf(val.y, val.y, pl));
         }
         v[m][a] = val;
       }
     }
+    if (MODE == 1 && OUT2) pp.add(col.mult * pl);
     __syncthreads();  // slots read: stage the next tile behind the transforms
     stage(tile + gridDim.x);
     xdft<D, +1>(
@@ -240,6 +244,10 @@ __global__ void __launch_bounds__(256, 2)
     }
   }
   cp_async_wait<0>();
+  if constexpr (MODE == 1 && OUT2) {
+    double sums[1] = {pp.value()};
+    if (grid_sum_last<1>(sums, ws) && threadIdx.x == 0) sc->pp = sums[0];
+  }
 }
 
 // Epilogue of the forward x pass for one output element (k_spec_div semantics): d = the
@@ -277,10 +285,14 @@ __device__ __forceinline__ void xfwd_finish(Acc<float> (&acc)[4], Geo g, DevScal
     double sums[4] = {acc[0].value(), acc[1].value(), acc[2].value(), acc[3].value()};
     if (!grid_sum_last<4>(sums, ws)) return;
     if (threadIdx.x == 0) div_setup_finish(sums, sc, g.invN, has_cx);
+  } else if constexpr (EPI == EPI_CGU) {
+    double sums[2] = {acc[0].value(), acc[1].value()};
+    if (!grid_sum_last<2>(sums, ws)) return;
+    if (threadIdx.x == 0) cg_update_finish(sums, sc, g.invN);
   } else if constexpr (EPI == EPI_CGW) {
     double sums[1] = {acc[0].value()};
     if (!grid_sum_last<1>(sums, ws)) return;
-    if (threadIdx.x == 0) div_cgw_finish(sums[0], sc, g.invN);
+    if (threadIdx.x == 0) cg_alpha(sums[0] * g.invN, sc);
   }
 }
 
@@ -358,10 +370,16 @@ constexpr int xfwd_own_smem_bytes() {
 }
 
 // Forward x pass of the own-transform path: M = [M_x, M_r] in the half-spectrum layout,
-// divergence i w_x F_x M_x + F_x M_r, epilogue of k_spec_div. The CTA's inputs form a stream of
-// items (M_x, M_r and the epilogue's spectra of its first tile, then of the next, ...) through
-// two shared-memory slots: item i sits in slot i % 2 and, once consumed, its slot receives item
-// i + 2 (cp.async).
+// divergence i w_x F_x M_x + F_x M_r, and the epilogue: EPI_APPLYD and EPI_SETUP as k_spec_div;
+// EPI_CGU the whole PCG update, w = p - a D p, x' += (alpha / N) p, r -= alpha w, ||z||^2 and
+// <z, r> (aux_in = p, cx = r in and aux_out = r out, out = x'). alpha is known here because the z
+// pass has summed k |grad p|^2 (k_zpass2): w is never stored, and the update needs no pass of its
+// own (7 spectra moved instead of 4 + 6). Measured at 256^3: 98 us instead of 64 + 67; the two sums
+// behind alpha cost the z pass 12 us and the x inverse 8 (one more grid-wide reduction in all, a few
+// microseconds of tail each); a gradient evaluation of 20 steps 196.5 -> 191.8 ms.
+// The CTA's inputs form a stream of items (M_x, M_r and the epilogue's spectra of its first tile,
+// then of the next, ...) through two shared-memory slots: item i sits in slot i % 2 and, once
+// consumed, its slot receives item i + 2 (cp.async). EPI_CGU reads x' straight from global memory.
 template <int NN, int EPI>
 __global__ void __launch_bounds__(256, 2)
     k_xfwd_own(Geo g, const float* __restrict__ M2, const float* __restrict__ aux_in,
@@ -375,7 +393,7 @@ __global__ void __launch_bounds__(256, 2)
   float2* slots = reinterpret_cast<float2*>(xfwd_dyn);  // 2 x NN * T
   float2* sm = slots + 2 * NN * T;
   float2* tw = sm + NN * T;
-  if (EPI == EPI_CGW && sc->status != 0) return;
+  if (EPI == EPI_CGU && sc->status != 0) return;
   fill_twb<D, -1>(tw, tw_g);
   const int c = threadIdx.x % T, gi = threadIdx.x / T;
   const int plane = NN * g.nh, Ns = plane * NN;
@@ -383,13 +401,15 @@ __global__ void __launch_bounds__(256, 2)
   const float a = EPI == EPI_APPLYD ? 0.f : (float)sc->a_cn;
   const float pcc = (float)sc->pc_c;
   const float invN = (float)g.invN;
+  const float al = EPI == EPI_CGU ? (float)sc->alpha : 0.f;
+  const float alN = EPI == EPI_CGU ? (float)(sc->alpha * g.invN) : 0.f;
   const float2* Mx = reinterpret_cast<const float2*>(M2);
   const float2* Mr = Mx + Ns;
   const float2* AX = reinterpret_cast<const float2*>(aux_in);
   const float2* CX = reinterpret_cast<const float2*>(cx);
   float2* O = reinterpret_cast<float2*>(out);
   float2* AO = reinterpret_cast<float2*>(aux_out);
-  const int naux = EPI == EPI_APPLYD ? 0 : (EPI == EPI_SETUP && CX ? 2 : 1);
+  const int naux = EPI == EPI_APPLYD ? 0 : (EPI == EPI_CGU || (EPI == EPI_SETUP && CX) ? 2 : 1);
   const int NI = 2 + naux;
   const int mytiles =
       (int)blockIdx.x < ntiles ? (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x
@@ -446,11 +466,30 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
     for (int m2 = 0; m2 < NB2; m2++) {
       const int k1 = gi + GR * m2;
+      constexpr int XH = 8;  // x' values in flight per thread
+      float2 xo[XH];
 #pragma unroll
       for (int k2 = 0; k2 < R2; k2++) {
         const int kx = k1 + R1 * k2;
+        if (EPI == EPI_CGU && k2 % XH == 0) {
+#pragma unroll
+          for (int i = 0; i < XH; i++) xo[i] = O[(kx + R1 * i) * plane + col.q];
+        }
         const float2 av = naux ? SA[kx * T + c] : make_float2(0.f, 0.f);
         const float2 xv = naux == 2 ? SX[kx * T + c] : make_float2(0.f, 0.f);
+        if constexpr (EPI == EPI_CGU) {
+          const float2 d = dsum[m2][k2];
+          const int idx = kx * plane + col.q;
+          const float wr = av.x - a * d.x, wi = av.y - a * d.y;
+          const float2 r = make_float2(xv.x - al * wr, xv.y - al * wi);
+          const float pm = pc_mult<float>(pcc, wavenum(kx, NN), col.wy, col.wz);
+          const float mr2 = col.mult * (r.x * r.x + r.y * r.y);
+          acc[0].add(pm * pm * mr2);
+          acc[1].add(pm * mr2);
+          AO[idx] = r;
+          O[idx] = make_float2(xo[k2 % XH].x + alN * av.x, xo[k2 % XH].y + alN * av.y);
+          continue;
+        }
         xfwd_epilogue<NN, EPI>(dsum[m2][k2], kx, kx * plane + col.q, col, a, pcc, invN, scale, av,
                                xv, naux == 2, O, AO, acc);
       }

@@ -160,10 +160,13 @@ __device__ __forceinline__ void pair_line(float2* E0, float2* E1, const float4* 
 // rev: blocks in descending order. The y-inverse pass writes the lines in ascending order and
 // the y-forward pass reads them in ascending order, so in descending order the z pass starts on
 // the lines still in L2 and ends on the ones the y-forward pass reads first.
-template <int NN>
+// DOT: sums k |grad p|^2 over the grid on the way and, with sum |p|^2 from k_xinv, sets alpha of
+// the PCG step: <p, A p> = sum p^2 + a sum k |grad p|^2, the derivatives being skew-symmetric.
+template <int NN, bool DOT>
 __global__ void __launch_bounds__(256, 2)
     k_zpass2(float* __restrict__ Hio, const float* __restrict__ kf,
-             const float2* __restrict__ tw_g, bool rev) {
+             const float2* __restrict__ tw_g, bool rev, DevScalars* __restrict__ sc, RedWs ws,
+             double invN) {
   using Z = Z2Geom<NN>;
   constexpr int R1 = Z::R1, R2 = Z::R2, KPT = Z::KPT, NQ = Z::NQ, LB = Z::LB, LS = Z::LS;
   constexpr int NP = NN * NN * NQ, PS = Z::PS;
@@ -199,6 +202,7 @@ __global__ void __launch_bounds__(256, 2)
   issue(0);
   issue(1);
   issue(2);
+  Acc<float> dot;
   float kv[2][KPT][R2];  // k of lines l0, l1 at t + R2 ii + R1 k2
   for (int b = 0; b < nblk; b++) {
     const int i0 = 4 * b, bi = (int)blockIdx.x + b * (int)gridDim.x;
@@ -243,12 +247,15 @@ __global__ void __launch_bounds__(256, 2)
         }
       }
       float2* OX = Hc + (size_t)(blk * LB + l) * NQ;
+      float dl = 0.f;  // this line's positive terms, then compensated
       float2* OY = OX + NP;
       pair_line<NN>(
           X + sh, Y + sh, twr, t, u,
           [&](int ii, int k2, float2 z) {
             const float kk = kv[j][ii][k2];
-            return make_float2(z.x * kk, z.y * kk);
+            const float2 s = make_float2(z.x * kk, z.y * kk);
+            if (DOT) dl = fmaf(s.x, z.x, fmaf(s.y, z.y, dl));
+            return s;
           },
           [&](int ii, int k2, float2 A, float2 B) {
             const int q = t + R2 * ii + R1 * k2;
@@ -262,6 +269,7 @@ __global__ void __launch_bounds__(256, 2)
             OX[q] = A;
             OY[q] = B;
           });
+      if (DOT) dot.add(dl);
     }
     __syncthreads();
     issue(i0 + 4);
@@ -292,10 +300,13 @@ __global__ void __launch_bounds__(256, 2)
       }
       float2* O0 = Hc + (size_t)2 * NP + (size_t)(blk * LB + l0) * NQ;
       float2* O1 = O0 + NQ;
+      float dl = 0.f;
       pair_line<NN>(
           P0 + sh, P1 + sh, twr, t, u,
           [&](int ii, int k2, float2 z) {
-            return make_float2(z.x * kv[0][ii][k2], z.y * kv[1][ii][k2]);
+            const float2 s = make_float2(z.x * kv[0][ii][k2], z.y * kv[1][ii][k2]);
+            if (DOT) dl = fmaf(s.x, z.x, fmaf(s.y, z.y, dl));
+            return s;
           },
           [&](int ii, int k2, float2 A, float2 B) {
             const int q = t + R2 * ii + R1 * k2;
@@ -303,11 +314,17 @@ __global__ void __launch_bounds__(256, 2)
             O0[q] = make_float2(-w * A.y, w * A.x);
             O1[q] = make_float2(-w * B.y, w * B.x);
           });
+      if (DOT) dot.add(dl);
     }
     __syncthreads();
     issue(i0 + 6);
   }
   cp_async_wait<0>();
+  if constexpr (DOT) {
+    double sums[1] = {dot.value()};
+    if (grid_sum_last<1>(sums, ws) && threadIdx.x == 0)
+      cg_alpha(sc->pp * invN + sc->a_cn * sums[0], sc);
+  }
 }
 
 }  // namespace glia
