@@ -4,12 +4,18 @@
 // instruction in each sub-partition), 64-bit integer add 58, the upper half of a 64 x 64-bit
 // product 6, conversions between FP64 and any other type 2. A DFT of R values is therefore taken
 // in block fixed point: the R inputs are aligned to the largest exponent among them, with
-// log2 R + 2 bits of headroom (57 bits of magnitude at R = 16, where a double has 53), the
-// butterflies run on integers, and each result is rounded once to a double; the conversions too
-// are integer code. No precision is given up: a butterfly in FP64 rounds to 53 bits at every step,
-// this once. Against long double, root mean square over a 16-point DFT: 5.3e-17 of the result's
-// 2-norm instead of 1.0e-16; D apply at 64^3 4.9e-16 instead of 1.3e-15 with cuFFT's FP64
-// transforms (white noise: 1.8e-16 instead of 6.8e-16).
+// log2 R + 2 bits of headroom (57 bits of magnitude at R = 16, where a double has 53), and the
+// butterflies run on integers. Between two DFTs of the same phase the values stay integers with an
+// exponent (memory blocks, below); doubles are made only where a phase needs them: 182 -> about 80
+// instructions per value and DFT, solve at 128^3 1.48 -> 1.0 ms.
+//
+// No precision is given up. A butterfly in FP64 rounds to 53 bits at every step, this keeps 57
+// below a block's largest value. Against long double, root mean square of the error relative to the
+// result: a 16-point DFT rounded to doubles 5.3e-17 (FP64 arithmetic 1.0e-16); D apply at 64^3
+// 4.0e-16 (cuFFT's FP64 transforms 1.3e-15), of white noise 2.2e-16 (6.8e-16). Fifty trips to the
+// spectrum and back change a smooth field's amplitude by 1e-20 to 4e-18 each (1e-16 to 3e-16 with
+// cuFFT): what rounding down takes away is given back (fx_transform), and a factor 1 is not a
+// multiplication. A 32^3 simulation of 20 steps: 2.0e-15 off long double, with cuFFT 7.6e-15.
 //
 // A block whose largest magnitude is below 2^-952 is taken as zero; one that holds a NaN, an
 // infinity or a magnitude above 2^1017 gives NaN.
@@ -274,6 +280,11 @@ GLIA_HD constexpr int fx_log2(int r) {
   return r <= 1 ? 0 : r <= 2 ? 1 : r <= 5 ? 2 : r <= 11 ? 3 : 4;
 }
 
+// Bits of a task's block: one more of headroom for the sums of a task (pairs, two inputs), and 58
+// at most (fx_get_iw; the shift into a block drops 5 of the exponent's 6 bits, the sixth is 2^-58
+// of the block's largest value).
+GLIA_HD constexpr int fx_block_bits(int r) { return 61 - fx_log2(r) < 58 ? 61 - fx_log2(r) : 58; }
+
 // results of a block: v 2^(-extra) with the block exponent E of B-bit inputs
 template <int R, int B>
 GLIA_HD void fx_store(const fx2 (&q)[R], double2 (&v)[R], int E, int adj) {
@@ -296,9 +307,81 @@ GLIA_HD int fx_block(const double2 (&v)[R]) {
   return (int)(m >> 20);
 }
 
-// ---- DFT tasks on R doubles ----------------------------------------------------------------
-// The inputs may be multiplied by i w(a) (rot), |w| < 128; results by a table's factors (tw(k),
-// its conjugate where CONJ).
+// ---- blocks in memory ----------------------------------------------------------------------
+// Between tasks a complex value stays in fixed point: value = v 2^(e - 1022 - 63), |v| < 2^63, the
+// exponent e (12 bits, one for all results of a task) in the low 6 bits of re (upper half) and im
+// (lower half). The results of a task are shifted up together until the largest fills the word,
+// so 57 bits below the block's largest value are kept. e = kFxBad marks NaN or overflow.
+enum { kFxBad = 4095 };
+GLIA_HD int fx_e(fx2 v) { return (((int)v.x & 63) << 6) | ((int)v.y & 63); }
+GLIA_HD fx2 fx_with_e(fx2 v, int e) {
+  return cmk<fx2>((v.x & ~(int64_t)63) | (e >> 6), (v.y & ~(int64_t)63) | (e & 63));
+}
+template <int B>
+GLIA_HD int fx_shift(int E, int e) {  // right shift that brings exponent e to a block E of B bits
+  return (int)fx_min((uint32_t)(E - e + 63 - B), 63u);
+}
+// rounds down: half a unit low on average (fx_transform makes up for it)
+template <int B>
+GLIA_HD fx2 fx_get(fx2 v, int E, int e) {
+  const int s = fx_shift<B>(E, e);
+  return cmk<fx2>(v.x >> s, v.y >> s);
+}
+// i w v, |w| < 128, E at least e plus the bits of w
+template <int B>
+GLIA_HD fx2 fx_get_iw(fx2 v, int E, int e, int w) {
+  static_assert(B <= 58, "the product is shifted by 7 less");
+  const int s = (int)fx_min((uint32_t)(E - e + 56 - B), 63u);
+  const int64_t x = ((v.x >> 7) * w) >> s, y = ((v.y >> 7) * w) >> s;
+  return cmk<fx2>(-y, x);
+}
+// exponent of w v (0 for w = 0), at least two above v's, so that the shift is not negative
+GLIA_HD int fx_e_w(int e, int w) {
+  const int a = (w < 0 ? -w : w) | 2;
+#ifdef __CUDA_ARCH__
+  return w == 0 ? 0 : e + 32 - __clz(a);
+#else
+  return w == 0 ? 0 : e + 32 - __builtin_clz((unsigned)a);
+#endif
+}
+// results q 2^(E - 1022 - B + adj) as memory blocks
+template <int R, int B>
+GLIA_HD void fx_put(fx2 (&q)[R], int E, int adj) {
+  uint32_t m = 1;
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+    const int32_t a = (int32_t)(q[i].x >> 32), b = (int32_t)(q[i].y >> 32);
+    m |= (uint32_t)(a ^ (a >> 31)) | (uint32_t)(b ^ (b >> 31));
+  }
+#ifdef __CUDA_ARCH__
+  const int z = __clz(m) - 1;
+#else
+  const int z = __builtin_clz(m) - 1;
+#endif
+  const bool zero = E < kFxTiny;
+  const int e = E > kFxHuge ? kFxBad : zero ? 0 : E - B + adj - z + 63;
+  const int64_t keep = zero ? 0 : ~(int64_t)63;
+#pragma unroll
+  for (int i = 0; i < R; i++)
+    q[i] = cmk<fx2>(((int64_t)((uint64_t)q[i].x << z) & keep) | (e >> 6),
+                    ((int64_t)((uint64_t)q[i].y << z) & keep) | (e & 63));
+}
+// a + i b and (a +- conj b) / 2, (a -+ conj b) / 2i of two blocks
+GLIA_HD fx2 fx_plus_i(fx2 a, fx2 b) {
+  const int ea = fx_e(a), eb = fx_e(b), E = (ea > eb ? ea : eb) + 1;
+  const fx2 p = fx_get<62>(a, E, ea), q = fx_get<62>(b, E, eb);
+  const fx2 r = cmk<fx2>(2 * (p.x - q.y), 2 * (p.y + q.x));
+  return fx_with_e(r, E > kFxHuge ? kFxBad : E);
+}
+GLIA_HD void fx_halves(fx2 a, fx2 b, fx2& s, fx2& d) {
+  const int ea = fx_e(a), eb = fx_e(b), E = ea > eb ? ea : eb;
+  const fx2 p = fx_get<62>(a, E, ea), q = fx_get<62>(b, E, eb);
+  const int e = E > kFxHuge ? kFxBad : E;
+  s = fx_with_e(cmk<fx2>(p.x + q.x, p.y - q.y), e);
+  d = fx_with_e(cmk<fx2>(p.y + q.y, q.x - p.x), e);
+}
+
+// doubles to a block in registers, and |w| times as much
 struct NoTw {};
 template <int R, int S, bool CONJ, class Tw>
 GLIA_HD void fx_twiddled(fx2 (&q)[R], Tw&& tw) {
@@ -321,33 +404,6 @@ template <int B>
 GLIA_HD int fx_exp_w(double2 v, int w) {  // exponent bound of w v, 0 for w = 0
   const int e = (int)(fx_mag(0u, v) >> 20);
   return w == 0 ? 0 : e + fx_wbits<B>(w < 0 ? -w : w);
-}
-
-template <int R, int S, bool CONJ, class Tw>
-GLIA_HD void fx_dft(double2 (&v)[R], Tw&& tw) {
-  constexpr int B = 62 - fx_log2(R);
-  constexpr int adj = std::is_same<std::decay_t<Tw>, NoTw>::value ? 0 : 1;
-  const int E = fx_block(v);
-  fx2 q[R];
-#pragma unroll
-  for (int i = 0; i < R; i++) q[i] = fx_in2<B>(v[i], E);
-  fx_twiddled<R, S, CONJ>(q, tw);
-  fx_store<R, B>(q, v, E, adj);
-}
-template <int R, int S, class W, class Tw>
-GLIA_HD void fx_dft_iw(double2 (&v)[R], W&& w, Tw&& tw) {
-  constexpr int B = 62 - fx_log2(R);
-  int E = 0;
-#pragma unroll
-  for (int i = 0; i < R; i++) {
-    const int e = fx_exp_w<B>(v[i], w(i));
-    E = E > e ? E : e;
-  }
-  fx2 q[R];
-#pragma unroll
-  for (int i = 0; i < R; i++) q[i] = fx_in2_iw<B>(v[i], E, w(i));
-  fx_twiddled<R, S, false>(q, tw);
-  fx_store<R, B>(q, v, E, 1);
 }
 
 }  // namespace glia

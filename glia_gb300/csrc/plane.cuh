@@ -25,9 +25,10 @@
 //   mixed  gradient  32^3, 16 steps   14.5 -> 6.8 ms      64^3, 40 steps   41.6 -> 24.9 ms
 //          forward   96^3, 20 steps   13.9 -> 6.2 ms
 //          gradient 128^3, 40 steps   88.0 -> 84.0 ms
-//   FP64   forward   64^3, 100 steps   151 -> 57 ms
-//          gradient 128^3, 6 steps     168 -> 48 ms
-//          solve    256^3               45 -> 15 ms
+//   FP64   forward   64^3, 100 steps   151 -> 46.5 ms
+//          gradient 128^3, 6 steps     164 -> 34.5 ms
+//          adjoint  120^3, 2 steps    48.7 -> 11.5 ms
+//          solve    256^3               45 -> 10.3 ms
 //
 // N = R1 R2 (R2 a power of two, so that a group of R2 threads is part of a warp). Inverse
 // transforms read index R2 a + b (R1-point DFTs over a, twiddle w^(b k1), R2-point DFTs over b) and
@@ -68,14 +69,16 @@ struct PlaneGeo {
   static constexpr int TC = NQ % 16 == 0 ? 16 : 8;  // SPLIT: columns per block
   static constexpr int PLANE = SPLIT ? 0 : NQ * PS2;
   // columns per tile: about one tile per resident CTA
-  static constexpr int T = N <= 32 ? 4 : N <= 64 ? 8 : N < 112 ? 16 : SPLIT ? 8 : sizeof(R) == 4 ? 28 : 32;
+  static constexpr int T =
+      N <= 32 ? 4 : N <= 64 ? 8 : N < 112 ? 16 : SPLIT ? 8 : sizeof(R) == 4 ? 28 : 32;
   static constexpr int XT = (PL + T - 1) / T;
   static constexpr int TILE = N * T;
   static constexpr int RED = 5 * 512 * 8 / (int)sizeof(C);  // partial sums of a phase
   static constexpr int LINES = SPLIT ? 16 * PS2 : 0;  // one pair of lines per group of R2 lanes
   static constexpr int BUF0 = 2 * TILE > RED ? 2 * TILE : RED;
   static constexpr int BUF1 = PLANE > LINES ? PLANE : LINES, BUF = BUF0 > BUF1 ? BUF0 : BUF1;
-  static constexpr int SMEM = (BUF + 4 * N) * (int)sizeof(C);  // + twiddles twice, kz' = 0 twice
+  // + twiddles twice, kz' = 0 twice, wave numbers
+  static constexpr int SMEM = (BUF + 4 * N + (GAP ? N / 2 : 0)) * (int)sizeof(C);
   static constexpr int MINB = SMEM > 110 * 1024 ? 1 : 2;
   static constexpr int NT = N <= 32 ? 128 : (MINB == 2 ? 256 : 512);
   static constexpr int NW = NT / 32, GPW = 32 / R2, NG = NW * GPW;
@@ -200,100 +203,209 @@ enum FxMode {
   FX_C0 = 32,    // of c = 0: re / im hold the two packed real values of each line
   FX_SUM = 64    // inputs i w0 src(a) + src2(a)
 };
-template <int R, int N, class AtS, class AtD>
-__device__ __forceinline__ void fx_task_body(const double2* src, const double2* src2, double2* dst,
-                                             AtS&& at_s, AtD&& at_d, const FxTw* tw, int twl,
-                                             int mode, int w0, int wl) {
-  constexpr int B = 61 - fx_log2(R);
-  double2 v[R];
+template <int R>
+__device__ __forceinline__ void fx_swap(fx2 (&q)[R], bool swap) {
 #pragma unroll
-  for (int a = 0; a < R; a++) v[a] = src[at_s(a)];
+  for (int a = 0; a < R; a++)
+    q[a] = cmk<fx2>(swap ? q[a].y : q[a].x, swap ? q[a].x : q[a].y);
+}
+// The transform of a block in registers and its twiddles (tw null: all 1); returns the power of two
+// its results lack. Inputs that were
+// rounded down (hx, hy = 1: re, im low by half a unit on average, -1: high) bias result 0 alone,
+// the transform of a constant being R at 0.
+template <int R>
+__device__ __forceinline__ int fx_transform(fx2 (&q)[R], const FxTw* tw, int twl, bool fwd, int hx,
+                                            int hy) {
+  fx_swap(q, fwd);
+  reg_dft<R, +1>(q);
+  q[0].x += (fwd ? hy : hx) * R / 2;
+  q[0].y += (fwd ? hx : hy) * R / 2;
+  if (tw) {
+    q[0] = cmk<fx2>(q[0].x >> 1, q[0].y >> 1);  // factor 1: exact, as a mean value wants it
+#pragma unroll
+    for (int k = 1; k < R; k++) q[k] = fx_tw(q[k], tw[k * twl]);
+  }
+  fx_swap(q, fwd);
+  return tw ? 1 : 0;
+}
+// Memory blocks src[a ls] -> dst[a ld].
+template <int R, int N>
+__device__ __noinline__ void fx_task1(const fx2* src, const fx2* src2, int ls, fx2* dst, int ld,
+                                      const FxTw* tw, int twl, int mode, int w0, int wl) {
+  constexpr int B = fx_block_bits(R);
   fx2 q[R];
-  int E;
+#pragma unroll
+  for (int a = 0; a < R; a++) q[a] = src[a * ls];
+  int E = 0;
   if (mode & (FX_IW | FX_IC)) {
     auto w = [&](int a) { return (mode & FX_IC) ? w0 : wavenum(w0 + wl * a, N); };
-    E = 0;
 #pragma unroll
-    for (int a = 0; a < R; a++) E = max(E, fx_exp_w<B>(v[a], w(a)));
+    for (int a = 0; a < R; a++) E = max(E, fx_e_w(fx_e(q[a]), w(a)));
 #pragma unroll
-    for (int a = 0; a < R; a++) q[a] = fx_in2_iw<B>(v[a], E, w(a));
-    if (mode & FX_SUM) {  // src on its own exponent first: one of the two in registers as doubles
+    for (int a = 0; a < R; a++) q[a] = fx_get_iw<B>(q[a], E, fx_e(q[a]), w(a));
+    if (mode & FX_SUM) {
       const int Eu = E;
+      fx2 v[R];
 #pragma unroll
-      for (int a = 0; a < R; a++) v[a] = src2[at_s(a)];
-      E = max(E, fx_block(v));
+      for (int a = 0; a < R; a++) v[a] = src2[a * ls];
+#pragma unroll
+      for (int a = 0; a < R; a++) E = max(E, fx_e(v[a]));
       const int sh = min(E - Eu, 63);
 #pragma unroll
       for (int a = 0; a < R; a++)
-        q[a] = cadd(cmk<fx2>(q[a].x >> sh, q[a].y >> sh), fx_in2<B>(v[a], E));
+        q[a] = cadd(cmk<fx2>(q[a].x >> sh, q[a].y >> sh), fx_get<B>(v[a], E, fx_e(v[a])));
     }
   } else {
-    E = fx_block(v);
 #pragma unroll
-    for (int a = 0; a < R; a++) q[a] = fx_in2<B>(v[a], E);
+    for (int a = 0; a < R; a++) E = max(E, fx_e(q[a]));
+#pragma unroll
+    for (int a = 0; a < R; a++) q[a] = fx_get<B>(q[a], E, fx_e(q[a]));
   }
-  int adj = 0;
-  if (R % 2 == 0 && (mode & FX_SPLIT)) {  // twice a and h
-    adj = -1;
-    if (mode & FX_C0) {
+  const int hx = (mode & FX_SUM) ? 0 : (mode & (FX_IW | FX_IC)) ? -1 : 1;
+  const int adj = fx_transform(q, tw, twl, mode & FX_FWD, hx, (mode & FX_SUM) ? 2 : 1);
+  fx_put<R, B>(q, E, adj);
 #pragma unroll
-      for (int i = 0; i < R / 2; i++) {
-        const fx2 z = q[2 * i], zq = q[2 * i + 1];
-        q[2 * i] = cmk<fx2>(2 * z.x, 2 * zq.x);
-        q[2 * i + 1] = cmk<fx2>(2 * z.y, 2 * zq.y);
-      }
-    } else {
-      // conj of an input that was multiplied by i c is minus i c times the conjugate
-      const int64_t s = (mode & FX_IC) ? -1 : 0;
+  for (int a = 0; a < R; a++) dst[a * ld] = q[a];
+}
+// Memory blocks src[(a >> 1) s2 + (a & 1) s1] -> dst[(a >> 1) d2 + (a & 1) d1], with FX_PAIR or
+// FX_SPLIT.
+template <int R>
+__device__ __noinline__ void fx_task2(const fx2* src, int s1, int s2, fx2* dst, int d1, int d2,
+                                      const FxTw* tw, int mode, int c) {
+  constexpr int B = fx_block_bits(R);
+  fx2 q[R];
 #pragma unroll
-      for (int i = 0; i < R / 2; i++) {
-        const fx2 z = q[2 * i];
-        const fx2 zq = cmk<fx2>((q[2 * i + 1].x ^ s) - s, (q[2 * i + 1].y ^ s) - s);
-        q[2 * i] = cmk<fx2>(z.x + zq.x, z.y - zq.y);
-        q[2 * i + 1] = cmk<fx2>(z.y + zq.y, zq.x - z.x);
-      }
+  for (int a = 0; a < R; a++) q[a] = src[(a >> 1) * s2 + (a & 1) * s1];
+  int E = 0;
+  if (mode & FX_IC) {
+#pragma unroll
+    for (int a = 0; a < R; a++) E = max(E, fx_e_w(fx_e(q[a]), c));
+#pragma unroll
+    for (int a = 0; a < R; a++) q[a] = fx_get_iw<B>(q[a], E, fx_e(q[a]), c);
+  } else {
+#pragma unroll
+    for (int a = 0; a < R; a++) E = max(E, fx_e(q[a]));
+#pragma unroll
+    for (int a = 0; a < R; a++) q[a] = fx_get<B>(q[a], E, fx_e(q[a]));
+  }
+  const bool c0 = c == 0;
+  if (mode & FX_SPLIT) {  // twice a and h
+    // conj of an input that was multiplied by i c is minus i c times the conjugate
+    const int64_t s = (mode & FX_IC) ? -1 : 0;
+#pragma unroll
+    for (int i = 0; i < R / 2; i++) {
+      const fx2 z = q[2 * i];
+      const fx2 zq = cmk<fx2>((q[2 * i + 1].x ^ s) - s, (q[2 * i + 1].y ^ s) - s);
+      q[2 * i] = c0 ? cmk<fx2>(2 * z.x, 2 * zq.x) : cmk<fx2>(z.x + zq.x, z.y - zq.y);
+      q[2 * i + 1] = c0 ? cmk<fx2>(2 * z.y, 2 * zq.y) : cmk<fx2>(z.y + zq.y, zq.x - z.x);
     }
-  }
-  const bool swap = mode & FX_FWD;
-#pragma unroll
-  for (int a = 0; a < R; a++)
-    q[a] = cmk<fx2>(swap ? q[a].y : q[a].x, swap ? q[a].x : q[a].y);
-  reg_dft<R, +1>(q);
-  if (tw) {
-    adj += 1;
-#pragma unroll
-    for (int k = 0; k < R; k++) q[k] = fx_tw(q[k], tw[k * twl]);
-  }
-#pragma unroll
-  for (int a = 0; a < R; a++)
-    q[a] = cmk<fx2>(swap ? q[a].y : q[a].x, swap ? q[a].x : q[a].y);
-  if (R % 2 == 0 && (mode & FX_PAIR)) {
-    const bool c0 = mode & FX_C0;
+    const bool ic = mode & FX_IC;  // the sums' roundings: re or im low by one
+    const int adj = fx_transform(q, tw, 1, true, ic ? 0 : 2, ic || c0 ? 2 : 0);
+    fx_put<R, B>(q, E, adj - 1);
+  } else {
+    fx_transform(q, nullptr, 0, false, (mode & FX_IC) ? -1 : 1, 1);
 #pragma unroll
     for (int i = 0; i < R / 2; i++) {
       const fx2 a = q[2 * i], h = q[2 * i + 1];
       q[2 * i] = c0 ? cmk<fx2>(a.x, h.x) : cmk<fx2>(a.x - h.y, a.y + h.x);
       q[2 * i + 1] = c0 ? cmk<fx2>(a.y, h.y) : cmk<fx2>(a.x + h.y, h.x - a.y);
     }
+    fx_put<R, B>(q, E, 0);
   }
-  fx_store<R, B>(q, v, E, adj);
 #pragma unroll
-  for (int a = 0; a < R; a++) dst[at_d(a)] = v[a];
+  for (int a = 0; a < R; a++) dst[(a >> 1) * d2 + (a & 1) * d1] = q[a];
 }
-// values at src[a ls], results at dst[a ld]
+// Doubles src[a l] -> memory blocks dst[a l].
 template <int R, int N>
-__device__ __noinline__ void fx_task1(const double2* src, const double2* src2, int ls,
-                                      double2* dst, int ld, const FxTw* tw, int twl, int mode,
-                                      int w0, int wl) {
-  fx_task_body<R, N>(src, src2, dst, [&](int a) { return a * ls; }, [&](int a) { return a * ld; },
-                     tw, twl, mode, w0, wl);
+__device__ __noinline__ void fx_enter2(const double2* src, fx2* dst, int l, const FxTw* tw,
+                                       int mode, int w0, int wl) {
+  constexpr int B = fx_block_bits(R);
+  double2 v[R];
+#pragma unroll
+  for (int a = 0; a < R; a++) v[a] = src[a * l];
+  fx2 q[R];
+  int E = 0;
+  if (mode & FX_IW) {
+#pragma unroll
+    for (int a = 0; a < R; a++) E = max(E, fx_exp_w<B>(v[a], wavenum(w0 + wl * a, N)));
+#pragma unroll
+    for (int a = 0; a < R; a++) q[a] = fx_in2_iw<B>(v[a], E, wavenum(w0 + wl * a, N));
+  } else {
+    E = fx_block(v);
+#pragma unroll
+    for (int a = 0; a < R; a++) q[a] = fx_in2<B>(v[a], E);
+  }
+  const int adj = fx_transform(q, tw, 1, mode & FX_FWD, 0, 0);
+  fx_put<R, B>(q, E, adj);
+#pragma unroll
+  for (int a = 0; a < R; a++) dst[a * l] = q[a];
 }
-// values at src[(a >> 1) s2 + (a & 1) s1], results at dst[(a >> 1) d2 + (a & 1) d1]
-template <int R, int N>
-__device__ __noinline__ void fx_task2(const double2* src, int s1, int s2, double2* dst, int d1,
-                                      int d2, const FxTw* tw, int twl, int mode, int w0, int wl) {
-  fx_task_body<R, N>(src, nullptr, dst, [&](int a) { return (a >> 1) * s2 + (a & 1) * s1; },
-                     [&](int a) { return (a >> 1) * d2 + (a & 1) * d1; }, tw, twl, mode, w0, wl);
+// Memory blocks src[a l] -> doubles dst[a l].
+template <int R>
+__device__ __noinline__ void fx_leave2(const fx2* src, double2* dst, int l, bool fwd) {
+  constexpr int B = fx_block_bits(R);
+  fx2 q[R];
+#pragma unroll
+  for (int a = 0; a < R; a++) q[a] = src[a * l];
+  int E = 0;
+#pragma unroll
+  for (int a = 0; a < R; a++) E = max(E, fx_e(q[a]));
+#pragma unroll
+  for (int a = 0; a < R; a++) q[a] = fx_get<B>(q[a], E, fx_e(q[a]));
+  fx_transform(q, nullptr, 0, fwd, 1, 1);
+  double2 v[R];
+  fx_store<R, B>(q, v, E, 0);
+#pragma unroll
+  for (int a = 0; a < R; a++) dst[a * l] = v[a];
+}
+// One row of a line pair in real space, in place: inverse transform, times the diffusivities
+// ka[a ks], kb[a ks] of the two lines, forward transform and twiddles. Returns sum k z^2.
+template <int R>
+__device__ __noinline__ double fx_middle2(fx2* row, const double* ka, const double* kb, int ks,
+                                          const FxTw* tw) {
+  constexpr int B = fx_block_bits(R), G = 62 - B;
+  double va[R], vb[R];
+#pragma unroll
+  for (int a = 0; a < R; a++) {
+    va[a] = ka[a * ks];
+    vb[a] = kb[a * ks];
+  }
+  fx2 q[R];
+#pragma unroll
+  for (int a = 0; a < R; a++) q[a] = row[a];
+  int E = 0;
+  uint32_t km = 0;
+#pragma unroll
+  for (int a = 0; a < R; a++) {
+    E = max(E, fx_e(q[a]));
+    km = fx_mag(km, cmk<double2>(va[a], vb[a]));
+  }
+  const int Ek = (int)(km >> 20);
+#pragma unroll
+  for (int a = 0; a < R; a++) q[a] = fx_get<B>(q[a], E, fx_e(q[a]));
+  fx_transform(q, nullptr, 0, false, 1, 1);  // z, |q| < 2^62.5
+  // k = m 2^(ek - 1085) with 63 bits of m; z m / 2^64 on the largest ek, then G more bits down
+  int64_t dot = 0;
+  auto times = [&](int64_t z, double k) {
+    const uint32_t hi = fx_hi(k);
+    const int64_t m = (int64_t)((((uint64_t)((hi & 0xfffffu) | 0x100000u) << 32) | fx_lo(k)) << 10);
+    const int64_t s = (int64_t)((int32_t)hi >> 31);
+    const int64_t p = fx_mulh(z, fx_split((m ^ s) - s)) >>
+                      fx_min((uint32_t)(Ek - (int)((hi >> 20) & 0x7ff)), 63u);
+    dot += fx_mulh(p, fx_split(z)) >> 5;
+    return p >> G;
+  };
+#pragma unroll
+  for (int a = 0; a < R; a++) q[a] = cmk<fx2>(times(q[a].x, va[a]), times(q[a].y, vb[a]));
+  double sum = scalbn((double)dot, 2 * E + Ek - 2996 - 2 * B);
+  if (E > kFxHuge || Ek > kFxHuge) sum = fx_nan();
+  if (E < kFxTiny || Ek < kFxTiny) sum = 0.0;
+  E = E > kFxHuge || Ek > kFxHuge ? (int)kFxBad : max(E + Ek - 1021 + G, 0);
+  const int adj = fx_transform(q, tw, 1, true, 1, 1);
+  fx_put<R, B>(q, E, adj);
+#pragma unroll
+  for (int a = 0; a < R; a++) row[a] = q[a];
+  return sum;
 }
 template <>
 struct Task<double2> {
@@ -329,6 +441,11 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
                 T = Geo_::T, NT = Geo_::NT, PS2 = Geo_::PS2, TILE = Geo_::TILE;
   constexpr int S = N * PL;
   constexpr bool FX = sizeof(R) == 8;
+  auto fx = [](auto* q) {  // the same memory as fixed-point blocks
+    using Q = std::conditional_t<std::is_const<std::remove_pointer_t<decltype(q)>>::value,
+                                 const fx2, fx2>;
+    return reinterpret_cast<Q*>(q);
+  };
   extern __shared__ double2 plane_dyn[];
   C* buf = reinterpret_cast<C*>(plane_dyn);
   using K = Task<C>;
@@ -338,6 +455,7 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
   Tw* twB = twA + N;                                 // [b R1 + k1], the same
   C* zcol = reinterpret_cast<C*>(twB + N);           // column kz' = 0 of a plane, forward
   C* zin = zcol + N;                                 // and inverse
+  [[maybe_unused]] double* wtab = reinterpret_cast<double*>(zin + N);  // double: wave numbers
   __shared__ double tot[5];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int i = tid; i < N; i += NT) {
@@ -345,10 +463,14 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
     const Tw w = reinterpret_cast<const Tw*>(A.tw)[b * k1];  // b k1 < N
     twA[i] = w;
     twB[b * R1 + k1] = w;
+    if constexpr (FX) wtab[i] = (double)wavenum(i, N);
   }
   __syncthreads();
   const R invN = (R)(1.0 / ((double)N * N * N));
   const double dinvN = 1.0 / ((double)N * N * N);
+  // double: the spectra sent to the planes keep their factor n^3
+  const double dscale = FX ? dinvN : 1.0;
+  const R a1 = (R)(A.a_cn * dscale), invN2 = invN * invN;
   const R a_cn = (R)A.a_cn, pcc = (R)A.pc_c;
   GridBarrier bar{A.bar, 0};
   // PCG scalars, the same in every CTA (thread 0 updates them)
@@ -388,7 +510,8 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
   auto totals = [&](int q_n, int s0) {
     for (int q = warp; q < q_n; q += Geo_::NW) {
       double x = 0;
-      for (int b = lane; b < (int)gridDim.x; b += 32) x += __ldcg(&A.part[(s0 + q) * gridDim.x + b]);
+      for (int b = lane; b < (int)gridDim.x; b += 32)
+        x += __ldcg(&A.part[(s0 + q) * gridDim.x + b]);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
       if (lane == 0) tot[q] = x;
@@ -420,10 +543,13 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
     return cmk<C>(v.x * e0 / (q0 * q0), v.y * e1 / (q1 * q1));
   };
 
+  // the twiddles of a task: none for index 0, where all are 1
+  [[maybe_unused]] auto at_tw = [](int i, const Tw* tw) { return i ? tw : nullptr; };
   Acc<R> acc[5];
   // Double: row k1 of a line pair in real space (places k2, z = k1 + R1 k2 of lines l0 and l1)
   auto line_middle = [&](int kind, C* row, int64_t l0, int64_t l1, int k1) {
     if constexpr (FX) {
+      const Tw* tw = at_tw(k1, twA + k1 * R2);
       if (kind == PS_FWD) {
 #pragma unroll 2
         for (int k2 = 0; k2 < R2; k2++) {
@@ -431,28 +557,18 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
           row[k2] = cmk<C>(A.in[l0 + m], A.in[l1 + m]);
           if (A.pre) row[k2] = reacted(row[k2], l0 + m, l1 + m);
         }
+        fx_enter2<R2, N>(row, fx(row), 1, tw, FX_FWD, 0, 0);
+      } else if (kind == PS_GRAD) {
+        acc[0].add(fx_middle2<R2>(fx(row), kf + l0 + k1, kf + l1 + k1, R1, tw));
       } else {
-        fx_task2<R2, N>(row, 1, 2, row, 1, 2, nullptr, 0, 0, 0, 0);
-        if (kind == PS_GRAD) {
+        fx_leave2<R2>(fx(row), row, 1, false);
 #pragma unroll 4
-          for (int k2 = 0; k2 < R2; k2++) {
-            const int m = k1 + R1 * k2;
-            const C z = row[k2];
-            const R sx = z.x * kf[l0 + m], sy = z.y * kf[l1 + m];
-            acc[0].add(sx * z.x + sy * z.y);
-            row[k2] = cmk<C>(sx, sy);
-          }
-        } else {
-#pragma unroll 4
-          for (int k2 = 0; k2 < R2; k2++) {
-            const int m = k1 + R1 * k2;
-            A.out[l0 + m] = row[k2].x;
-            A.out[l1 + m] = row[k2].y;
-          }
+        for (int k2 = 0; k2 < R2; k2++) {
+          const int m = k1 + R1 * k2;
+          A.out[l0 + m] = row[k2].x;
+          A.out[l1 + m] = row[k2].y;
         }
       }
-      if (kind != PS_BACK)
-        fx_task2<R2, N>(row, 1, 2, row, 1, 2, twA + k1 * R2, 1, FX_FWD, 0, 0);
     }
   };
 
@@ -478,31 +594,30 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
             const C* G = (kind == PS_GRAD && j == 0 ? Gp : Gp + S) + x * PL + cb * TC;
             if (cb == 0)
               for (int ky = tid; ky < N; ky += NT) {
-                const C z = G[ky * NH], w = G[ky * NH + NQ];
-                zin[ky] = cmk<C>(z.x - w.y, z.y + w.x);
+                fx(zin)[ky] = fx_plus_i(fx(G)[ky * NH], fx(G)[ky * NH + NQ]);
               }
             __syncthreads();
             for (int task = tid; task < TC * R2; task += NT) {
               const int b = task / TC, c = task - b * TC;
               const bool c0 = cb == 0 && c == 0;
               const int ld = c0 ? 1 : NH;
-              fx_task1<R1, N>((c0 ? zin : G + c) + b * ld, nullptr, R2 * ld, buf + b * TC + c,
-                              R2 * TC, twA + b, R2, j == 1 ? FX_IW : 0, b, R2);
+              fx_task1<R1, N>(fx((c0 ? zin : G + c) + b * ld), nullptr, R2 * ld,
+                              fx(buf + b * TC + c), R2 * TC, at_tw(b, twA + b), R2,
+                              j == 1 ? FX_IW : 0, b, R2);
             }
             __syncthreads();
             for (int task = tid; task < TC * R1; task += NT) {
               const int k1 = task / TC, c = task - k1 * TC, cc = cb * TC + c;
-              fx_task2<R2, N>(buf + k1 * R2 * TC + c, TC, 2 * TC, W + k1 * (R2 / 2) * N + c,
-                              (cc == 0 ? NQ : N - cc) - cc, N, nullptr, 0,
-                              FX_PAIR | (j == 2 ? FX_IC : 0) | (cc == 0 ? FX_C0 : 0), cc, 0);
+              fx_task2<R2>(fx(buf + k1 * R2 * TC + c), TC, 2 * TC, fx(W + k1 * (R2 / 2) * N + c),
+                           (cc == 0 ? NQ : N - cc) - cc, N, nullptr,
+                           FX_PAIR | (j == 2 ? FX_IC : 0), cc);
             }
           } else {
             for (int task = tid; task < TC * R1; task += NT) {
               const int k1 = task / TC, c = task - k1 * TC, cc = cb * TC + c;
-              fx_task2<R2, N>(W + k1 * (R2 / 2) * N + c, (cc == 0 ? NQ : N - cc) - cc, N,
-                              buf + k1 * R2 * TC + c, TC, 2 * TC, twA + k1 * R2, 1,
-                              FX_FWD | FX_SPLIT | (j == 2 ? FX_IC : 0) | (cc == 0 ? FX_C0 : 0),
-                              cc, 0);
+              fx_task2<R2>(fx(W + k1 * (R2 / 2) * N + c), (cc == 0 ? NQ : N - cc) - cc, N,
+                           fx(buf + k1 * R2 * TC + c), TC, 2 * TC, at_tw(k1, twA + k1 * R2),
+                           FX_SPLIT | (j == 2 ? FX_IC : 0), cc);
             }
             __syncthreads();
             C* M = Mp + j * S + x * PL;
@@ -510,16 +625,15 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
               const int b = task / TC, c = task - b * TC;
               const bool c0 = cb == 0 && c == 0;
               const int ld = c0 ? 1 : NH;
-              fx_task1<R1, N>(buf + b * TC + c, nullptr, R2 * TC,
-                              (c0 ? zcol : M + cb * TC + c) + b * ld, R2 * ld, nullptr, 0, FX_FWD,
-                              0, 0);
+              fx_task1<R1, N>(fx(buf + b * TC + c), nullptr, R2 * TC,
+                              fx((c0 ? zcol : M + cb * TC + c) + b * ld), R2 * ld, nullptr, 0,
+                              FX_FWD, 0, 0);
             }
             __syncthreads();
             if (cb == 0)
               for (int ky = tid; ky < N; ky += NT) {
-                const C z = zcol[ky], zm = zcol[ky == 0 ? 0 : N - ky];
-                M[ky * NH] = cmk<C>((R)0.5 * (z.x + zm.x), (R)0.5 * (z.y - zm.y));
-                M[ky * NH + NQ] = cmk<C>((R)0.5 * (z.y + zm.y), (R)-0.5 * (z.x - zm.x));
+                fx_halves(fx(zcol)[ky], fx(zcol)[ky == 0 ? 0 : N - ky], fx(M)[ky * NH],
+                          fx(M)[ky * NH + NQ]);
               }
           }
           __syncthreads();
@@ -539,7 +653,8 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
           C* const W = A.W + (((int64_t)j * N + x) * NQ + pr) * N + t;
           const bool on = id < pairs;
           if (kind != PS_FWD) {
-            if (on) fx_task1<R1, N>(W, nullptr, R2, col, R2 + 1, twA + t, R2, 0, 0, 0);
+            if (on)
+              fx_task1<R1, N>(fx(W), nullptr, R2, fx(col), R2 + 1, at_tw(t, twA + t), R2, 0, 0, 0);
             __syncwarp();
           }
           if (on) {
@@ -548,7 +663,7 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
           }
           if (kind != PS_BACK) {
             __syncwarp();
-            if (on) fx_task1<R1, N>(col, nullptr, R2 + 1, W, R2, nullptr, 0, FX_FWD, 0, 0);
+            if (on) fx_task1<R1, N>(fx(col), nullptr, R2 + 1, fx(W), R2, nullptr, 0, FX_FWD, 0, 0);
           }
           __syncwarp();
         }
@@ -568,8 +683,12 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
           // y inverse: the kz = 0 and kz = N/2 columns as one, then rows ky = R2 a + b of column c
           const C* G = (step == PS_GRAD && j == 0 ? Gp : Gp + S) + x * PL;
           for (int ky = tid; ky < N; ky += NT) {
-            const C z = G[ky * NH], w = G[ky * NH + NQ];
-            zin[ky] = cmk<C>(z.x - w.y, z.y + w.x);
+            if constexpr (FX) {
+              fx(zin)[ky] = fx_plus_i(fx(G)[ky * NH], fx(G)[ky * NH + NQ]);
+            } else {
+              const C z = G[ky * NH], w = G[ky * NH + NQ];
+              zin[ky] = cmk<C>(z.x - w.y, z.y + w.x);
+            }
           }
           __syncthreads();
           for (int task = tid; task < NQ * R2; task += NT) {
@@ -577,9 +696,9 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
             const C* src = c == 0 ? zin : G + c;
             const int ld = c == 0 ? 1 : NH;
             if constexpr (FX) {
-              fx_task1<R1, N>(src + b * ld, nullptr, R2 * ld,
-                              buf + (b >> 1) * PS2 + ((b & 1) ? odd(c) : even(c)), R2 / 2 * PS2,
-                              twA + b, R2, j == 1 ? FX_IW : 0, b, R2);
+              fx_task1<R1, N>(fx(src + b * ld), nullptr, R2 * ld,
+                              fx(buf + (b >> 1) * PS2 + ((b & 1) ? odd(c) : even(c))),
+                              R2 / 2 * PS2, at_tw(b, twA + b), R2, j == 1 ? FX_IW : 0, b, R2);
             } else {
             C u[R1];
 #pragma unroll
@@ -601,8 +720,8 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
             C* row = buf + k1 * (R2 / 2) * PS2 + even(c);
             const int od = odd(c) - even(c);
             if constexpr (FX) {
-              fx_task2<R2, N>(row, od, PS2, row, od, PS2, nullptr, 0,
-                              FX_PAIR | (j == 2 ? FX_IC : 0) | (c == 0 ? FX_C0 : 0), c, 0);
+              fx_task2<R2>(fx(row), od, PS2, fx(row), od, PS2, nullptr,
+                           FX_PAIR | (j == 2 ? FX_IC : 0), c);
             } else {
             C v[R2];
 #pragma unroll
@@ -625,7 +744,9 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
             // thread t: index R2 a + t in place, then rows k1 = t, t + R2, ... in place, and back
             C* const col = E + t;
             if (step != PS_FWD) {
-              if (on) fx_task1<R1, N>(col, nullptr, R2 + 1, col, R2 + 1, twA + t, R2, 0, 0, 0);
+              if (on)
+                fx_task1<R1, N>(fx(col), nullptr, R2 + 1, fx(col), R2 + 1, at_tw(t, twA + t), R2,
+                                0, 0, 0);
               __syncwarp();
             }
             if (on) {
@@ -634,7 +755,9 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
             }
             if (step != PS_BACK) {
               __syncwarp();
-              if (on) fx_task1<R1, N>(col, nullptr, R2 + 1, col, R2 + 1, nullptr, 0, FX_FWD, 0, 0);
+              if (on)
+                fx_task1<R1, N>(fx(col), nullptr, R2 + 1, fx(col), R2 + 1, nullptr, 0, FX_FWD, 0,
+                                0);
             }
             continue;
           } else {
@@ -729,9 +852,8 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
             C* row = buf + k1 * (R2 / 2) * PS2 + even(c);
             const int od = odd(c) - even(c);
             if constexpr (FX) {
-              fx_task2<R2, N>(row, od, PS2, row, od, PS2, twA + k1 * R2, 1,
-                              FX_FWD | FX_SPLIT | (j == 2 ? FX_IC : 0) | (c == 0 ? FX_C0 : 0), c,
-                              0);
+              fx_task2<R2>(fx(row), od, PS2, fx(row), od, PS2, at_tw(k1, twA + k1 * R2),
+                           FX_SPLIT | (j == 2 ? FX_IC : 0), c);
             } else {
             C v[R2];
 #pragma unroll
@@ -748,8 +870,8 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
             C* dst = c == 0 ? zcol : M + c;
             const int ld = c == 0 ? 1 : NH;
             if constexpr (FX) {
-              fx_task1<R1, N>(buf + (b >> 1) * PS2 + ((b & 1) ? odd(c) : even(c)), nullptr,
-                              R2 / 2 * PS2, dst + b * ld, R2 * ld, nullptr, 0, FX_FWD, 0, 0);
+              fx_task1<R1, N>(fx(buf + (b >> 1) * PS2 + ((b & 1) ? odd(c) : even(c))), nullptr,
+                              R2 / 2 * PS2, fx(dst + b * ld), R2 * ld, nullptr, 0, FX_FWD, 0, 0);
             } else {
             C u[R1];
 #pragma unroll
@@ -763,9 +885,14 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
           }
           __syncthreads();
           for (int ky = tid; ky < N; ky += NT) {  // kz' = 0 into kz = 0 and kz = N/2
-            const C z = zcol[ky], zm = zcol[ky == 0 ? 0 : N - ky];
-            M[ky * NH] = cmk<C>((R)0.5 * (z.x + zm.x), (R)0.5 * (z.y - zm.y));
-            M[ky * NH + NQ] = cmk<C>((R)0.5 * (z.y + zm.y), (R)-0.5 * (z.x - zm.x));
+            if constexpr (FX) {
+              fx_halves(fx(zcol)[ky], fx(zcol)[ky == 0 ? 0 : N - ky], fx(M)[ky * NH],
+                        fx(M)[ky * NH + NQ]);
+            } else {
+              const C z = zcol[ky], zm = zcol[ky == 0 ? 0 : N - ky];
+              M[ky * NH] = cmk<C>((R)0.5 * (z.x + zm.x), (R)0.5 * (z.y - zm.y));
+              M[ky * NH + NQ] = cmk<C>((R)0.5 * (z.y + zm.y), (R)-0.5 * (z.x - zm.x));
+            }
           }
         }
       }
@@ -786,7 +913,7 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
         if (tid == 0) {
           if (cg.iter == 0) tot[0] = cg.pp;  // of the set-up's first direction
           cg.dpi_old = cg.dpi;
-          cg.dpi = tot[0] * dinvN + A.a_cn * tot[1];
+          cg.dpi = tot[0] * dinvN + A.a_cn * tot[1] * dscale * dscale;
           cg.beta_old = cg.beta;
           cg.it = cg.iter + 1;
           if (cg.dpi == 0.0 || (cg.iter > 0 && cg.dpi * cg.dpi_old <= 0.0))
@@ -811,8 +938,8 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
             if (q >= PL) continue;
             const C* src = Mp + i * S + q;
             if constexpr (FX) {  // M_x, then i w_y M_y + M_z
-              fx_task1<R1, N>(src + b * PL, i == 1 ? src + S + b * PL : nullptr, R2 * PL,
-                              buf + i * TILE + b * T + c, R2 * T, twA + b, R2,
+              fx_task1<R1, N>(fx(src + b * PL), fx(src + S + b * PL), R2 * PL,
+                              fx(buf + i * TILE + b * T + c), R2 * T, at_tw(b, twA + b), R2,
                               i == 1 ? FX_FWD | FX_IC | FX_SUM : FX_FWD, wavenum(q / NH, N), 0);
               continue;
             } else {
@@ -849,7 +976,7 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
           };
           // what a step does at one spectrum element: d = the forward x transform's result (the
           // divergence for two inputs); returns the value that is transformed back
-          auto element = [&](int k2, C d) -> C {
+          [[maybe_unused]] auto element = [&](int k2, C d) -> C {
             const int e = at(k2);
             switch (step) {
               case PS_SPEC:
@@ -912,19 +1039,82 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
             }
           };
           if constexpr (FX) {
-            if (nin) fx_task2<R2, N>(sl, T, 2 * T, sl, T, 2 * T, nullptr, 0, FX_FWD, 0, 0);
-            if (nin == 2)
-              fx_task2<R2, N>(sl + TILE, T, 2 * T, sl + TILE, T, 2 * T, nullptr, 0, FX_FWD,
-                              0, 0);
+            // The same in double. FP64 operations are what this costs: a task's sums are taken
+            // without the multiplicity, ||z||^2 and <z, r> of the set-up are those of its first direction,
+            // and the spectra sent to the planes keep their factor n^3 (a1 = a_cn / n^3).
+            double part[4] = {0, 0, 0, 0};
+            auto element_fx = [&](int k2, C d) -> C {
+              const int e = at(k2);
+              switch (step) {
+                case PS_SPEC:
+                case PS_ENTER:
+                  ch[e] = d;
+                  return d;
+                case PS_OPEN:
+                  return ch[e];
+                case PS_SMOOTH:
+                  return cmul2(d, A.mulk[e]);
+                case PS_SETUP: {
+                  const C c0 = ch[e];
+                  const R P = pm(k2);
+                  const R br = P * (c0.x + a1 * d.x), bi = P * (c0.y + a1 * d.y);
+                  const C r = cmk<C>((R)2 * a1 * d.x, (R)2 * a1 * d.y);
+                  const C p = cmk<C>(P * r.x, P * r.y);  // the first direction
+                  part[0] = fma(br, br, fma(bi, bi, part[0]));
+                  part[1] = fma(p.x, p.x, fma(p.y, p.y, part[1]));
+                  part[2] = fma(p.x, r.x, fma(p.y, r.y, part[2]));
+                  if (A.cx) {
+                    const C xv = A.cx[e];
+                    part[3] = fma(xv.x, d.x, fma(xv.y, d.y, part[3]));
+                  }
+                  xh[e] = cmk<C>(c0.x * invN, c0.y * invN);
+                  rh[e] = r;
+                  ph[e] = p;
+                  return p;
+                }
+                case PS_UPDATE: {
+                  const C p = ph[e], xv = xh[e], rv = rh[e];
+                  const R P = pm(k2);
+                  const C r = cmk<C>(rv.x - al * (p.x - a1 * d.x), rv.y - al * (p.y - a1 * d.y));
+                  xh[e] = cmk<C>(xv.x + alN * p.x, xv.y + alN * p.y);
+                  rh[e] = r;
+                  const R t = P * (r.x * r.x + r.y * r.y);
+                  part[0] = fma(P, t, part[0]);
+                  part[1] += t;
+                  return d;
+                }
+                case PS_DIR: {
+                  const C rv = rh[e], po = ph[e];
+                  const R P = pm(k2);
+                  const C p = cmk<C>(fma(P, rv.x, bc * po.x), fma(P, rv.y, bc * po.y));
+                  ph[e] = p;
+                  part[0] = fma(p.x, p.x, fma(p.y, p.y, part[0]));
+                  return p;
+                }
+                case PS_LEAVE:
+                  return xh[e];
+                case PS_APPLY:
+                  return cmk<C>(d.x * invN2, d.y * invN2);
+                default: {  // PS_DOT
+                  const C xv = A.cx[e];
+                  part[0] = fma(xv.x, d.x, fma(xv.y, d.y, part[0]));
+                  return d;
+                }
+              }
+            };
+            const Tw* tw = at_tw(k1, twA + k1 * R2);
+            if (nin) fx_leave2<R2>(fx(sl), sl, T, true);
+            if (nin == 2) fx_leave2<R2>(fx(sl + TILE), sl + TILE, T, true);
 #pragma unroll 2
             for (int k2 = 0; k2 < R2; k2++) {
               C d = sl[k2 * T];
-              if (nin == 2) d = cadd(cimul<C>((R)wavenum(k1 + R1 * k2, N), d), sl[TILE + k2 * T]);
-              sl[k2 * T] = element(k2, d);
+              if (nin == 2) d = cadd(cimul<C>(wtab[k1 + R1 * k2], d), sl[TILE + k2 * T]);
+              sl[k2 * T] = element_fx(k2, d);
             }
-            if (nout == 2)
-              fx_task2<R2, N>(sl, T, 2 * T, sl + TILE, T, 2 * T, twA + k1 * R2, 1, FX_IW, k1, R1);
-            if (nout) fx_task2<R2, N>(sl, T, 2 * T, sl, T, 2 * T, twA + k1 * R2, 1, 0, 0, 0);
+#pragma unroll
+            for (int q = 0; q < 4; q++) acc[q].s += mult * part[q];
+            if (nout == 2) fx_enter2<R2, N>(sl, fx(sl + TILE), T, tw, FX_IW, k1, R1);
+            if (nout) fx_enter2<R2, N>(sl, fx(sl), T, tw, 0, 0, 0);
             continue;
           } else {
           C d[R2];
@@ -969,8 +1159,8 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
             if (q >= PL) continue;
             C* dst = Gp + (1 - i) * S + q;  // i = 0: G_0, i = 1: G_x
             if constexpr (FX) {
-              fx_task1<R1, N>(buf + i * TILE + b * T + c, nullptr, R2 * T, dst + b * PL, R2 * PL,
-                              nullptr, 0, 0, 0, 0);
+              fx_task1<R1, N>(fx(buf + i * TILE + b * T + c), nullptr, R2 * T, fx(dst + b * PL),
+                              R2 * PL, nullptr, 0, 0, 0, 0);
             } else {
             C u[R1];
 #pragma unroll
@@ -985,7 +1175,7 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
       }
       if (step == PS_SETUP) {
         const double v[5] = {acc[0].value(), acc[1].value(), acc[2].value(), acc[3].value(),
-                             acc[4].value()};
+                             FX ? acc[1].value() : acc[4].value()};
         partials(v, 5, 1);
       } else if (step == PS_UPDATE || step == PS_DOT) {
         const double v[2] = {acc[0].value(), acc[1].value()};
@@ -1041,7 +1231,7 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
             cg.status = 2;
             cg.it = 1;
           }
-          if (A.cx && blockIdx.x == 0) A.sc->acc[6] += A.kdot_weight * tot[3] * dinvN;
+          if (A.cx && blockIdx.x == 0) A.sc->acc[6] += A.kdot_weight * tot[3] * dinvN * dscale;
           cg.step = cg.status == 0 ? PS_GRAD : PS_LEAVE;
         }
         __syncthreads();
@@ -1074,7 +1264,7 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
         break;
       case PS_DOT:
         totals(1, 2);
-        if (blockIdx.x == 0 && tid == 0) A.sc->acc[6] += A.kdot_weight * tot[0] * dinvN;
+        if (blockIdx.x == 0 && tid == 0) A.sc->acc[6] += A.kdot_weight * tot[0] * dinvN * dscale;
         bar.leave();
         return;
       default:  // PS_SMOOTH, PS_LEAVE, PS_APPLY
@@ -1088,7 +1278,8 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
       }
     }
   }
-  if ((A.prog == PP_SOLVE || A.prog == PP_SOLVE_SPEC) && blockIdx.x == 0 && tid == 0) {  // outcome and sweep statistics
+  // outcome and sweep statistics
+  if ((A.prog == PP_SOLVE || A.prog == PP_SOLVE_SPEC) && blockIdx.x == 0 && tid == 0) {
     DevScalars* s = A.sc;
     s->it = cg.it;
     s->iter = cg.iter;
