@@ -1,0 +1,15 @@
+// Plane kernels of the FP64 engine, 104^3 to 144^3 (one CTA per SM).
+#include "plane.cuh"
+
+namespace glia {
+PlaneKernel plane_kernel_f64_mid(int n) {
+  switch (n) {
+    case 104: return plane_entry<double, 104>();
+    case 112: return plane_entry<double, 112>();
+    case 120: return plane_entry<double, 120>();
+    case 128: return plane_entry<double, 128>();
+    case 144: return plane_entry<double, 144>();
+    default: return PlaneKernel{nullptr, 0, 0, 0, false};
+  }
+}
+}  // namespace glia

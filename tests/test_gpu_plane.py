@@ -14,7 +14,8 @@ from tests.gpu_common import FP64, MIXED, configure, gpu, small_problem
 from tests.helpers import rel_l2
 
 pytestmark = pytest.mark.gpu
-SIZES = {FP64: [16, 32, 64, 96, 120, 128, 256], MIXED: [16, 32, 64, 96, 128]}
+SIZES = {FP64: [*range(16, 129, 8), 144, 160, 176, 192, 208, 224, 240, 256],
+         MIXED: [*range(16, 129, 8), 160, 176, 192, 208, 224]}
 CASES = [(p, n) for p in (FP64, MIXED) for n in SIZES[p]]
 
 
@@ -49,9 +50,9 @@ def test_d_apply_against_numpy(prec, n):
     g.close()
 
 
-@pytest.mark.parametrize("prec,n", [c for c in CASES if c[1] <= 128])
+@pytest.mark.parametrize("prec,n", [c for c in CASES if c[1] <= 192])
 def test_solve_state_and_gradient_match_the_cufft_path(prec, n, monkeypatch):
-    if n == 16:  # too coarse for the seeded white matter: the whole brain mask instead
+    if n < 32:  # too coarse for the seeded white matter: the whole brain mask instead
         wl = syn.GradientWorkload(n=n, nt=2, n_gauss=4)
         m = syn.ellipsoid_mask(n)
         tissue = syn.Tissue(wm=m * 1.0, gm=m * 0.0, csf=m * 0.0, vt=m * 0.0, mask=m)

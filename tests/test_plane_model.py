@@ -5,7 +5,7 @@ the model takes a phase's stages over whole index ranges at once."""
 import numpy as np
 import pytest
 
-SIZES = [16, 32, 64, 96, 120, 128]
+SIZES = [*range(16, 129, 8), 144, 160]
 
 
 def geometry(n, single):
