@@ -68,9 +68,18 @@ struct PlaneGeo {
   static constexpr bool SPLIT = GAP && NQ * PS2 * 16 > 200 * 1024;
   static constexpr int TC = NQ % 16 == 0 ? 16 : 8;  // SPLIT: columns per block
   static constexpr int PLANE = SPLIT ? 0 : NQ * PS2;
-  // columns per tile: about one tile per resident CTA
-  static constexpr int T =
-      N <= 32 ? 4 : N <= 64 ? 8 : N < 112 ? 16 : SPLIT ? 8 : sizeof(R) == 4 ? 28 : 32;
+  // columns per tile of a column phase: the fewest rounds of tiles over the resident CTAs that at
+  // most MAXT columns allow, then the smallest multiple of 4 (a sector) that needs no more; float
+  // 8 or 16 up to 16, whose divisions are shifts (12 costs 2 % at 72^3), 4 only up to 32^3
+  static constexpr int PB = PLANE * (int)sizeof(C);
+  static constexpr int CTAS = PB > 110 * 1024 ? 152 : 304;
+  static constexpr int MAXT = sizeof(R) == 4 ? 32 : CTAS == 304 ? 24 : 210 * 1024 / (2 * N * 16);
+  static constexpr int PER = (PL + CTAS - 1) / CTAS, ROUNDS = (PER + MAXT - 1) / MAXT;
+  static constexpr int T4 = ((PER + ROUNDS - 1) / ROUNDS + 3) / 4 * 4;
+  static constexpr int T = SPLIT                             ? 8
+                           : N > 32 && T4 < 8                ? 8
+                           : sizeof(R) == 4 && T4 == 12      ? 16
+                                                             : T4;
   static constexpr int XT = (PL + T - 1) / T;
   static constexpr int TILE = N * T;
   static constexpr int RED = 5 * 512 * 8 / (int)sizeof(C);  // partial sums of a phase
@@ -82,6 +91,13 @@ struct PlaneGeo {
   static constexpr int MINB = SMEM > 110 * 1024 ? 1 : 2;
   static constexpr int NT = N <= 32 ? 128 : (MINB == 2 ? 256 : 512);
   static constexpr int NW = NT / 32, GPW = 32 / R2, NG = NW * GPW;
+  // the two transforms of a column side by side instead of in turn: always in double, in float where
+  // it fills the threads better (elsewhere its spills cost 1 to 2 %). Solve, before -> after, with
+  // T above (before: 16 columns from 72^3 to 104^3, then 28 in float and 32 in double): mixed 64^3
+  // 129 -> 126 us, 104^3 255 -> 242, 144^3 542 -> 509, 160^3 679 -> 617, 192^3 978 -> 910; FP64
+  // 32^3 108 -> 103, 64^3 256 -> 246, 112^3 1005 -> 886, 128^3 1047 -> 992, 144^3 2070 -> 1867
+  static constexpr bool BOTH =
+      sizeof(R) == 8 || (2 * T * R2 + NT - 1) / NT < 2 * ((T * R2 + NT - 1) / NT);
   static_assert(R1 * R2 == N && N % 2 == 0, "decomposition");
   static_assert(R1 <= 16, "register DFT");
   static_assert(!SPLIT || (NG == 16 && N * TC <= BUF), "column block and lines fit the buffer");
@@ -440,7 +456,7 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
   constexpr int N = NN, R1 = Geo_::R1, R2 = Geo_::R2, NQ = Geo_::NQ, NH = Geo_::NH, PL = Geo_::PL,
                 T = Geo_::T, NT = Geo_::NT, PS2 = Geo_::PS2, TILE = Geo_::TILE;
   constexpr int S = N * PL;
-  constexpr bool FX = sizeof(R) == 8;
+  constexpr bool FX = sizeof(R) == 8, BOTH = Geo_::BOTH;
   auto fx = [](auto* q) {  // the same memory as fixed-point blocks
     using Q = std::conditional_t<std::is_const<std::remove_pointer_t<decltype(q)>>::value,
                                  const fx2, fx2>;
@@ -932,9 +948,11 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
       }
       const R al = (R)cg.alpha, alN = (R)(cg.alpha * dinvN), bc = (R)cg.bcoef;
       for (int tile = blockIdx.x; tile < Geo_::XT; tile += gridDim.x) {
-        for (int i = 0; i < nin; i++) {  // forward, first part: rows x = R2 a + b
-          for (int task = tid; task < T * R2; task += NT) {
-            const int c = task % T, b = task / T, q = tile * T + c;
+        // forward, first part: rows x = R2 a + b
+        for (int i0 = 0; i0 < (BOTH ? 1 : nin); i0++) {
+          for (int task = tid; task < (BOTH ? nin : 1) * T * R2; task += NT) {
+            const int c = task % T, ib = task / T, i = BOTH ? ib >= R2 : i0;
+            const int b = BOTH ? ib - i * R2 : ib, q = tile * T + c;
             if (q >= PL) continue;
             const C* src = Mp + i * S + q;
             if constexpr (FX) {  // M_x, then i w_y M_y + M_z
@@ -1153,9 +1171,11 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
           }
         }
         __syncthreads();
-        for (int i = 0; i < nout; i++) {  // inverse, second part: rows x = b + R2 a
-          for (int task = tid; task < T * R2; task += NT) {
-            const int c = task % T, b = task / T, q = tile * T + c;
+        // inverse, second part: rows x = b + R2 a
+        for (int i0 = 0; i0 < (BOTH ? 1 : nout); i0++) {
+          for (int task = tid; task < (BOTH ? nout : 1) * T * R2; task += NT) {
+            const int c = task % T, ib = task / T, i = BOTH ? ib >= R2 : i0;
+            const int b = BOTH ? ib - i * R2 : ib, q = tile * T + c;
             if (q >= PL) continue;
             C* dst = Gp + (1 - i) * S + q;  // i = 0: G_0, i = 1: G_x
             if constexpr (FX) {

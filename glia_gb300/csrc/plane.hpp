@@ -53,9 +53,9 @@ struct PlaneKernel {
 };
 // One instantiation per grid size, in translation units by size: every multiple of 8 that factors
 // into R1 <= 16 and R2 = 4, 8 or 16 (plane.cuh). That leaves 136, 152, 168, 184, 200, 216, 232 and
-// 248 (a factor of 17 or more) on cuFFT's transforms and, in float, 144 (not faster here) and 240
-// (its plane does not fit). Time of a solve, cuFFT's transforms / this kernel: double 2.2 to 5.7 at
-// every size; float 1.7 to 1.9 up to 88, 1.4 to 1.6 up to 120, above see plane_f32_large.cu.
+// 248 (a factor of 17 or more) on cuFFT's transforms and, in float, 240 (its plane does not fit).
+// Time of a solve, cuFFT's transforms / this kernel: double 2.2 to 5.7 at every size; float 1.7 to
+// 1.9 up to 88, 1.4 to 1.6 up to 120, above see plane_f32_large.cu.
 PlaneKernel plane_kernel_f32_small(int n);
 PlaneKernel plane_kernel_f32_large(int n);
 PlaneKernel plane_kernel_f64_small(int n);

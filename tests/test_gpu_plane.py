@@ -15,7 +15,7 @@ from tests.helpers import rel_l2
 
 pytestmark = pytest.mark.gpu
 SIZES = {FP64: [*range(16, 129, 8), 144, 160, 176, 192, 208, 224, 240, 256],
-         MIXED: [*range(16, 129, 8), 160, 176, 192, 208, 224]}
+         MIXED: [*range(16, 129, 8), 144, 160, 176, 192, 208, 224]}
 CASES = [(p, n) for p in (FP64, MIXED) for n in SIZES[p]]
 
 
