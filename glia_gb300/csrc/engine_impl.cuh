@@ -371,7 +371,15 @@ class Engine final : public EngineBase {
   }
   void plane_launch(PlaneArgs<R>& a, double bytes) {
     void* args[] = {&a};
-    const int grid = std::min({plane_.items, plane_res_, red_blocks_});
+    int grid = std::min({plane_.items, plane_res_, red_blocks_});
+    // Beside other branches of a captured batch: a solve alone is bound by latency, so several, each
+    // on a part of the chip, do more than one after the other on all of it. A half of the resident
+    // CTAs, a quarter up to 64^3, or a branch's share where that is more. Two large and six small
+    // problems, 10 steps, ms by CTAs of the large / small ones, 304 / 304, 152 / 152, 152 / 76 and
+    // 101 / 76: 128^3 + 64^3 49.5, 46.2, 44.7, 47.2; 96^3 + 48^3 28.3, 26.1, 24.0, 25.2;
+    // 64^3 + 32^3 18.3, 18.2, 16.9, 17.0. 228, which leaves no room for two, takes 57 and 33
+    if (capture_ && cap_branches_ > 1 && plane_.any_grid)
+      grid = std::min(grid, std::max(g_.n > 64 ? sms_ : sms_ / 2, 2 * sms_ / cap_branches_));
     GLIA_TIMED(KS_PLANE, bytes,
                GLIA_CUDA(cudaLaunchCooperativeKernel(plane_.fn, dim3(grid), dim3(plane_.threads),
                                                      args, plane_.smem, stream_)));
@@ -2104,7 +2112,8 @@ class Engine final : public EngineBase {
     GLIA_CUDA(cudaStreamSynchronize(stream_));
     cap_ready_ = true;
   }
-  void eval_capture() override {
+  void eval_capture(int branches) override {
+    cap_branches_ = branches;
     if (!cap_ready_) throw Error(GLIA_ERR_STATE, "eval_capture needs eval_prepare first");
     const glia_stats saved = st_;  // capturing runs nothing: the counts come with eval_finish
     capture_ = true;
@@ -2374,7 +2383,7 @@ class Engine final : public EngineBase {
     if (b < 1) return;
     plane_ = k;
     plane_res_ = sms_ * b;
-    plane_part_ = dalloc<double>((int64_t)kPlanePartials * plane_res_);
+    plane_part_ = dalloc<double>((int64_t)kPlanePartials * std::max(plane_res_, k.items));
     plane_bar_ = dalloc<unsigned>(2);
     // exp(2 pi i j / n): float2, or cos and sin in 64-bit fixed point
     using Tw = std::conditional_t<std::is_same<R, float>::value, float2, FxTw>;
@@ -2590,8 +2599,9 @@ class Engine final : public EngineBase {
   double cap_reg_ = 0;
   std::vector<double> cap_x_;
   // plane kernel (plane.cuh) of this grid size: resident CTAs, partial sums, barrier, twiddles
-  PlaneKernel plane_{nullptr, 0, 0, 0, false};
+  PlaneKernel plane_{};
   R* plane_w_ = nullptr;
+  int cap_branches_ = 1;  // evaluations that run side by side in the graph being captured
   int plane_res_ = 0;
   double* plane_part_ = nullptr;
   unsigned* plane_bar_ = nullptr;

@@ -98,6 +98,10 @@ struct PlaneGeo {
   // 32^3 108 -> 103, 64^3 256 -> 246, 112^3 1005 -> 886, 128^3 1047 -> 992, 144^3 2070 -> 1867
   static constexpr bool BOTH =
       sizeof(R) == 8 || (2 * T * R2 + NT - 1) / NT < 2 * ((T * R2 + NT - 1) / NT);
+  // float kernels with a tile per CTA keep their partial sums per work item instead of per CTA: the
+  // result does not depend on the number of CTAs, so a solve may run on fewer beside others
+  static constexpr int ITEMS = XT > 3 * N ? XT : 3 * N;
+  static constexpr bool PER_ITEM = sizeof(R) == 4 && XT <= 304;
   static_assert(R1 * R2 == N && N % 2 == 0, "decomposition");
   static_assert(R1 <= 16, "register DFT");
   static_assert(!SPLIT || (NG == 16 && N * TC <= BUF), "column block and lines fit the buffer");
@@ -507,9 +511,12 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
   C* __restrict__ const ch = A.chat;
   const R* __restrict__ const kf = A.k;
 
-  // per-CTA partial sums of slots s0 ... s0 + Q - 1, and their totals after the next barrier
+  // partial sums (per CTA, or per work item `i`) of slots s0 ... s0 + Q - 1, and their totals
+  // after the next barrier; slot `planes` holds the planes' sums, the others the columns'
   // (few FP64 operations: all threads' values go to shared memory and one warp adds each sum)
-  auto partials = [&](const double* v, int q_n, int s0) {
+  constexpr bool PI = Geo_::PER_ITEM;
+  const int stride = PI ? Geo_::ITEMS : (int)gridDim.x;
+  auto partials = [&](const double* v, int q_n, int s0, int i) {
     double* all = reinterpret_cast<double*>(buf);
     __syncthreads();
     for (int q = 0; q < q_n; q++) all[q * NT + tid] = v[q];
@@ -520,14 +527,14 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
       for (int w = 0; w < Geo_::NW; w++) x += all[q * NT + 32 * w + lane];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-      if (lane == 0) A.part[(s0 + q) * gridDim.x + blockIdx.x] = x;
+      if (lane == 0) A.part[(s0 + q) * stride + i] = x;
     }
   };
-  auto totals = [&](int q_n, int s0) {
+  auto totals = [&](int q_n, int s0, int planes) {
     for (int q = warp; q < q_n; q += Geo_::NW) {
       double x = 0;
-      for (int b = lane; b < (int)gridDim.x; b += 32)
-        x += __ldcg(&A.part[(s0 + q) * gridDim.x + b]);
+      const int count = !PI ? (int)gridDim.x : s0 + q == planes ? 3 * N : Geo_::XT;
+      for (int b = lane; b < count; b += 32) x += __ldcg(&A.part[(s0 + q) * stride + b]);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
       if (lane == 0) tot[q] = x;
@@ -562,6 +569,28 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
   // the twiddles of a task: none for index 0, where all are 1
   [[maybe_unused]] auto at_tw = [](int i, const Tw* tw) { return i ? tw : nullptr; };
   Acc<R> acc[5];
+  // the sums of a work item (PER_ITEM) or of all of a CTA's
+  auto sums = [&](int kind, int i) {
+    if (kind == PS_GRAD) {
+      const double v[1] = {acc[0].value()};
+      partials(v, 1, 1, i);
+    } else if (kind == PS_SETUP) {
+      const double v[5] = {acc[0].value(), acc[1].value(), acc[2].value(), acc[3].value(),
+                           FX ? acc[1].value() : acc[4].value()};
+      partials(v, 5, 1, i);
+    } else if (kind == PS_UPDATE || kind == PS_DOT) {
+      const double v[2] = {acc[0].value(), acc[1].value()};
+      partials(v, 2, 2, i);
+    } else if (kind == PS_DIR) {
+      const double v[1] = {acc[0].value()};
+      partials(v, 1, 0, i);
+    }
+    if constexpr (PI) {
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < 5; q++) acc[q] = Acc<R>();
+    }
+  };
   // Double: row k1 of a line pair in real space (places k2, z = k1 + R1 k2 of lines l0 and l1)
   auto line_middle = [&](int kind, C* row, int64_t l0, int64_t l1, int k1) {
     if constexpr (FX) {
@@ -685,7 +714,7 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
         }
         if (kind == PS_GRAD) {
           const double v[1] = {acc[0].value()};
-          partials(v, 1, 1);
+          partials(v, 1, 1, blockIdx.x);
         }
       }
     }
@@ -911,11 +940,9 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
             }
           }
         }
+        if (PI && step == PS_GRAD) sums(step, item);
       }
-      if (step == PS_GRAD) {
-        const double v[1] = {acc[0].value()};
-        partials(v, 1, 1);
-      }
+      if (!PI && step == PS_GRAD) sums(step, blockIdx.x);
     } else if (step >= PS_SPEC) {
       // ----------------------------------------------------------------------------- columns
       const int nin = step == PS_SPEC || step == PS_ENTER || step == PS_SMOOTH ? 1
@@ -925,7 +952,7 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
                        : step == PS_SPEC || step == PS_UPDATE || step == PS_DOT  ? 0
                                                                                  : 2;
       if (step == PS_UPDATE) {  // alpha
-        totals(2, 0);
+        totals(2, 0, 1);
         if (tid == 0) {
           if (cg.iter == 0) tot[0] = cg.pp;  // of the set-up's first direction
           cg.dpi_old = cg.dpi;
@@ -1192,18 +1219,9 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
           }
         }
         if (nout) __syncthreads();
+        if (PI) sums(step, tile);
       }
-      if (step == PS_SETUP) {
-        const double v[5] = {acc[0].value(), acc[1].value(), acc[2].value(), acc[3].value(),
-                             FX ? acc[1].value() : acc[4].value()};
-        partials(v, 5, 1);
-      } else if (step == PS_UPDATE || step == PS_DOT) {
-        const double v[2] = {acc[0].value(), acc[1].value()};
-        partials(v, 2, 2);
-      } else if (step == PS_DIR) {
-        const double v[1] = {acc[0].value()};
-        partials(v, 1, 0);
-      }
+      if (!PI) sums(step, blockIdx.x);
     }
     if (step == PS_SPEC || (Geo_::SPLIT ? step == PS_LINE && kind == PS_BACK : step == PS_BACK))
       break;
@@ -1237,7 +1255,7 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
         break;
       case PS_SETUP:
         started = true;
-        totals(5, 1);
+        totals(5, 1, -1);
         if (tid == 0) {
           double snorm = tot[0] * dinvN;
           cg.dp = tot[1] * dinvN;
@@ -1258,7 +1276,7 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
         step = cg.step;
         break;
       case PS_UPDATE:
-        totals(2, 2);
+        totals(2, 2, -1);
         if (tid == 0) {
           cg.dp = tot[0] * dinvN;
           cg.status = converged(cg.dp);
@@ -1283,7 +1301,7 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
         step = PS_GRAD;
         break;
       case PS_DOT:
-        totals(1, 2);
+        totals(1, 2, -1);
         if (blockIdx.x == 0 && tid == 0) A.sc->acc[6] += A.kdot_weight * tot[0] * dinvN * dscale;
         bar.leave();
         return;
@@ -1321,7 +1339,7 @@ template <typename R, int N>
 PlaneKernel plane_entry() {
   using P = PlaneGeo<R, N>;
   return PlaneKernel{reinterpret_cast<const void*>(&k_plane<R, N>), P::NT, P::SMEM,
-                     P::XT > 3 * N ? P::XT : 3 * N, P::SPLIT};
+                     P::ITEMS, P::SPLIT, P::PER_ITEM};
 }
 
 }  // namespace glia

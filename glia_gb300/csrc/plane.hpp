@@ -15,7 +15,7 @@ enum PlaneProg {
   PP_DOT         // acc[6] += kdot_weight <cx, D in>
 };
 
-constexpr int kPlanePartials = 6;  // partial-sum slots per CTA
+constexpr int kPlanePartials = 6;  // partial-sum slots
 
 template <typename R>
 struct PlaneArgs {
@@ -39,7 +39,7 @@ struct PlaneArgs {
   double a_cn, pc_c, rtol, abstol, divtol, kdot_weight;
   int maxit;
   DevScalars* sc;
-  double* part;    // kPlanePartials values per CTA
+  double* part;    // kPlanePartials values per CTA or work item
   unsigned* bar;   // two counters, zero between launches
   const void* tw;  // exp(2 pi i j / n), j < n: float2, or FxTw for double
   const R* pf;     // double: the preconditioner 1 / (1 + pc_c |w|^2) per spectrum element
@@ -50,6 +50,7 @@ struct PlaneKernel {
   int threads, smem;
   int items;       // most work items of a phase
   bool split;      // needs W
+  bool any_grid;   // the result does not depend on the number of CTAs
 };
 // One instantiation per grid size, in translation units by size: every multiple of 8 that factors
 // into R1 <= 16 and R2 = 4, 8 or 16 (plane.cuh). That leaves 136, 152, 168, 184, 200, 216, 232 and

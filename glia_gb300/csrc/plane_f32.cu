@@ -19,7 +19,7 @@ PlaneKernel plane_kernel_f32_small(int n) {
     case 112: return plane_entry<float, 112>();
     case 120: return plane_entry<float, 120>();
     case 128: return plane_entry<float, 128>();
-    default: return PlaneKernel{nullptr, 0, 0, 0, false};
+    default: return PlaneKernel{};
   }
 }
 }  // namespace glia

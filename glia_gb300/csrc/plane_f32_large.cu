@@ -13,7 +13,7 @@ PlaneKernel plane_kernel_f32_large(int n) {
     case 192: return plane_entry<float, 192>();
     case 208: return plane_entry<float, 208>();
     case 224: return plane_entry<float, 224>();
-    default: return PlaneKernel{nullptr, 0, 0, 0, false};
+    default: return PlaneKernel{};
   }
 }
 }  // namespace glia

@@ -15,7 +15,7 @@ PlaneKernel plane_kernel_f64_small(int n) {
     case 80: return plane_entry<double, 80>();
     case 88: return plane_entry<double, 88>();
     case 96: return plane_entry<double, 96>();
-    default: return PlaneKernel{nullptr, 0, 0, 0, false};
+    default: return PlaneKernel{};
   }
 }
 }  // namespace glia

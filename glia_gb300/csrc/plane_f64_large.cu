@@ -12,7 +12,7 @@ PlaneKernel plane_kernel_f64_large(int n) {
     case 224: return plane_entry<double, 224>();
     case 240: return plane_entry<double, 240>();
     case 256: return plane_entry<double, 256>();
-    default: return PlaneKernel{nullptr, 0, 0, 0, false};
+    default: return PlaneKernel{};
   }
 }
 }  // namespace glia

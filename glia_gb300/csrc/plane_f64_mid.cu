@@ -9,7 +9,7 @@ PlaneKernel plane_kernel_f64_mid(int n) {
     case 120: return plane_entry<double, 120>();
     case 128: return plane_entry<double, 128>();
     case 144: return plane_entry<double, 144>();
-    default: return PlaneKernel{nullptr, 0, 0, 0, false};
+    default: return PlaneKernel{};
   }
 }
 }  // namespace glia
