@@ -459,11 +459,10 @@ class Engine final : public EngineBase {
 
   // First half of a spectral D apply, from the spectrum src (plain) or from the new PCG direction
   // p = P r + b p (CGDIR: src = r, pdir = p), up to the spectra of k grad u that d_back
-  // diverges. Own transforms (default, FP32, n = 64 ... 256): k_xinv -> G in g3r_, k_yinv_bulk
-  // (or k_yinv) -> packed lines in g3s_, k_zpass2 (or k_zpass; k multiplied there, in place),
-  // k_yfwd -> M in g3r_. "2d": the
-  // x pass writes (x, ky, kz) per component to g3s_ and cuFFT does batched 2-D (y, z)
-  // transforms around k_mul_k3. Otherwise g3s_ holds the full 3-D spectra.
+  // diverges. Grids without a plane kernel. Own transforms (FP32, n = 256): k_xinv -> G in g3r_,
+  // k_yinv_bulk (or k_yinv) -> packed lines in g3s_, k_zpass2 (k multiplied there, in place),
+  // k_yfwd -> M in g3r_. "2d": the x pass writes (x, ky, kz) per component to g3s_ and cuFFT does
+  // batched 2-D (y, z) transforms around k_mul_k3. Otherwise g3s_ holds the full 3-D spectra.
   template <bool CGDIR>
   void d_front(const R* src, R* pdir) {
     if (own_) {  // no cuFFT: x, y, z passes of our own, k multiplied inside the z pass
@@ -2325,14 +2324,14 @@ class Engine final : public EngineBase {
                                 stream_));
       GLIA_CUDA(cudaStreamSynchronize(stream_));
     }
-    // Transform path of the FP32 D apply at n = 64, 128, 256 (GLIA_XPASS): by default the x, y
-    // and z passes are the library's own kernels (ownfft.cuh, no cuFFT inside the PCG loop);
-    // "2d" keeps the x pass and lets cuFFT do batched 2-D (y, z) transforms with k multiplied in
-    // between; "0" uses batched 3-D cuFFT transforms.
+    // Transform path of the D apply (GLIA_XPASS). By default the plane kernel of the grid size
+    // (plane.hpp), or in FP32 at n = 256 own x, y and z passes (ownfft.cuh, no cuFFT inside the PCG
+    // loop), or else batched 3-D cuFFT transforms. "2d" (FP32, n = 64, 128, 256): own x pass, cuFFT
+    // for batched 2-D (y, z) transforms with k multiplied in between; "0": cuFFT.
     const char* xenv = std::getenv("GLIA_XPASS");
     xpass_ = std::is_same<R, float>::value && (n == 64 || n == 128 || n == 256) && !zpass_ &&
              !ref_ && !(xenv && xenv[0] == '0');
-    own_ = xpass_ && !(xenv && std::strcmp(xenv, "2d") == 0);
+    own_ = xpass_ && n == 256 && !(xenv && std::strcmp(xenv, "2d") == 0);
     // Grids with a plane kernel run every solve as one launch, in either precision.
     if (!ref_ && !zpass_ && !(xenv && (xenv[0] == '0' || std::strcmp(xenv, "2d") == 0)))
       init_plane();

@@ -40,7 +40,7 @@ enum KSlot {
   KS_XFWD_CGW,           // k_xfwd<EPI_CGW>: forward x transforms, divergence, w = A p
   KS_XFWD_APPLYD,        // k_xfwd<EPI_APPLYD>: forward x transforms, divergence, D u
   KS_YINV,               // k_yinv_bulk (or k_yinv): inverse y transforms, packed kz = 0 / n/2
-  KS_ZFUSED,             // k_zpass2 (or k_zpass): z C2R, k multiply, z R2C per line
+  KS_ZFUSED,             // k_zpass2: z C2R, k multiply, z R2C per line
   KS_YFWD,               // k_yfwd: forward y transforms, unpacking
   KS_XFWD_CGU,           // k_xfwd_own<EPI_CGU>: forward x transforms, w = A p, x and r updated
   KS_PLANE,              // k_plane: a whole solve (or D apply, transform) of a small grid

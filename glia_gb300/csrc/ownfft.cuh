@@ -36,14 +36,6 @@ template <>
 struct YDecomp<256> {
   static constexpr int N = 256, R1 = 16, R2 = 16, T = 16;
 };
-template <>
-struct YDecomp<128> {
-  static constexpr int N = 128, R1 = 16, R2 = 8, T = 32;
-};
-template <>
-struct YDecomp<64> {
-  static constexpr int N = 64, R1 = 8, R2 = 8, T = 32;
-};
 
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);

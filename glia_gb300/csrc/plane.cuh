@@ -22,13 +22,13 @@
 // took 7 kernels and a conditional graph node an iteration and a graph launch a solve, 35 to 60 us
 // an iteration whatever the size. A barrier costs 1.0 us, a phase at 64^3 4 to 10 us (float).
 // In FP64 the arithmetic is the bound, see fx.cuh. Measured on GB300, before -> after:
-//   mixed  gradient  32^3, 16 steps   14.5 -> 6.8 ms      64^3, 40 steps   41.6 -> 24.9 ms
-//          forward   96^3, 20 steps   13.9 -> 6.2 ms
-//          gradient 128^3, 40 steps   88.0 -> 84.0 ms
-//   FP64   forward   64^3, 100 steps   151 -> 46.5 ms
-//          gradient 128^3, 6 steps     164 -> 34.5 ms
-//          adjoint  120^3, 2 steps    48.7 -> 11.5 ms
-//          solve    256^3               45 -> 10.3 ms
+//   mixed  gradient  32^3, 16 steps   14.5 -> 6.6 ms      64^3, 40 steps   40.5 -> 23.5 ms
+//          forward   96^3, 20 steps   13.8 -> 5.9 ms
+//          gradient 128^3, 40 steps   88.0 -> 81.5 ms
+//   FP64   forward   64^3, 100 steps   151 -> 45.5 ms
+//          gradient 128^3, 6 steps     166 -> 32.8 ms
+//          adjoint  120^3, 2 steps    48.7 -> 10.5 ms
+//          solve    256^3               49 -> 10.7 ms
 //
 // N = R1 R2 (R2 a power of two, so that a group of R2 threads is part of a warp). Inverse
 // transforms read index R2 a + b (R1-point DFTs over a, twiddle w^(b k1), R2-point DFTs over b) and

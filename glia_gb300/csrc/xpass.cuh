@@ -1,5 +1,5 @@
 // xpass.cuh — the x direction of the spectral D apply, fused into the kernels that already stream
-// the spectra (FP32, n = 64, 128, 256).
+// the spectra (FP32; n = 256 by default, 64, 128 and 256 around 2-D cuFFT transforms).
 //
 // A three-dimensional transform is a 2-D transform over (y, z) for every x plus a 1-D transform
 // along x. cuFFT does the (y, z) part as a contiguous batched 2-D transform; these kernels do the
@@ -152,8 +152,8 @@ __device__ __forceinline__ void xdft(float2* sm, const float2* twb, int c, int g
 // so two x transforms give the three components: G_x = F^-1(i w_x u) / N and
 // G_y, G_z = i w_y, i w_z F^-1(u) / N. The inputs of the CTA's next tile are staged into shared
 // memory (cp.async) while the current tile is transformed.
-// OUT2 (own y / z passes): in MODE 1 also sum |p|^2 (DevScalars::pp); two arrays out, [G_x, G_0] with G_0 = F^-1(u) / N; otherwise three,
-// [G_x, G_y, G_z].
+// OUT2 (own y / z passes): two arrays out, [G_x, G_0] with G_0 = F^-1(u) / N, and in MODE 1 also
+// sum |p|^2 (DevScalars::pp); otherwise three, [G_x, G_y, G_z].
 template <int NN, int MODE, bool OUT2>
 __global__ void __launch_bounds__(256, 2)
     k_xinv(Geo g, const float* __restrict__ src, float* __restrict__ pdir, float* __restrict__ G3,

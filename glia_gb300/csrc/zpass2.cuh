@@ -29,14 +29,6 @@ template <>
 struct Z2Decomp<256> {
   static constexpr int R1 = 16, R2 = 16;
 };
-template <>
-struct Z2Decomp<128> {
-  static constexpr int R1 = 16, R2 = 8;
-};
-template <>
-struct Z2Decomp<64> {
-  static constexpr int R1 = 8, R2 = 8;
-};
 
 template <int NN>
 struct Z2Geom {
