@@ -15,8 +15,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT_DIR, "libglia_rd.so")
-UNITS = ["capi.cu", "engine_f32.cu", "engine_f64.cu", "noalloc.cu", "plane_f32.cu",
-         "plane_f32_large.cu", "plane_f64.cu", "plane_f64_mid.cu", "plane_f64_large.cu"]
+UNITS = ["capi.cu", "engine_f32.cu", "engine_f64.cu", "noalloc.cu", "plane_f64.cu",
+         "plane_f64_mid.cu", "plane_f64_large.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
          "-Xcompiler", "-Wno-unknown-pragmas"]

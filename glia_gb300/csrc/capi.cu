@@ -405,7 +405,7 @@ int glia_batch_capture(glia_batch* b, const double* const* x, const int* nx,
           cudaStream_t s = static_cast<cudaStream_t>(c->eng->stream());
           BATCH_CUDA(cudaStreamWaitEvent(s, start, 0));  // fork: the branch joins the capture
           try {
-            c->eng->eval_capture((int)kv.second.size());
+            c->eng->eval_capture();
           } catch (const glia::Error& e) {
             c->err = e.what();
             throw glia::Error(e.code, "context " + std::to_string(i) + ": " + e.what());

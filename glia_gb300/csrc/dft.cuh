@@ -1,9 +1,9 @@
-// dft.cuh — small DFTs in registers, for float2 and double2.
+// dft.cuh — small DFTs in registers, of doubles and of 64-bit fixed-point values (fx.cuh).
 //
-// X[k] = sum_j v[j] exp(S 2 pi i j k / R), natural order in and out, R = 2 ... 16. Powers of two are radix-4 butterflies (the factors +-i and -1 are
-// sign changes and swaps, never multiplications); R = A B with coprime A, B is the prime-factor
-// mapping of Good and Thomas (no twiddles between the two parts); 9 = 3 x 3 has twiddles; odd
-// primes use the symmetric sums x[j] +- x[p - j].
+// X[k] = sum_j v[j] exp(S 2 pi i j k / R), natural order in and out, R = 2 ... 16. Powers of two are
+// radix-4 butterflies (the factors +-i and -1 are sign changes and swaps, never multiplications);
+// R = A B with coprime A, B is the prime-factor mapping of Good and Thomas (no twiddles between the
+// two parts); 9 = 3 x 3 has twiddles; odd primes use the symmetric sums x[j] +- x[p - j].
 #pragma once
 
 #include <cuda_runtime.h>
@@ -20,10 +20,6 @@ __host__ __device__ __forceinline__ fx2 ctw_fx(fx2 z);
 template <int R, int S>
 __host__ __device__ __forceinline__ void odd_dft_fx(fx2 (&v)[R]);
 template <>
-struct CReal<float2> {
-  using type = float;
-};
-template <>
 struct CReal<double2> {
   using type = double;
 };
@@ -37,44 +33,17 @@ __host__ __device__ __forceinline__ C cmk(creal_t<C> x, creal_t<C> y) {
   c.y = y;
   return c;
 }
-// float2: one packed instruction (sm_100 and later) instead of two, the same roundings. The z pass at
-// 256^3, bound by instruction issue: 115 -> 108 us (with the sum of k |grad p|^2).
 template <class C>
 __host__ __device__ __forceinline__ C cadd(C a, C b) {
-#ifdef __CUDA_ARCH__
-  if constexpr (std::is_same<C, float2>::value) {
-    float2 r;
-    asm("{.reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n"
-        " add.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;}"
-        : "=f"(r.x), "=f"(r.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return r;
-  }
-#endif
   return cmk<C>(a.x + b.x, a.y + b.y);
 }
 template <class C>
 __host__ __device__ __forceinline__ C csub(C a, C b) {
-#ifdef __CUDA_ARCH__
-  if constexpr (std::is_same<C, float2>::value) {
-    float2 r;
-    asm("{.reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n"
-        " sub.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;}"
-        : "=f"(r.x), "=f"(r.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return r;
-  }
-#endif
   return cmk<C>(a.x - b.x, a.y - b.y);
 }
 template <class C>
 __host__ __device__ __forceinline__ C cmul2(C a, C b) {
   return cmk<C>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-// a times conj(b)
-template <class C>
-__host__ __device__ __forceinline__ C cmulc(C a, C b) {
-  return cmk<C>(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
 }
 // i w a
 template <class C>

@@ -51,10 +51,10 @@ class EngineBase {
   // An evaluation split for CUDA-graph capture (batches): eval_prepare does the host-dependent
   // part for x and d1 (coefficients, Phi p, data upload); eval_capture enqueues the forward,
   // residual, adjoint and gradient sweeps on the context's stream while that stream is being
-  // captured, with no host synchronisation (branches: evaluations of the graph that run side by
-  // side, this one included); eval_finish reads the results after the captured graph has run.
+  // captured, with no host synchronisation; eval_finish reads the results after the captured
+  // graph has run.
   virtual void eval_prepare(const double* x, int nx, const void* d1) = 0;
-  virtual void eval_capture(int branches) = 0;
+  virtual void eval_capture() = 0;
   virtual void eval_finish(double* J, double* dJ) = 0;
   virtual void* stream() const = 0;
   virtual glia_stats stats() const = 0;

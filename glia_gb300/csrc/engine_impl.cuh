@@ -26,7 +26,6 @@
 #include "zpass2.cuh"
 #include "zpass.cuh"
 #include "ownfft.cuh"
-#include "fx.cuh"
 #include "plane.hpp"
 
 #define GLIA_TIMED(slot, bytes, ...)             \
@@ -323,7 +322,7 @@ class Engine final : public EngineBase {
   // which: 0 state, 1 adjoint, 2 other (set-up, recomputation) for the iteration counters.
   // The fused engine does not wait for the solve: its outcome is folded into device counters
   // that sync_sweep() reads once per sweep.
-  // pre: a reaction step taken on c first (fused engine with a plane kernel only).
+  // pre: a reaction step taken on c first (with a plane kernel only).
   struct Pre {
     int mode = 0;  // PlaneArgs::pre
     const R* lin = nullptr;
@@ -348,20 +347,23 @@ class Engine final : public EngineBase {
   }
 
   // Arguments and launch of the grid's plane kernel (plane.cuh), all CTAs resident at once.
-  PlaneArgs<R> plane_args(int prog, const R* in, R* out, R* chat) {
-    using C = typename CT<R>::C;
-    PlaneArgs<R> a{};
+  static constexpr bool kPlane = std::is_same<R, double>::value;
+  bool plane() const { return plane_.fn != nullptr; }
+  static double2* cx2(R* p) { return reinterpret_cast<double2*>(p); }
+  static const double2* cx2(const R* p) { return reinterpret_cast<const double2*>(p); }
+  PlaneArgs plane_args(int prog, const R* in, R* out, R* chat) {
+    PlaneArgs a{};
     a.prog = prog;
     a.in = in;
     a.out = out;
     a.k = kxx_;
-    a.chat = reinterpret_cast<C*>(chat);
-    a.xhat = reinterpret_cast<C*>(xhat_);
-    a.rhat = reinterpret_cast<C*>(rhat_);
-    a.phat = reinterpret_cast<C*>(phat_);
-    a.G = reinterpret_cast<C*>(g3r_);
-    a.M = reinterpret_cast<C*>(g3s_);
-    a.W = reinterpret_cast<C*>(plane_w_);
+    a.chat = cx2(chat);
+    a.xhat = cx2(xhat_);
+    a.rhat = cx2(rhat_);
+    a.phat = cx2(phat_);
+    a.G = cx2(g3r_);
+    a.M = cx2(g3s_);
+    a.W = cx2(plane_w_);
     a.sc = sc_;
     a.part = plane_part_;
     a.bar = plane_bar_;
@@ -369,69 +371,57 @@ class Engine final : public EngineBase {
     a.pf = plane_pf_;
     return a;
   }
-  void plane_launch(PlaneArgs<R>& a, double bytes) {
+  void plane_launch(PlaneArgs& a, double bytes) {
     void* args[] = {&a};
-    int grid = std::min({plane_.items, plane_res_, red_blocks_});
-    // Beside other branches of a captured batch: a solve alone is bound by latency, so several, each
-    // on a part of the chip, do more than one after the other on all of it. A half of the resident
-    // CTAs, a quarter up to 64^3, or a branch's share where that is more. Two large and six small
-    // problems, 10 steps, ms by CTAs of the large / small ones, 304 / 304, 152 / 152, 152 / 76 and
-    // 101 / 76: 128^3 + 64^3 49.5, 46.2, 44.7, 47.2; 96^3 + 48^3 28.3, 26.1, 24.0, 25.2;
-    // 64^3 + 32^3 18.3, 18.2, 16.9, 17.0. 228, which leaves no room for two, takes 57 and 33
-    if (capture_ && cap_branches_ > 1 && plane_.any_grid)
-      grid = std::min(grid, std::max(g_.n > 64 ? sms_ : sms_ / 2, 2 * sms_ / cap_branches_));
+    const int grid = std::min({plane_.items, plane_res_, red_blocks_});
     GLIA_TIMED(KS_PLANE, bytes,
                GLIA_CUDA(cudaLaunchCooperativeKernel(plane_.fn, dim3(grid), dim3(plane_.threads),
                                                      args, plane_.smem, stream_)));
   }
-  bool plane() const { return plane_.fn != nullptr; }
-  // Whether the plane kernel also takes a solve's two ends (real field <-> spectrum): in FP64. The
-  // mixed engine keeps cuFFT there: each FP32 round trip c -> spectrum -> c loses a little of the
-  // field (2.2e-7 of a smooth one at 64^3 with cuFFT, 0.7e-7 with the plane kernel), the same way
-  // every time, and hundreds of solves add up to 1e-5 and more, so the ends decide which answer
-  // within the path's accuracy a simulation gives. Users' answers stay where they were.
-  bool plane_ends() const { return std::is_same<R, double>::value; }
   // spectrum of a real field
   void spectrum(const R* in, R* out) {
-    if (!plane() || !plane_ends()) {
-      r2c(r2c1_, in, out);
-      return;
+    if constexpr (kPlane) {
+      if (plane()) {
+        PlaneArgs a = plane_args(PP_SPEC, in, nullptr, out);
+        plane_launch(a, FB() + SB());
+        st_.total_fft_execs += 1;
+        return;
+      }
     }
-    PlaneArgs<R> a = plane_args(PP_SPEC, in, nullptr, out);
-    plane_launch(a, FB() + SB());
-    st_.total_fft_execs += 1;
+    r2c(r2c1_, in, out);
+  }
+  void plane_solve(R* c, double dts, R* chat, const R* cx, double kdot_w, int which, Pre pre) {
+    PlaneArgs a = plane_args(PP_SOLVE, c, c, chat);
+    a.which = which;
+    a.pre = pre.mode;
+    a.rho = rho_;
+    a.lin = pre.lin;
+    a.half = pre.half;
+    a.dt = dt_;
+    a.cx = cx2(cx);
+    a.a_cn = 0.5 * dts;
+    a.pc_c = 0.25 * pc_dt_ * pc_kbar_;
+    if (plane_pc_ != a.pc_c) {
+      k_pc_field<R><<<pw_blocks_, kThreads, 0, stream_>>>(g_, plane_pf_, a.pc_c);
+      GLIA_LAUNCH_CHECK();
+      plane_pc_ = a.pc_c;
+    }
+    a.rtol = rtol_;
+    a.abstol = abstol_;
+    a.divtol = divtol_;
+    a.maxit = maxit_;
+    a.kdot_weight = kdot_w;
+    plane_launch(a, 3 * FB());  // c in and out, k
+    graph_solves_ = true;
+    st_.total_fft_execs += 2;
   }
 
   void fused_solve(R* c, double dts, R* chat, const R* cx, double kdot_w, int which, Pre pre) {
-    if (plane()) {
-      if (!plane_ends()) r2c(r2c1_, c, chat);
-      PlaneArgs<R> a = plane_args(plane_ends() ? PP_SOLVE : PP_SOLVE_SPEC, c, c, chat);
-      a.which = which;
-      a.pre = pre.mode;
-      a.rho = rho_;
-      a.lin = pre.lin;
-      a.half = pre.half;
-      a.dt = (R)dt_;
-      a.cx = reinterpret_cast<const typename CT<R>::C*>(cx);
-      a.a_cn = 0.5 * dts;
-      a.pc_c = 0.25 * pc_dt_ * pc_kbar_;
-      if (plane_pf_ && plane_pc_ != a.pc_c) {
-        k_pc_field<R><<<pw_blocks_, kThreads, 0, stream_>>>(g_, plane_pf_, a.pc_c);
-        GLIA_LAUNCH_CHECK();
-        plane_pc_ = a.pc_c;
+    if constexpr (kPlane) {
+      if (plane()) {
+        plane_solve(c, dts, chat, cx, kdot_w, which, pre);
+        return;
       }
-      a.rtol = rtol_;
-      a.abstol = abstol_;
-      a.divtol = divtol_;
-      a.maxit = maxit_;
-      a.kdot_weight = kdot_w;
-      plane_launch(a, 3 * FB());  // c in and out, k
-      graph_solves_ = true;
-      if (plane_ends())
-        st_.total_fft_execs += 2;
-      else
-        c2r(c2r1_, xhat_, c);
-      return;
     }
     k_solve_config<<<1, 1, 0, stream_>>>(sc_, 0.5 * dts, 0.25 * pc_dt_ * pc_kbar_, rtol_, abstol_,
                                          divtol_, maxit_, kdot_w);
@@ -459,17 +449,18 @@ class Engine final : public EngineBase {
 
   // First half of a spectral D apply, from the spectrum src (plain) or from the new PCG direction
   // p = P r + b p (CGDIR: src = r, pdir = p), up to the spectra of k grad u that d_back
-  // diverges. Grids without a plane kernel. Own transforms (FP32, n = 256): k_xinv -> G in g3r_,
-  // k_yinv_bulk (or k_yinv) -> packed lines in g3s_, k_zpass2 (k multiplied there, in place),
-  // k_yfwd -> M in g3r_. "2d": the x pass writes (x, ky, kz) per component to g3s_ and cuFFT does
-  // batched 2-D (y, z) transforms around k_mul_k3. Otherwise g3s_ holds the full 3-D spectra.
+  // diverges. Own transforms (default, FP32, n = 64 ... 256): k_xinv -> G in g3r_, k_yinv_bulk
+  // (or k_yinv) -> packed lines in g3s_, k_zpass2 (or k_zpass; k multiplied there, in place),
+  // k_yfwd -> M in g3r_. "2d": the
+  // x pass writes (x, ky, kz) per component to g3s_ and cuFFT does batched 2-D (y, z)
+  // transforms around k_mul_k3. Otherwise g3s_ holds the full 3-D spectra.
   template <bool CGDIR>
   void d_front(const R* src, R* pdir) {
     if (own_) {  // no cuFFT: x, y, z passes of our own, k multiplied inside the z pass
       GLIA_TIMED(KS_XINV, SB() * (CGDIR ? 5 : 3), launch_xinv<CGDIR>(src, pdir));
-      GLIA_TIMED(KS_YINV, SB() * 2 + FB() * 3, launch_own(0, CGDIR));
-      GLIA_TIMED(KS_ZFUSED, FB() * 7, launch_own(1, CGDIR));
-      GLIA_TIMED(KS_YFWD, FB() * 3 + SB() * 2, launch_own(2, CGDIR));
+      GLIA_TIMED(KS_YINV, SB() * 2 + FB() * 3, launch_own(0));
+      GLIA_TIMED(KS_ZFUSED, FB() * 7, launch_own(1));
+      GLIA_TIMED(KS_YFWD, FB() * 3 + SB() * 2, launch_own(2));
       return;
     }
     if (xpass_) {
@@ -510,16 +501,21 @@ class Engine final : public EngineBase {
       constexpr int MODE = CGDIR ? 1 : 0;
       const int grid = std::min(xres_inv_, pw_blocks_);
       k_xinv<NN, MODE, OUT2><<<grid, 256, xinv_smem_bytes<NN, MODE>(), stream_>>>(
-          g_, src, pdir, G, sc_, ws_, tw256_);
+          g_, src, pdir, G, sc_, tw256_);
     }
   }
   template <bool CGDIR>
   void launch_xinv(const R* src, R* pdir) {
     const int n = g_.n;
-    if (own_) xinv_n<256, CGDIR, true>(src, pdir, g3r_);
-    else if (n == 256) xinv_n<256, CGDIR, false>(src, pdir, g3s_);
-    else if (n == 128) xinv_n<128, CGDIR, false>(src, pdir, g3s_);
-    else xinv_n<64, CGDIR, false>(src, pdir, g3s_);
+    if (own_) {
+      if (n == 256) xinv_n<256, CGDIR, true>(src, pdir, g3r_);
+      else if (n == 128) xinv_n<128, CGDIR, true>(src, pdir, g3r_);
+      else xinv_n<64, CGDIR, true>(src, pdir, g3r_);
+    } else {
+      if (n == 256) xinv_n<256, CGDIR, false>(src, pdir, g3s_);
+      else if (n == 128) xinv_n<128, CGDIR, false>(src, pdir, g3s_);
+      else xinv_n<64, CGDIR, false>(src, pdir, g3s_);
+    }
   }
   template <int NN, int EPI, bool IN2>
   void xfwd_n(const R* G, const R* aux_in, const R* cx, R* out, R* aux_out, R scale, int blocks) {
@@ -537,8 +533,10 @@ class Engine final : public EngineBase {
     const int n = g_.n;
     blocks = std::min(xres_fwd_, blocks);
     if (own_) {
-      xfwd_n<256, EPI, true>(g3r_, aux_in, cx, out, aux_out, scale, blocks);
-    } else if constexpr (EPI != EPI_CGU) {
+      if (n == 256) xfwd_n<256, EPI, true>(g3r_, aux_in, cx, out, aux_out, scale, blocks);
+      else if (n == 128) xfwd_n<128, EPI, true>(g3r_, aux_in, cx, out, aux_out, scale, blocks);
+      else xfwd_n<64, EPI, true>(g3r_, aux_in, cx, out, aux_out, scale, blocks);
+    } else {
       if (n == 256) xfwd_n<256, EPI, false>(g3s_, aux_in, cx, out, aux_out, scale, blocks);
       else if (n == 128) xfwd_n<128, EPI, false>(g3s_, aux_in, cx, out, aux_out, scale, blocks);
       else xfwd_n<64, EPI, false>(g3s_, aux_in, cx, out, aux_out, scale, blocks);
@@ -546,28 +544,34 @@ class Engine final : public EngineBase {
   }
   // own y / z passes: 0 = y inverse (g3r_ -> g3s_), 1 = z pass (g3s_ in place, k), 2 = k_yfwd
   // (g3s_ -> g3r_)
-  // dot: the z pass also sets alpha (PCG iterations)
-  void launch_own(int which, bool dot) {
+  template <int NN>
+  void own_n(int which) {
     if constexpr (std::is_same<R, float>::value) {
-      constexpr int NN = 256;
-      const int grid = std::min(own_res_[which], pw_blocks_);
       if (which == 0 && yinv_bulk_)
-        k_yinv_bulk<NN><<<grid, 256, yinv_bulk_smem_bytes<NN>(), stream_>>>(g3r_, g3s_, tw256_,
-                                                                             sc_);
+        k_yinv_bulk<NN><<<std::min(own_res_[0], pw_blocks_), 256, yinv_bulk_smem_bytes<NN>(),
+                          stream_>>>(g3r_, g3s_, tw256_, sc_);
       else if (which == 0)
-        k_yinv<NN><<<grid, 256, yinv_smem_bytes<NN>(), stream_>>>(g3r_, g3s_, tw256_);
-      else if (which == 1 && dot)
-        k_zpass2<NN, true><<<std::min(grid, red_blocks_), 256, zpass2_smem_bytes<NN>(), stream_>>>(
-            g3s_, kxx_, tw256_, zrev_, sc_, ws_, g_.invN);
+        k_yinv<NN><<<std::min(own_res_[0], pw_blocks_), 256, yinv_smem_bytes<NN>(), stream_>>>(
+            g3r_, g3s_, tw256_);
+      else if (which == 1 && zpass2_)
+        k_zpass2<NN><<<std::min(own_res_[1], pw_blocks_), 256, zpass2_smem_bytes<NN>(),
+                       stream_>>>(g3s_, kxx_, tw256_, zrev_);
       else if (which == 1)
-        k_zpass2<NN, false><<<grid, 256, zpass2_smem_bytes<NN>(), stream_>>>(
-            g3s_, kxx_, tw256_, zrev_, sc_, ws_, g_.invN);
+        k_zpass<NN><<<std::min(own_res_[1], pw_blocks_), 256, zpass_smem_bytes<NN>(), stream_>>>(
+            g3s_, kxx_, tw256_);
       else if (tma_)
-        k_yfwd_tma<NN><<<grid, 256, yfwd_tma_smem_bytes<NN>(), stream_>>>(kmap_, g3r_, tw256_,
-                                                                           sc_);
+        k_yfwd_tma<NN><<<std::min(own_res_[2], pw_blocks_), 256, yfwd_tma_smem_bytes<NN>(),
+                         stream_>>>(kmap_, g3r_, tw256_, sc_);
       else
-        k_yfwd<NN><<<grid, 256, yfwd_smem_bytes<NN>(), stream_>>>(g3s_, g3r_, tw256_);
+        k_yfwd<NN><<<std::min(own_res_[2], pw_blocks_), 256, yfwd_smem_bytes<NN>(), stream_>>>(
+            g3s_, g3r_, tw256_);
     }
+  }
+  void launch_own(int which) {
+    const int n = g_.n;
+    if (n == 256) own_n<256>(which);
+    else if (n == 128) own_n<128>(which);
+    else own_n<64>(which);
   }
   // resident CTAs of the x-pass and own-transform kernels on this device (persistent grids:
   // every CTA walks the same number of tiles to within one)
@@ -581,27 +585,31 @@ class Engine final : public EngineBase {
         GLIA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, 256, smem));
         return std::max(1, std::min(b, kMaxRedBlocksPerSm));
       };
-      if constexpr (NN == 256) if (own_) {
+      if (own_) {
         xres_inv_ = sms_ * std::min(per_sm(k_xinv<NN, 0, true>, xinv_smem_bytes<NN, 0>()),
                                     per_sm(k_xinv<NN, 1, true>, xinv_smem_bytes<NN, 1>()));
         constexpr int fs = xfwd_own_smem_bytes<NN>();
         xres_fwd_ = sms_ * std::min({per_sm(k_xfwd_own<NN, EPI_APPLYD>, fs),
                                      per_sm(k_xfwd_own<NN, EPI_SETUP>, fs),
-                                     per_sm(k_xfwd_own<NN, EPI_CGU>, fs)});
+                                     per_sm(k_xfwd_own<NN, EPI_CGW>, fs)});
         // y-inverse rows staged by bulk copies (default) or per-thread cp.async
         // (GLIA_YINV_BULK=0)
         const char* yb = std::getenv("GLIA_YINV_BULK");
         yinv_bulk_ = !(yb && yb[0] == '0');
         own_res_[0] = sms_ * (yinv_bulk_ ? per_sm(k_yinv_bulk<NN>, yinv_bulk_smem_bytes<NN>())
                                          : per_sm(k_yinv<NN>, yinv_smem_bytes<NN>()));
+        // z pass: two real lines per complex transform (k_zpass2) unless GLIA_ZPASS2=0 picks
+        // the even/odd half-length version (k_zpass)
+        const char* z2 = std::getenv("GLIA_ZPASS2");
+        zpass2_ = !(z2 && z2[0] == '0');
         // z pass over its line blocks in descending order (default; GLIA_ZREV=0 ascending): the
         // y-inverse pass before it writes the lines in ascending order, so the z pass starts on
         // the lines still in L2, and the y-forward pass after it (ascending) starts on the lines
         // the z pass wrote last
         const char* zr = std::getenv("GLIA_ZREV");
         zrev_ = !(zr && zr[0] == '0');
-        own_res_[1] = sms_ * std::min(per_sm(k_zpass2<NN, false>, zpass2_smem_bytes<NN>()),
-                                      per_sm(k_zpass2<NN, true>, zpass2_smem_bytes<NN>()));
+        own_res_[1] = sms_ * (zpass2_ ? per_sm(k_zpass2<NN>, zpass2_smem_bytes<NN>())
+                                      : per_sm(k_zpass<NN>, zpass_smem_bytes<NN>()));
         const char* te = std::getenv("GLIA_TMA");
         tma_ = te && te[0] == '1';
         own_res_[2] = sms_ * (tma_ ? per_sm(k_yfwd_tma<NN>, yfwd_tma_smem_bytes<NN>())
@@ -610,9 +618,7 @@ class Engine final : public EngineBase {
         // 2T floats x n rows (used by k_yfwd<TMA = true>, GLIA_TMA=1)
         if (tma_)
           kmap_ = make_tmap_f32_2d(g3s_, (uint64_t)NN, 3ull * NN * NN, 2 * YDecomp<NN>::T, NN);
-        return;
-      }
-      {
+      } else {
         xres_inv_ = sms_ * std::min(per_sm(k_xinv<NN, 0, false>, xinv_smem_bytes<NN, 0>()),
                                     per_sm(k_xinv<NN, 1, false>, xinv_smem_bytes<NN, 1>()));
         xres_fwd_ = sms_ * std::min({per_sm(k_xfwd<NN, EPI_APPLYD>, 0),
@@ -625,11 +631,6 @@ class Engine final : public EngineBase {
   // one PCG iteration of the fused engine (launched directly, or captured as the loop body)
   void cg_iteration() {
     d_front<true>(rhat_, phat_);  // p = P r + b p and the spectra of k grad p
-    if (own_) {  // alpha is known: w = A p and the update of x and r in one pass
-      GLIA_TIMED(KS_XFWD_CGU, SB() * 7,
-                 launch_xfwd<EPI_CGU>(phat_, rhat_, xhat_, rhat_, R(0), red_blocks_));
-      return;
-    }
     d_back<EPI_CGW>(phat_, nullptr, what_, nullptr, R(0));  // w = A p, <p, w>, alpha
     GLIA_TIMED(KS_CG_UPDATE, SB() * 6,
                k_cg_update<R><<<red_blocks_, kThreads, 0, stream_>>>(g_, xhat_, phat_, rhat_,
@@ -999,11 +1000,13 @@ class Engine final : public EngineBase {
       ref_applyD(dc, c);
       return;
     }
-    if (plane()) {
-      PlaneArgs<R> a = plane_args(PP_APPLY, c, dc, chat_);
-      plane_launch(a, 3 * FB());
-      st_.total_fft_execs += 2;
-      return;
+    if constexpr (kPlane) {
+      if (plane()) {
+        PlaneArgs a = plane_args(PP_APPLY, c, dc, chat_);
+        plane_launch(a, 3 * FB());
+        st_.total_fft_execs += 2;
+        return;
+      }
     }
     r2c(r2c1_, c, chat_);
     d_front<false>(chat_, nullptr);
@@ -1073,12 +1076,14 @@ class Engine final : public EngineBase {
       return;
     }
     const R* K = smoother_kernel(sigma);
-    if (plane()) {
-      PlaneArgs<R> a = plane_args(PP_SMOOTH, in, out, chat_);
-      a.mulk = reinterpret_cast<const typename CT<R>::C*>(K);
-      plane_launch(a, 2 * FB() + SB());
-      st_.total_fft_execs += 2;
-      return;
+    if constexpr (kPlane) {
+      if (plane()) {
+        PlaneArgs a = plane_args(PP_SMOOTH, in, out, chat_);
+        a.mulk = cx2(K);
+        plane_launch(a, 2 * FB() + SB());
+        st_.total_fft_execs += 2;
+        return;
+      }
     }
     r2c(r2c1_, in, chat_);
     k_spec_mul<R><<<pw_blocks_, kThreads, 0, stream_>>>(Ns_, 1, chat_, K);
@@ -1541,7 +1546,7 @@ class Engine final : public EngineBase {
   // half; 2: linearised at lin): a plane kernel takes it as it reads the field of the next solve,
   // otherwise it runs here.
   Pre react(R* c, int mode, const R* lin, R* half) {
-    if (plane() && plane_ends() && k_scale_ != 0) return Pre{mode, lin, half};
+    if (plane() && k_scale_ != 0) return Pre{mode, lin, half};
     if (mode == 1)
       reaction(c, half);
     else
@@ -1814,13 +1819,15 @@ class Engine final : public EngineBase {
   }
   // acc[6] += w <c_0, D alpha_0>: a D apply on alpha_0 whose spectral epilogue takes the dot
   void kappa_dot_at(const R* chat0, double w) {
-    if (plane()) {
-      PlaneArgs<R> a = plane_args(PP_DOT, p0_, nullptr, xhat_);
-      a.cx = reinterpret_cast<const typename CT<R>::C*>(chat0);
-      a.kdot_weight = w;
-      plane_launch(a, 2 * FB() + SB());
-      st_.total_fft_execs += 1;
-      return;
+    if constexpr (kPlane) {
+      if (plane()) {
+        PlaneArgs a = plane_args(PP_DOT, p0_, nullptr, xhat_);
+        a.cx = cx2(chat0);
+        a.kdot_weight = w;
+        plane_launch(a, 2 * FB() + SB());
+        st_.total_fft_execs += 1;
+        return;
+      }
     }
     k_solve_config<<<1, 1, 0, stream_>>>(sc_, 0.0, 0.0, rtol_, abstol_, divtol_, maxit_, w);
     GLIA_LAUNCH_CHECK();
@@ -2111,8 +2118,7 @@ class Engine final : public EngineBase {
     GLIA_CUDA(cudaStreamSynchronize(stream_));
     cap_ready_ = true;
   }
-  void eval_capture(int branches) override {
-    cap_branches_ = branches;
+  void eval_capture() override {
     if (!cap_ready_) throw Error(GLIA_ERR_STATE, "eval_capture needs eval_prepare first");
     const glia_stats saved = st_;  // capturing runs nothing: the counts come with eval_finish
     capture_ = true;
@@ -2324,18 +2330,26 @@ class Engine final : public EngineBase {
                                 stream_));
       GLIA_CUDA(cudaStreamSynchronize(stream_));
     }
-    // Transform path of the D apply (GLIA_XPASS). By default the plane kernel of the grid size
-    // (plane.hpp), or in FP32 at n = 256 own x, y and z passes (ownfft.cuh, no cuFFT inside the PCG
-    // loop), or else batched 3-D cuFFT transforms. "2d" (FP32, n = 64, 128, 256): own x pass, cuFFT
-    // for batched 2-D (y, z) transforms with k multiplied in between; "0": cuFFT.
+    // Transform path of the FP32 D apply at n = 64, 128, 256 (GLIA_XPASS): by default the x, y
+    // and z passes are the library's own kernels (ownfft.cuh, no cuFFT inside the PCG loop);
+    // "2d" keeps the x pass and lets cuFFT do batched 2-D (y, z) transforms with k multiplied in
+    // between; "0" uses batched 3-D cuFFT transforms.
     const char* xenv = std::getenv("GLIA_XPASS");
     xpass_ = std::is_same<R, float>::value && (n == 64 || n == 128 || n == 256) && !zpass_ &&
              !ref_ && !(xenv && xenv[0] == '0');
-    own_ = xpass_ && n == 256 && !(xenv && std::strcmp(xenv, "2d") == 0);
-    // Grids with a plane kernel run every solve as one launch, in either precision.
-    if (!ref_ && !zpass_ && !(xenv && (xenv[0] == '0' || std::strcmp(xenv, "2d") == 0)))
+    own_ = xpass_ && !(xenv && std::strcmp(xenv, "2d") == 0);
+    // FP64 grids with a plane kernel (plane.hpp) run every solve as one launch; "0" and "2d" keep
+    // cuFFT's transforms there.
+    //
+    // FP32 has none. Every solve transforms the whole field back, which leaves rounding of 6e-8 of
+    // the field's maximum in tumour-free tissue, and the logistic reaction multiplies it by up to
+    // exp(rho T): any change of the transforms inside a solve, even in its last bits, draws that
+    // rounding anew. With float plane kernels a simulation of rho T = 10 moved by 1.5e-4 (5e-3 at
+    // single voxels), its gradient by 2e-2, more than float results may move; at rho T = 14 by 7e-3
+    // and 0.9. They also ran contexts side by side worse, a solve taking every SM: eight 64^3
+    // gradients of 10 steps from 8 threads 18.5 -> 28.9 ms, though one alone took 9.1 -> 7.1 ms.
+    if (kPlane && !ref_ && !(xenv && (xenv[0] == '0' || std::strcmp(xenv, "2d") == 0)))
       init_plane();
-    if (plane()) xpass_ = own_ = false;
     size_t w2[2] = {0, 0};
     if (xpass_ && !own_) {
       int dims[2] = {n, n};
@@ -2373,8 +2387,7 @@ class Engine final : public EngineBase {
       for (cufftHandle p : {r2c2d3_, c2r2d3_}) GLIA_CUFFT(cufftSetWorkArea(p, fft_ws_));
   }
   void init_plane() {
-    using C = typename CT<R>::C;
-    const PlaneKernel k = plane_kernel<R>(g_.n);
+    const PlaneKernel k = plane_kernel(g_.n);
     if (!k.fn) return;
     GLIA_CUDA(cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem));
     int b = 0;
@@ -2382,23 +2395,15 @@ class Engine final : public EngineBase {
     if (b < 1) return;
     plane_ = k;
     plane_res_ = sms_ * b;
-    plane_part_ = dalloc<double>((int64_t)kPlanePartials * std::max(plane_res_, k.items));
+    plane_part_ = dalloc<double>((int64_t)kPlanePartials * plane_res_);
     plane_bar_ = dalloc<unsigned>(2);
-    // exp(2 pi i j / n): float2, or cos and sin in 64-bit fixed point
-    using Tw = std::conditional_t<std::is_same<R, float>::value, float2, FxTw>;
-    std::vector<Tw> tw(g_.n);
-    for (int j = 0; j < g_.n; j++) {
-      const long double a = 2.0L * 3.14159265358979323846264338327950288L * j / g_.n;
-      if constexpr (std::is_same<R, float>::value)
-        tw[j] = make_float2((float)std::cos(a), (float)std::sin(a));
-      else
-        tw[j] = FxTw{fx_from(std::cos(a)), fx_from(std::sin(a))};
-    }
-    plane_tw_ = dalloc<C>(g_.n);
+    std::vector<int4> tw(g_.n);
+    plane_twiddles(g_.n, tw.data());
+    plane_tw_ = dalloc<int4>(g_.n);
     if (k.split) plane_w_ = dalloc<R>(3 * N_);
-    if constexpr (std::is_same<R, double>::value) plane_pf_ = dalloc<R>(Ns_);
+    plane_pf_ = dalloc<R>(Ns_);
     GLIA_CUDA(cudaMemsetAsync(plane_bar_, 0, 2 * sizeof(unsigned), stream_));
-    GLIA_CUDA(cudaMemcpyAsync(plane_tw_, tw.data(), g_.n * sizeof(Tw), cudaMemcpyHostToDevice,
+    GLIA_CUDA(cudaMemcpyAsync(plane_tw_, tw.data(), g_.n * sizeof(int4), cudaMemcpyHostToDevice,
                               stream_));
     GLIA_CUDA(cudaStreamSynchronize(stream_));
   }
@@ -2588,6 +2593,7 @@ class Engine final : public EngineBase {
   CUtensorMap kmap_{};               // TMA map of the packed line arrays (k_yfwd)
   bool tma_ = false;                 // k_yfwd stages with TMA copies (GLIA_TMA=1)
   bool zrev_ = true;                 // k_zpass2 line blocks in descending order
+  bool zpass2_ = true;               // z pass with two real lines per complex transform
   bool yinv_bulk_ = true;            // y-inverse rows staged by bulk copies
   bool own_ = false;  // own y and z passes (x pass on): no cuFFT inside the D apply
   // graph-captured evaluations (eval_prepare / eval_capture / eval_finish)
@@ -2600,12 +2606,11 @@ class Engine final : public EngineBase {
   // plane kernel (plane.cuh) of this grid size: resident CTAs, partial sums, barrier, twiddles
   PlaneKernel plane_{};
   R* plane_w_ = nullptr;
-  int cap_branches_ = 1;  // evaluations that run side by side in the graph being captured
   int plane_res_ = 0;
   double* plane_part_ = nullptr;
   unsigned* plane_bar_ = nullptr;
-  typename CT<R>::C* plane_tw_ = nullptr;
-  R* plane_pf_ = nullptr;  // FP64: preconditioner field for pc_c = plane_pc_
+  int4* plane_tw_ = nullptr;
+  R* plane_pf_ = nullptr;  // preconditioner field for pc_c = plane_pc_
   double plane_pc_ = -1;
   float2* tw_ = nullptr;
   char* fft_ws_ = nullptr;

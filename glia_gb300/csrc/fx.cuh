@@ -182,12 +182,9 @@ GLIA_HD void odd_dft_fx(fx2 (&v)[R]) {
 struct __align__(16) FxTw {
   Fc c, s;
 };
-// z w / 2 and z conj(w) / 2
+// z w / 2
 GLIA_HD fx2 fx_tw(fx2 z, FxTw w) {
   return cmk<fx2>(fx_mulh(z.x, w.c) - fx_mulh(z.y, w.s), fx_mulh(z.x, w.s) + fx_mulh(z.y, w.c));
-}
-GLIA_HD fx2 fx_twc(fx2 z, FxTw w) {
-  return cmk<fx2>(fx_mulh(z.x, w.c) + fx_mulh(z.y, w.s), fx_mulh(z.y, w.c) - fx_mulh(z.x, w.s));
 }
 
 // ---- doubles in and out of a block ---------------------------------------------------------
@@ -382,15 +379,6 @@ GLIA_HD void fx_halves(fx2 a, fx2 b, fx2& s, fx2& d) {
 }
 
 // doubles to a block in registers, and |w| times as much
-struct NoTw {};
-template <int R, int S, bool CONJ, class Tw>
-GLIA_HD void fx_twiddled(fx2 (&q)[R], Tw&& tw) {
-  reg_dft<R, S>(q);
-  if constexpr (!std::is_same<std::decay_t<Tw>, NoTw>::value) {
-#pragma unroll
-    for (int k = 0; k < R; k++) q[k] = CONJ ? fx_twc(q[k], tw(k)) : fx_tw(q[k], tw(k));
-  }
-}
 template <int B>
 GLIA_HD fx2 fx_in2(double2 v, int E) {
   return cmk<fx2>(fx_in<B>(v.x, E), fx_in<B>(v.y, E));

@@ -41,7 +41,6 @@ struct DevScalars {
   double last_dp;
   int dev_fault;         // a bounded device wait ran out (1: TMA copy did not arrive)
   int pad2;
-  double pp;             // sum |p|^2 over the half spectrum (own-transform PCG)
   double m1_keep;        // ||O c(1) - d||^2 of a graph-captured evaluation (read after it ran)
 };
 
@@ -140,7 +139,7 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-enum DivEpi { EPI_APPLYD = 0, EPI_SETUP = 1, EPI_CGW = 2, EPI_CGU = 3 };
+enum DivEpi { EPI_APPLYD = 0, EPI_SETUP = 1, EPI_CGW = 2 };
 
 // Scalar epilogue of a solve set-up (last block, thread 0): PETSc's n = 0 convergence test from
 // sums = [||B b||^2, ||z0||^2, <z0, r0>, <cx, D c>] (Parseval sums, times 1/N).
@@ -165,8 +164,9 @@ __device__ __forceinline__ void div_setup_finish(const double (&sums)[4], DevSca
   if (has_cx) sc->acc[6] += sc->kdot_weight * sums[3] * invN;
 }
 
-// Scalar epilogue of <p, A p> (last block, thread 0): PETSc's indefiniteness check, alpha.
-__device__ __forceinline__ void cg_alpha(double dpi, DevScalars* sc) {
+// Scalar epilogue of w = A p (last block, thread 0): PETSc's indefiniteness check, alpha.
+__device__ __forceinline__ void div_cgw_finish(double pw_sum, DevScalars* sc, double invN) {
+  const double dpi = pw_sum * invN;
   sc->dpi_old = sc->dpi;
   sc->dpi = dpi;
   sc->beta_old = sc->beta;
@@ -177,27 +177,6 @@ __device__ __forceinline__ void cg_alpha(double dpi, DevScalars* sc) {
     sc->status = -9;
   else
     sc->alpha = sc->beta / dpi;
-}
-// Scalar epilogue of the x, r update (last block, thread 0): sums = [||z||^2, <z, r>]; PETSc's
-// convergence test and the next direction's coefficient.
-__device__ __forceinline__ void cg_update_finish(const double (&sums)[2], DevScalars* sc,
-                                                 double invN) {
-  const double dp = sqrt(sums[0] * invN);
-  sc->dp = dp;
-  int st = conv_test(dp, sc);
-  if (st == 0) {
-    const double bnew = sums[1] * invN;
-    sc->beta = bnew;
-    sc->bcoef = bnew / sc->beta_old;
-    sc->iter = sc->iter + 1;
-    if (bnew == 0.0) {
-      st = 2;
-      sc->it = sc->iter + 1;
-    } else if (sc->iter >= sc->maxit) {
-      st = -3;
-    }
-  }
-  sc->status = st;
 }
 
 // Divergence in spectral space, D = sum_j i w_j G_j (the spectrum of div(k grad u)), fused with
@@ -274,7 +253,7 @@ __global__ void __launch_bounds__(kThreads)
   } else {
     double a1[1] = {acc[0].value()};
     if (!grid_sum_last<1>(a1, ws)) return;
-    if (threadIdx.x == 0) cg_alpha(a1[0] * g.invN, sc);
+    if (threadIdx.x == 0) div_cgw_finish(a1[0], sc, g.invN);
   }
 }
 
@@ -316,7 +295,24 @@ __global__ void __launch_bounds__(kThreads)
   }
   double sums[2] = {acc[0].value(), acc[1].value()};
   if (!grid_sum_last<2>(sums, ws)) return;
-  if (threadIdx.x == 0) cg_update_finish(sums, sc, g.invN);
+  if (threadIdx.x == 0) {
+    const double dp = sqrt(sums[0] * g.invN);
+    sc->dp = dp;
+    int st = conv_test(dp, sc);
+    if (st == 0) {
+      const double bnew = sums[1] * g.invN;
+      sc->beta = bnew;
+      sc->bcoef = bnew / sc->beta_old;
+      sc->iter = sc->iter + 1;
+      if (bnew == 0.0) {
+        st = 2;
+        sc->it = sc->iter + 1;
+      } else if (sc->iter >= sc->maxit) {
+        st = -3;
+      }
+    }
+    sc->status = st;
+  }
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -40,10 +40,9 @@ enum KSlot {
   KS_XFWD_CGW,           // k_xfwd<EPI_CGW>: forward x transforms, divergence, w = A p
   KS_XFWD_APPLYD,        // k_xfwd<EPI_APPLYD>: forward x transforms, divergence, D u
   KS_YINV,               // k_yinv_bulk (or k_yinv): inverse y transforms, packed kz = 0 / n/2
-  KS_ZFUSED,             // k_zpass2: z C2R, k multiply, z R2C per line
+  KS_ZFUSED,             // k_zpass2 (or k_zpass): z C2R, k multiply, z R2C per line
   KS_YFWD,               // k_yfwd: forward y transforms, unpacking
-  KS_XFWD_CGU,           // k_xfwd_own<EPI_CGU>: forward x transforms, w = A p, x and r updated
-  KS_PLANE,              // k_plane: a whole solve (or D apply, transform) of a small grid
+  KS_PLANE,              // k_plane: a whole FP64 solve (or D apply, transform)
   KS_COUNT
 };
 
@@ -55,7 +54,7 @@ static const char* const kSlotNames[KS_COUNT] = {
     "cufft_c2r_x3",       "ref_vector_ops", "ref_dot",         "k_zpass_mulk",
     "cufft_c2c_2d",       "k_xinv",         "k_xfwd_setup",    "k_xfwd_cgw",
     "k_xfwd_applyd",      "k_yinv_bulk",    "k_zpass2",         "k_yfwd",
-    "k_xfwd_cgu",         "k_plane"};
+    "k_plane"};
 
 struct KTimer {
   bool on = false;

@@ -1,4 +1,5 @@
-// plane.cuh — a whole diffusion solve (or D apply, smoother, transform) as one persistent kernel.
+// plane.cuh — a whole FP64 diffusion solve (or D apply, smoother, transform) as one persistent
+// kernel.
 //
 // Grids whose (y, z) plane fits in shared memory. A three-dimensional transform is split by
 // direction into two kinds of phase, separated by grid-wide barriers:
@@ -18,17 +19,11 @@
 // The scalars live in every CTA: after each barrier all CTAs add the same per-CTA partial sums in
 // the same order and take the same decision.
 //
-// Why. Up to 128^3 every array stays in L2 and a solve is bound by latency: as separate launches it
-// took 7 kernels and a conditional graph node an iteration and a graph launch a solve, 35 to 60 us
-// an iteration whatever the size. A barrier costs 1.0 us, a phase at 64^3 4 to 10 us (float).
-// In FP64 the arithmetic is the bound, see fx.cuh. Measured on GB300, before -> after:
-//   mixed  gradient  32^3, 16 steps   14.5 -> 6.6 ms      64^3, 40 steps   40.5 -> 23.5 ms
-//          forward   96^3, 20 steps   13.8 -> 5.9 ms
-//          gradient 128^3, 40 steps   88.0 -> 81.5 ms
-//   FP64   forward   64^3, 100 steps   151 -> 45.5 ms
-//          gradient 128^3, 6 steps     166 -> 32.8 ms
-//          adjoint  120^3, 2 steps    48.7 -> 10.5 ms
-//          solve    256^3               49 -> 10.7 ms
+// FP64 only. Arithmetic is the bound there, see fx.cuh; a barrier costs 1.0 us. As separate launches
+// a solve took 7 kernels and a conditional graph node an iteration, and cuFFT's transforms ran at the
+// FP64 units' rate. Measured on GB300, before -> after:
+//   forward   64^3, 100 steps   150 -> 45 ms      gradient 128^3, 6 steps   164 -> 32 ms
+//   adjoint  120^3, 2 steps    48.7 -> 10.5 ms    solve    256^3           46 -> 10.3 ms
 //
 // N = R1 R2 (R2 a power of two, so that a group of R2 threads is part of a warp). Inverse
 // transforms read index R2 a + b (R1-point DFTs over a, twiddle w^(b k1), R2-point DFTs over b) and
@@ -52,56 +47,42 @@ namespace glia {
 
 __host__ __device__ constexpr int plane_r2(int n) { return n <= 56 ? 4 : (n < 144 ? 8 : 16); }
 
-template <typename R, int NN>
+template <int NN>
 struct PlaneGeo {
-  using C = typename CT<R>::C;
+  using C = double2;
   static constexpr int N = NN, R2 = plane_r2(NN), R1 = NN / R2;
   static constexpr int NQ = N / 2, NH = N / 2 + 1;
   static constexpr int PL = N * NH;       // complex per x plane of a half spectrum
-  // complex per pair of lines: groups of R2 < 16 lanes that share a wavefront meet different banks
-  // (float), or one slot after every R2 (double, where exchanges in place have no swizzle)
-  static constexpr int GAP = sizeof(R) == 8 ? 1 : 0;
-  static constexpr int PS2 =
-      GAP ? N + R1 : N + (R2 == 4 ? 4 : (R2 == 8 && N % 16 == 0) ? 8 : 0);
-  static __host__ __device__ constexpr int slot(int k) { return GAP ? k + k / R2 : k; }
-  // double planes above 200 KB: y and z in phases of their own (column blocks, lines), see k_plane
-  static constexpr bool SPLIT = GAP && NQ * PS2 * 16 > 200 * 1024;
+  // complex per pair of lines: one slot of padding after every R2, so that the lanes of a group
+  // meet different banks when they exchange in place
+  static constexpr int PS2 = N + R1;
+  static __host__ __device__ constexpr int slot(int k) { return k + k / R2; }
+  // planes above 200 KB: y and z in phases of their own (column blocks, lines), see k_plane
+  static constexpr bool SPLIT = NQ * PS2 * 16 > 200 * 1024;
   static constexpr int TC = NQ % 16 == 0 ? 16 : 8;  // SPLIT: columns per block
   static constexpr int PLANE = SPLIT ? 0 : NQ * PS2;
   // columns per tile of a column phase: the fewest rounds of tiles over the resident CTAs that at
-  // most MAXT columns allow, then the smallest multiple of 4 (a sector) that needs no more; float
-  // 8 or 16 up to 16, whose divisions are shifts (12 costs 2 % at 72^3), 4 only up to 32^3
+  // most MAXT columns allow, then the smallest multiple of 4 (a sector) that needs no more; 4 only
+  // up to 32^3. Solve, fixed tiles of 16 (32 from 112^3) -> these: 32^3 108 -> 103 us, 64^3
+  // 256 -> 246, 112^3 1005 -> 886, 128^3 1047 -> 992, 144^3 2070 -> 1867
   static constexpr int PB = PLANE * (int)sizeof(C);
-  static constexpr int CTAS = PB > 110 * 1024 ? 152 : 304;
-  static constexpr int MAXT = sizeof(R) == 4 ? 32 : CTAS == 304 ? 24 : 210 * 1024 / (2 * N * 16);
+  static constexpr int CTAS = PB > 110 * 1024 ? 152 : 304;  // resident on 152 SMs
+  static constexpr int MAXT = CTAS == 304 ? 24 : 210 * 1024 / (2 * N * 16);
   static constexpr int PER = (PL + CTAS - 1) / CTAS, ROUNDS = (PER + MAXT - 1) / MAXT;
   static constexpr int T4 = ((PER + ROUNDS - 1) / ROUNDS + 3) / 4 * 4;
-  static constexpr int T = SPLIT                             ? 8
-                           : N > 32 && T4 < 8                ? 8
-                           : sizeof(R) == 4 && T4 == 12      ? 16
-                                                             : T4;
+  static constexpr int T = SPLIT ? 8 : N > 32 && T4 < 8 ? 8 : T4;
   static constexpr int XT = (PL + T - 1) / T;
   static constexpr int TILE = N * T;
   static constexpr int RED = 5 * 512 * 8 / (int)sizeof(C);  // partial sums of a phase
   static constexpr int LINES = SPLIT ? 16 * PS2 : 0;  // one pair of lines per group of R2 lanes
   static constexpr int BUF0 = 2 * TILE > RED ? 2 * TILE : RED;
   static constexpr int BUF1 = PLANE > LINES ? PLANE : LINES, BUF = BUF0 > BUF1 ? BUF0 : BUF1;
-  // + twiddles twice, kz' = 0 twice, wave numbers
-  static constexpr int SMEM = (BUF + 4 * N + (GAP ? N / 2 : 0)) * (int)sizeof(C);
+  // + twiddles, kz' = 0 twice, wave numbers
+  static constexpr int SMEM = (BUF + 3 * N + N / 2) * (int)sizeof(C);
   static constexpr int MINB = SMEM > 110 * 1024 ? 1 : 2;
   static constexpr int NT = N <= 32 ? 128 : (MINB == 2 ? 256 : 512);
   static constexpr int NW = NT / 32, GPW = 32 / R2, NG = NW * GPW;
-  // the two transforms of a column side by side instead of in turn: always in double, in float where
-  // it fills the threads better (elsewhere its spills cost 1 to 2 %). Solve, before -> after, with
-  // T above (before: 16 columns from 72^3 to 104^3, then 28 in float and 32 in double): mixed 64^3
-  // 129 -> 126 us, 104^3 255 -> 242, 144^3 542 -> 509, 160^3 679 -> 617, 192^3 978 -> 910; FP64
-  // 32^3 108 -> 103, 64^3 256 -> 246, 112^3 1005 -> 886, 128^3 1047 -> 992, 144^3 2070 -> 1867
-  static constexpr bool BOTH =
-      sizeof(R) == 8 || (2 * T * R2 + NT - 1) / NT < 2 * ((T * R2 + NT - 1) / NT);
-  // float kernels with a tile per CTA keep their partial sums per work item instead of per CTA: the
-  // result does not depend on the number of CTAs, so a solve may run on fewer beside others
-  static constexpr int ITEMS = XT > 3 * N ? XT : 3 * N;
-  static constexpr bool PER_ITEM = sizeof(R) == 4 && XT <= 304;
+  static constexpr int ITEMS = XT > 3 * N ? XT : 3 * N;  // most work items of a phase
   static_assert(R1 * R2 == N && N % 2 == 0, "decomposition");
   static_assert(R1 <= 16, "register DFT");
   static_assert(!SPLIT || (NG == 16 && N * TC <= BUF), "column block and lines fit the buffer");
@@ -141,79 +122,10 @@ struct GridBarrier {
   }
 };
 
-// The DFT tasks of the phases, in registers: float data as they are, doubles in block fixed point
-// (fx.cuh). tw(k) is the table's factor of result k.
-template <class C>
-struct Task;
-template <>
-struct Task<float2> {
-  using Tw = float2;
-  template <int R, int S, bool CONJ, class F>
-  static __device__ __forceinline__ void dft_tw(float2 (&v)[R], F&& tw) {
-    reg_dft<R, S>(v);
-#pragma unroll
-    for (int k = 0; k < R; k++) v[k] = CONJ ? cmulc(v[k], tw(k)) : cmul2(v[k], tw(k));
-  }
-  template <int R, int S>
-  static __device__ __forceinline__ void dft(float2 (&v)[R]) {
-    reg_dft<R, S>(v);
-  }
-  // inputs times i w(a)
-  template <int R, int S, class W, class F>
-  static __device__ __forceinline__ void dft_iw_tw(float2 (&v)[R], W&& w, F&& tw) {
-#pragma unroll
-    for (int a = 0; a < R; a++) v[a] = cimul<float2>((float)w(a), v[a]);
-    dft_tw<R, S, false>(v, tw);
-  }
-  // inputs i w u(a) + v(a), loaded here
-  template <int R, int S, class U, class V, class F>
-  static __device__ __forceinline__ void dft_sum_tw(float2 (&q)[R], U&& u, V&& v, int w, F&& tw) {
-    float2 x[R];
-#pragma unroll
-    for (int a = 0; a < R; a++) q[a] = v(a);
-#pragma unroll
-    for (int a = 0; a < R; a++) x[a] = u(a);
-#pragma unroll
-    for (int a = 0; a < R; a++) q[a] = cadd(q[a], cimul<float2>((float)w, x[a]));
-    dft_tw<R, S, true>(q, tw);
-  }
-  // results (times i w when dz) in pairs a, h -> Z[c] = a + i h, Z[N - c] = conj a + i conj h;
-  // c = 0: re / im hold the two packed real values of each
-  template <int R>
-  static __device__ __forceinline__ void dft_pair(float2 (&v)[R], int c, bool dz) {
-    reg_dft<R, +1>(v);
-#pragma unroll
-    for (int i = 0; i < R / 2; i++) {
-      float2 a = v[2 * i], h = v[2 * i + 1];
-      if (dz) {
-        a = cimul<float2>((float)c, a);
-        h = cimul<float2>((float)c, h);
-      }
-      v[2 * i] = c == 0 ? make_float2(a.x, h.x) : make_float2(a.x - h.y, a.y + h.x);
-      v[2 * i + 1] = c == 0 ? make_float2(a.y, h.y) : make_float2(a.x + h.y, h.x - a.y);
-    }
-  }
-  // the way back: pairs Z[c], Z[N - c] -> a, h (times i w when dz), DFT
-  template <int R, class F>
-  static __device__ __forceinline__ void split_dft_tw(float2 (&v)[R], int c, bool dz, F&& tw) {
-#pragma unroll
-    for (int i = 0; i < R / 2; i++) {
-      const float2 z = v[2 * i], zq = v[2 * i + 1];
-      float2 a = make_float2(0.5f * (z.x + zq.x), 0.5f * (z.y - zq.y));
-      float2 h = make_float2(0.5f * (z.y + zq.y), -0.5f * (z.x - zq.x));
-      if (c == 0) {
-        a = make_float2(z.x, zq.x);
-        h = make_float2(z.y, zq.y);
-      }
-      v[2 * i] = dz ? cimul<float2>((float)c, a) : a;
-      v[2 * i + 1] = dz ? cimul<float2>((float)c, h) : h;
-    }
-    dft_tw<R, -1, true>(v, tw);
-  }
-};
-// Doubles: block fixed point (fx.cuh). One body per radix for every use, called, not inlined: the
-// integer code of a 16-point task is about 3000 instructions, and inlined at each use it ran out
-// of the instruction cache (measured: 5.6 stalled warps waiting for instructions per issue).
+// The DFT tasks of the phases, in registers and in block fixed point (fx.cuh). One body per radix
+// for every use, called, not inlined: the integer code of a 16-point task is about 3000
+// instructions, and inlined at each use it ran out of the instruction cache (measured: 5.6 stalled
+// warps waiting for instructions per issue).
 enum FxMode {
   FX_FWD = 1,    // forward transform (real and imaginary parts swapped around an inverse one)
   FX_IW = 2,     // inputs times i w(a), w(a) the wave number of w0 + wl a
@@ -427,10 +339,6 @@ __device__ __noinline__ double fx_middle2(fx2* row, const double* ka, const doub
   for (int a = 0; a < R; a++) row[a] = q[a];
   return sum;
 }
-template <>
-struct Task<double2> {
-  using Tw = FxTw;
-};
 
 enum PlaneStep {
   PS_FWD = 0,   // planes: real field -> y, z forward
@@ -442,7 +350,6 @@ enum PlaneStep {
   PS_YFWD,      // SPLIT: columns of planes, y forward, W -> M
   PS_SPEC,      // columns: M_0 -> spectrum (stored)
   PS_ENTER,     // columns: M_0 -> spectrum (stored) -> G_x, G_0
-  PS_OPEN,      // columns: given spectrum -> G_x, G_0
   PS_SMOOTH,    // columns: M_0 -> spectrum times mulk -> G_0
   PS_SETUP,     // columns: M -> D c, solve set-up, first direction -> G_x, G_0
   PS_UPDATE,    // columns: M -> D p, x and r
@@ -452,15 +359,14 @@ enum PlaneStep {
   PS_DOT        // columns: M -> <cx, D u>
 };
 
-template <typename R, int NN>
-__global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
-    k_plane(const __grid_constant__ PlaneArgs<R> A) {
-  using Geo_ = PlaneGeo<R, NN>;
-  using C = typename Geo_::C;
+template <int NN>
+__global__ void __launch_bounds__(PlaneGeo<NN>::NT, PlaneGeo<NN>::MINB)
+    k_plane(const __grid_constant__ PlaneArgs A) {
+  using Geo_ = PlaneGeo<NN>;
+  using C = double2;
   constexpr int N = NN, R1 = Geo_::R1, R2 = Geo_::R2, NQ = Geo_::NQ, NH = Geo_::NH, PL = Geo_::PL,
                 T = Geo_::T, NT = Geo_::NT, PS2 = Geo_::PS2, TILE = Geo_::TILE;
   constexpr int S = N * PL;
-  constexpr bool FX = sizeof(R) == 8, BOTH = Geo_::BOTH;
   auto fx = [](auto* q) {  // the same memory as fixed-point blocks
     using Q = std::conditional_t<std::is_const<std::remove_pointer_t<decltype(q)>>::value,
                                  const fx2, fx2>;
@@ -468,30 +374,23 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
   };
   extern __shared__ double2 plane_dyn[];
   C* buf = reinterpret_cast<C*>(plane_dyn);
-  using K = Task<C>;
-  using Tw = typename K::Tw;
+  using Tw = FxTw;
   static_assert(sizeof(Tw) == sizeof(C), "table entry");
   Tw* twA = reinterpret_cast<Tw*>(buf + Geo_::BUF);  // [k1 R2 + b] exp(+2 pi i b k1 / N)
-  Tw* twB = twA + N;                                 // [b R1 + k1], the same
-  C* zcol = reinterpret_cast<C*>(twB + N);           // column kz' = 0 of a plane, forward
+  C* zcol = reinterpret_cast<C*>(twA + N);           // column kz' = 0 of a plane, forward
   C* zin = zcol + N;                                 // and inverse
-  [[maybe_unused]] double* wtab = reinterpret_cast<double*>(zin + N);  // double: wave numbers
-  __shared__ double tot[5];
+  double* wtab = reinterpret_cast<double*>(zin + N);  // wave numbers
+  __shared__ double tot[4];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int i = tid; i < N; i += NT) {
     const int k1 = i / R2, b = i - k1 * R2;
-    const Tw w = reinterpret_cast<const Tw*>(A.tw)[b * k1];  // b k1 < N
-    twA[i] = w;
-    twB[b * R1 + k1] = w;
-    if constexpr (FX) wtab[i] = (double)wavenum(i, N);
+    twA[i] = reinterpret_cast<const Tw*>(A.tw)[b * k1];  // b k1 < N
+    wtab[i] = (double)wavenum(i, N);
   }
   __syncthreads();
-  const R invN = (R)(1.0 / ((double)N * N * N));
-  const double dinvN = 1.0 / ((double)N * N * N);
-  // double: the spectra sent to the planes keep their factor n^3
-  const double dscale = FX ? dinvN : 1.0;
-  const R a1 = (R)(A.a_cn * dscale), invN2 = invN * invN;
-  const R a_cn = (R)A.a_cn, pcc = (R)A.pc_c;
+  const double invN = 1.0 / ((double)N * N * N);
+  // the spectra sent to the planes keep their factor n^3
+  const double a1 = A.a_cn * invN, invN2 = invN * invN;
   GridBarrier bar{A.bar, 0};
   // PCG scalars, the same in every CTA (thread 0 updates them)
   __shared__ struct {
@@ -509,14 +408,11 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
   C* __restrict__ const rh = A.rhat;
   C* __restrict__ const ph = A.phat;
   C* __restrict__ const ch = A.chat;
-  const R* __restrict__ const kf = A.k;
+  const double* __restrict__ const kf = A.k;
 
-  // partial sums (per CTA, or per work item `i`) of slots s0 ... s0 + Q - 1, and their totals
-  // after the next barrier; slot `planes` holds the planes' sums, the others the columns'
+  // partial sums per CTA of slots s0 ... s0 + Q - 1, and their totals after the next barrier
   // (few FP64 operations: all threads' values go to shared memory and one warp adds each sum)
-  constexpr bool PI = Geo_::PER_ITEM;
-  const int stride = PI ? Geo_::ITEMS : (int)gridDim.x;
-  auto partials = [&](const double* v, int q_n, int s0, int i) {
+  auto partials = [&](const double* v, int q_n, int s0) {
     double* all = reinterpret_cast<double*>(buf);
     __syncthreads();
     for (int q = 0; q < q_n; q++) all[q * NT + tid] = v[q];
@@ -527,14 +423,14 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
       for (int w = 0; w < Geo_::NW; w++) x += all[q * NT + 32 * w + lane];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-      if (lane == 0) A.part[(s0 + q) * stride + i] = x;
+      if (lane == 0) A.part[(s0 + q) * (int)gridDim.x + blockIdx.x] = x;
     }
   };
-  auto totals = [&](int q_n, int s0, int planes) {
+  auto totals = [&](int q_n, int s0) {
     for (int q = warp; q < q_n; q += Geo_::NW) {
       double x = 0;
-      const int count = !PI ? (int)gridDim.x : s0 + q == planes ? 3 * N : Geo_::XT;
-      for (int b = lane; b < count; b += 32) x += __ldcg(&A.part[(s0 + q) * stride + b]);
+      for (int b = lane; b < (int)gridDim.x; b += 32)
+        x += __ldcg(&A.part[(s0 + q) * (int)gridDim.x + b]);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
       if (lane == 0) tot[q] = x;
@@ -551,68 +447,54 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
 
   // the reaction step on two voxels as their field is read
   auto reacted = [&](C v, int64_t i0, int64_t i1) {
-    const R e0 = exp(A.rho[i0] * A.dt), e1 = exp(A.rho[i1] * A.dt);
+    const double e0 = exp(A.rho[i0] * A.dt), e1 = exp(A.rho[i1] * A.dt);
     if (A.pre == 1) {  // logistic (k_reaction_fwd)
       if (A.half) {
         A.half[i0] = v.x;
         A.half[i1] = v.y;
       }
-      const R c0 = v.x * e0, c1 = v.y * e1;
-      return cmk<C>(c0 / (c0 + (R)1 - v.x), c1 / (c1 + (R)1 - v.y));
+      const double c0 = v.x * e0, c1 = v.y * e1;
+      return cmk<C>(c0 / (c0 + 1.0 - v.x), c1 / (c1 + 1.0 - v.y));
     }
     // linearised at lin (k_reaction_lin)
-    const R c0 = A.lin[i0], c1 = A.lin[i1];
-    const R q0 = c0 * e0 + (R)1 - c0, q1 = c1 * e1 + (R)1 - c1;
+    const double c0 = A.lin[i0], c1 = A.lin[i1];
+    const double q0 = c0 * e0 + 1.0 - c0, q1 = c1 * e1 + 1.0 - c1;
     return cmk<C>(v.x * e0 / (q0 * q0), v.y * e1 / (q1 * q1));
   };
 
   // the twiddles of a task: none for index 0, where all are 1
-  [[maybe_unused]] auto at_tw = [](int i, const Tw* tw) { return i ? tw : nullptr; };
-  Acc<R> acc[5];
-  // the sums of a work item (PER_ITEM) or of all of a CTA's
-  auto sums = [&](int kind, int i) {
-    if (kind == PS_GRAD) {
-      const double v[1] = {acc[0].value()};
-      partials(v, 1, 1, i);
-    } else if (kind == PS_SETUP) {
-      const double v[5] = {acc[0].value(), acc[1].value(), acc[2].value(), acc[3].value(),
-                           FX ? acc[1].value() : acc[4].value()};
-      partials(v, 5, 1, i);
-    } else if (kind == PS_UPDATE || kind == PS_DOT) {
-      const double v[2] = {acc[0].value(), acc[1].value()};
-      partials(v, 2, 2, i);
-    } else if (kind == PS_DIR) {
-      const double v[1] = {acc[0].value()};
-      partials(v, 1, 0, i);
-    }
-    if constexpr (PI) {
-      __syncthreads();
-#pragma unroll
-      for (int q = 0; q < 5; q++) acc[q] = Acc<R>();
-    }
+  auto at_tw = [](int i, const Tw* tw) { return i ? tw : nullptr; };
+  double acc[4];
+  auto sums = [&](int kind) {
+    if (kind == PS_GRAD)
+      partials(acc, 1, 1);
+    else if (kind == PS_SETUP)
+      partials(acc, 4, 1);
+    else if (kind == PS_UPDATE || kind == PS_DOT)
+      partials(acc, 2, 2);
+    else if (kind == PS_DIR)
+      partials(acc, 1, 0);
   };
-  // Double: row k1 of a line pair in real space (places k2, z = k1 + R1 k2 of lines l0 and l1)
+  // Row k1 of a line pair in real space (places k2, z = k1 + R1 k2 of lines l0 and l1)
   auto line_middle = [&](int kind, C* row, int64_t l0, int64_t l1, int k1) {
-    if constexpr (FX) {
-      const Tw* tw = at_tw(k1, twA + k1 * R2);
-      if (kind == PS_FWD) {
+    const Tw* tw = at_tw(k1, twA + k1 * R2);
+    if (kind == PS_FWD) {
 #pragma unroll 2
-        for (int k2 = 0; k2 < R2; k2++) {
-          const int m = k1 + R1 * k2;
-          row[k2] = cmk<C>(A.in[l0 + m], A.in[l1 + m]);
-          if (A.pre) row[k2] = reacted(row[k2], l0 + m, l1 + m);
-        }
-        fx_enter2<R2, N>(row, fx(row), 1, tw, FX_FWD, 0, 0);
-      } else if (kind == PS_GRAD) {
-        acc[0].add(fx_middle2<R2>(fx(row), kf + l0 + k1, kf + l1 + k1, R1, tw));
-      } else {
-        fx_leave2<R2>(fx(row), row, 1, false);
+      for (int k2 = 0; k2 < R2; k2++) {
+        const int m = k1 + R1 * k2;
+        row[k2] = cmk<C>(A.in[l0 + m], A.in[l1 + m]);
+        if (A.pre) row[k2] = reacted(row[k2], l0 + m, l1 + m);
+      }
+      fx_enter2<R2, N>(row, fx(row), 1, tw, FX_FWD, 0, 0);
+    } else if (kind == PS_GRAD) {
+      acc[0] += fx_middle2<R2>(fx(row), kf + l0 + k1, kf + l1 + k1, R1, tw);
+    } else {
+      fx_leave2<R2>(fx(row), row, 1, false);
 #pragma unroll 4
-        for (int k2 = 0; k2 < R2; k2++) {
-          const int m = k1 + R1 * k2;
-          A.out[l0 + m] = row[k2].x;
-          A.out[l1 + m] = row[k2].y;
-        }
+      for (int k2 = 0; k2 < R2; k2++) {
+        const int m = k1 + R1 * k2;
+        A.out[l0 + m] = row[k2].x;
+        A.out[l1 + m] = row[k2].y;
       }
     }
   };
@@ -621,12 +503,12 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
   auto even = [](int c) { return Geo_::slot(c); };
   auto odd = [](int c) { return Geo_::slot(c == 0 ? NQ : N - c); };
 
-  int step = A.prog == PP_SOLVE_SPEC ? PS_OPEN : Geo_::SPLIT ? PS_LINE : PS_FWD;
+  int step = Geo_::SPLIT ? PS_LINE : PS_FWD;
   bool started = false;  // the solve's set-up is done
   int kind = PS_FWD;  // SPLIT: the plane phase that the current y and line phases are part of
   for (;;) {
 #pragma unroll
-    for (int q = 0; q < 5; q++) acc[q] = Acc<R>{};
+    for (int q = 0; q < 4; q++) acc[q] = 0.0;
     if constexpr (Geo_::SPLIT) {
       if (step == PS_YINV || step == PS_YFWD) {
         // ------------------------------------------------------ SPLIT: column blocks of planes
@@ -712,10 +594,7 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
           }
           __syncwarp();
         }
-        if (kind == PS_GRAD) {
-          const double v[1] = {acc[0].value()};
-          partials(v, 1, 1, blockIdx.x);
-        }
+        if (kind == PS_GRAD) sums(kind);
       }
     }
     if (step <= PS_BACK && !Geo_::SPLIT) {
@@ -728,53 +607,24 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
           // y inverse: the kz = 0 and kz = N/2 columns as one, then rows ky = R2 a + b of column c
           const C* G = (step == PS_GRAD && j == 0 ? Gp : Gp + S) + x * PL;
           for (int ky = tid; ky < N; ky += NT) {
-            if constexpr (FX) {
-              fx(zin)[ky] = fx_plus_i(fx(G)[ky * NH], fx(G)[ky * NH + NQ]);
-            } else {
-              const C z = G[ky * NH], w = G[ky * NH + NQ];
-              zin[ky] = cmk<C>(z.x - w.y, z.y + w.x);
-            }
+            fx(zin)[ky] = fx_plus_i(fx(G)[ky * NH], fx(G)[ky * NH + NQ]);
           }
           __syncthreads();
           for (int task = tid; task < NQ * R2; task += NT) {
             const int b = task / NQ, c = task - b * NQ;
             const C* src = c == 0 ? zin : G + c;
             const int ld = c == 0 ? 1 : NH;
-            if constexpr (FX) {
-              fx_task1<R1, N>(fx(src + b * ld), nullptr, R2 * ld,
-                              fx(buf + (b >> 1) * PS2 + ((b & 1) ? odd(c) : even(c))),
-                              R2 / 2 * PS2, at_tw(b, twA + b), R2, j == 1 ? FX_IW : 0, b, R2);
-            } else {
-            C u[R1];
-#pragma unroll
-            for (int a = 0; a < R1; a++) u[a] = src[(R2 * a + b) * ld];
-            auto tw = [&](int k1) { return twA[k1 * R2 + b]; };
-            if (j == 1)
-              K::template dft_iw_tw<R1, +1>(u, [&](int a) { return wavenum(R2 * a + b, N); }, tw);
-            else
-              K::template dft_tw<R1, +1, false>(u, tw);
-#pragma unroll
-            for (int k1 = 0; k1 < R1; k1++) {
-              buf[(k1 * (R2 / 2) + (b >> 1)) * PS2 + ((b & 1) ? odd(c) : even(c))] = u[k1];
-            }
-            }
+            fx_task1<R1, N>(fx(src + b * ld), nullptr, R2 * ld,
+                            fx(buf + (b >> 1) * PS2 + ((b & 1) ? odd(c) : even(c))),
+                            R2 / 2 * PS2, at_tw(b, twA + b), R2, j == 1 ? FX_IW : 0, b, R2);
           }
           __syncthreads();
           for (int task = tid; task < NQ * R1; task += NT) {
             const int k1 = task / NQ, c = task - k1 * NQ;
             C* row = buf + k1 * (R2 / 2) * PS2 + even(c);
             const int od = odd(c) - even(c);
-            if constexpr (FX) {
-              fx_task2<R2>(fx(row), od, PS2, fx(row), od, PS2, nullptr,
-                           FX_PAIR | (j == 2 ? FX_IC : 0), c);
-            } else {
-            C v[R2];
-#pragma unroll
-            for (int b = 0; b < R2; b++) v[b] = row[(b >> 1) * PS2 + (b & 1) * od];
-            K::template dft_pair<R2>(v, c, j == 2);
-#pragma unroll
-            for (int b = 0; b < R2; b++) row[(b >> 1) * PS2 + (b & 1) * od] = v[b];
-            }
+            fx_task2<R2>(fx(row), od, PS2, fx(row), od, PS2, nullptr,
+                         FX_PAIR | (j == 2 ? FX_IC : 0), c);
           }
           __syncthreads();
         }
@@ -785,108 +635,23 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
           C* E = buf + (on ? pr : 0) * PS2;
           const int p0 = 2 * pr, y0 = p0 / R2 + R1 * (p0 % R2), y1 = y0 + R1;
           const int64_t l0 = ((int64_t)x * N + y0) * N, l1 = ((int64_t)x * N + y1) * N;
-          if constexpr (FX) {
-            // thread t: index R2 a + t in place, then rows k1 = t, t + R2, ... in place, and back
-            C* const col = E + t;
-            if (step != PS_FWD) {
-              if (on)
-                fx_task1<R1, N>(fx(col), nullptr, R2 + 1, fx(col), R2 + 1, at_tw(t, twA + t), R2,
-                                0, 0, 0);
-              __syncwarp();
-            }
-            if (on) {
-              for (int k1 = t; k1 < R1; k1 += R2)
-                line_middle(step, E + k1 * (R2 + 1), l0, l1, k1);
-            }
-            if (step != PS_BACK) {
-              __syncwarp();
-              if (on)
-                fx_task1<R1, N>(fx(col), nullptr, R2 + 1, fx(col), R2 + 1, nullptr, 0, FX_FWD, 0,
-                                0);
-            }
-            continue;
-          } else {
-          auto ex = [&](int k1, int q) -> C& { return E[k1 * R2 + (q ^ (k1 & (R2 - 1)))]; };
+          // thread t: index R2 a + t in place, then rows k1 = t, t + R2, ... in place, and back
+          C* const col = E + t;
           if (step != PS_FWD) {
-            C u[R1];
-            if (on) {
-#pragma unroll
-              for (int a = 0; a < R1; a++) u[a] = E[R2 * a + t];
-              K::template dft_tw<R1, +1, false>(u, [&](int k1) { return twA[k1 * R2 + t]; });
-            }
-            __syncwarp();
-            if (on) {
-#pragma unroll
-              for (int k1 = 0; k1 < R1; k1++) ex(k1, t) = u[k1];
-            }
+            if (on)
+              fx_task1<R1, N>(fx(col), nullptr, R2 + 1, fx(col), R2 + 1, at_tw(t, twA + t), R2,
+                              0, 0, 0);
             __syncwarp();
           }
           if (on) {
-#pragma unroll
-            for (int ii = 0; ii < (R1 + R2 - 1) / R2; ii++) {
-              const int k1 = t + R2 * ii;
-              if (R1 % R2 != 0 && k1 >= R1) continue;
-              C v[R2];
-              if (step == PS_FWD) {
-#pragma unroll
-                for (int k2 = 0; k2 < R2; k2++) {
-                  const int m = k1 + R1 * k2;
-                  v[k2] = cmk<C>(A.in[l0 + m], A.in[l1 + m]);
-                }
-                if (A.pre) {
-#pragma unroll
-                  for (int k2 = 0; k2 < R2; k2++)
-                    v[k2] = reacted(v[k2], l0 + k1 + R1 * k2, l1 + k1 + R1 * k2);
-                }
-              } else {
-                R ka[R2], kb[R2];
-                if (step == PS_GRAD) {
-#pragma unroll
-                  for (int k2 = 0; k2 < R2; k2++) {
-                    ka[k2] = kf[l0 + k1 + R1 * k2];
-                    kb[k2] = kf[l1 + k1 + R1 * k2];
-                  }
-                }
-#pragma unroll
-                for (int q = 0; q < R2; q++) v[q] = ex(k1, q);
-                K::template dft<R2, +1>(v);  // v[k2]: lines a, b at z = k1 + R1 k2
-                if (step == PS_GRAD) {
-#pragma unroll
-                  for (int k2 = 0; k2 < R2; k2++) {
-                    const R sx = v[k2].x * ka[k2], sy = v[k2].y * kb[k2];
-                    acc[0].add(sx * v[k2].x + sy * v[k2].y);
-                    v[k2] = cmk<C>(sx, sy);
-                  }
-                } else {
-#pragma unroll
-                  for (int k2 = 0; k2 < R2; k2++) {
-                    const int m = k1 + R1 * k2;
-                    A.out[l0 + m] = v[k2].x;
-                    A.out[l1 + m] = v[k2].y;
-                  }
-                }
-              }
-              if (step != PS_BACK) {
-                K::template dft_tw<R2, -1, true>(v, [&](int q) { return twB[q * R1 + k1]; });
-#pragma unroll
-                for (int q = 0; q < R2; q++) ex(k1, q) = v[q];
-              }
-            }
+            for (int k1 = t; k1 < R1; k1 += R2)
+              line_middle(step, E + k1 * (R2 + 1), l0, l1, k1);
           }
           if (step != PS_BACK) {
             __syncwarp();
-            C u[R1];
-            if (on) {
-#pragma unroll
-              for (int k1 = 0; k1 < R1; k1++) u[k1] = ex(k1, t);
-              K::template dft<R1, -1>(u);
-            }
-            __syncwarp();
-            if (on) {
-#pragma unroll
-              for (int a = 0; a < R1; a++) E[R2 * a + t] = u[a];
-            }
-          }
+            if (on)
+              fx_task1<R1, N>(fx(col), nullptr, R2 + 1, fx(col), R2 + 1, nullptr, 0, FX_FWD, 0,
+                              0);
           }
         }
         __syncthreads();
@@ -896,17 +661,8 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
             const int k1 = task / NQ, c = task - k1 * NQ;
             C* row = buf + k1 * (R2 / 2) * PS2 + even(c);
             const int od = odd(c) - even(c);
-            if constexpr (FX) {
-              fx_task2<R2>(fx(row), od, PS2, fx(row), od, PS2, at_tw(k1, twA + k1 * R2),
-                           FX_SPLIT | (j == 2 ? FX_IC : 0), c);
-            } else {
-            C v[R2];
-#pragma unroll
-            for (int b = 0; b < R2; b++) v[b] = row[(b >> 1) * PS2 + (b & 1) * od];
-            K::template split_dft_tw<R2>(v, c, j == 2, [&](int b) { return twA[k1 * R2 + b]; });
-#pragma unroll
-            for (int b = 0; b < R2; b++) row[(b >> 1) * PS2 + (b & 1) * od] = v[b];
-            }
+            fx_task2<R2>(fx(row), od, PS2, fx(row), od, PS2, at_tw(k1, twA + k1 * R2),
+                         FX_SPLIT | (j == 2 ? FX_IC : 0), c);
           }
           __syncthreads();
           C* M = Mp + j * S + x * PL;
@@ -914,49 +670,31 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
             const int b = task / NQ, c = task - b * NQ;
             C* dst = c == 0 ? zcol : M + c;
             const int ld = c == 0 ? 1 : NH;
-            if constexpr (FX) {
-              fx_task1<R1, N>(fx(buf + (b >> 1) * PS2 + ((b & 1) ? odd(c) : even(c))), nullptr,
-                              R2 / 2 * PS2, fx(dst + b * ld), R2 * ld, nullptr, 0, FX_FWD, 0, 0);
-            } else {
-            C u[R1];
-#pragma unroll
-            for (int k1 = 0; k1 < R1; k1++) {
-              u[k1] = buf[(k1 * (R2 / 2) + (b >> 1)) * PS2 + ((b & 1) ? odd(c) : even(c))];
-            }
-            K::template dft<R1, -1>(u);
-#pragma unroll
-            for (int a = 0; a < R1; a++) dst[(b + R2 * a) * ld] = u[a];
-            }
+            fx_task1<R1, N>(fx(buf + (b >> 1) * PS2 + ((b & 1) ? odd(c) : even(c))), nullptr,
+                            R2 / 2 * PS2, fx(dst + b * ld), R2 * ld, nullptr, 0, FX_FWD, 0, 0);
           }
           __syncthreads();
           for (int ky = tid; ky < N; ky += NT) {  // kz' = 0 into kz = 0 and kz = N/2
-            if constexpr (FX) {
-              fx_halves(fx(zcol)[ky], fx(zcol)[ky == 0 ? 0 : N - ky], fx(M)[ky * NH],
-                        fx(M)[ky * NH + NQ]);
-            } else {
-              const C z = zcol[ky], zm = zcol[ky == 0 ? 0 : N - ky];
-              M[ky * NH] = cmk<C>((R)0.5 * (z.x + zm.x), (R)0.5 * (z.y - zm.y));
-              M[ky * NH + NQ] = cmk<C>((R)0.5 * (z.y + zm.y), (R)-0.5 * (z.x - zm.x));
-            }
+            fx_halves(fx(zcol)[ky], fx(zcol)[ky == 0 ? 0 : N - ky], fx(M)[ky * NH],
+                      fx(M)[ky * NH + NQ]);
           }
         }
-        if (PI && step == PS_GRAD) sums(step, item);
       }
-      if (!PI && step == PS_GRAD) sums(step, blockIdx.x);
+      if (step == PS_GRAD) sums(step);
     } else if (step >= PS_SPEC) {
       // ----------------------------------------------------------------------------- columns
       const int nin = step == PS_SPEC || step == PS_ENTER || step == PS_SMOOTH ? 1
-                      : step == PS_OPEN || step == PS_DIR || step == PS_LEAVE  ? 0
+                      : step == PS_DIR || step == PS_LEAVE                     ? 0
                                                                                : 2;
       const int nout = step == PS_SMOOTH || step == PS_LEAVE || step == PS_APPLY ? 1
                        : step == PS_SPEC || step == PS_UPDATE || step == PS_DOT  ? 0
                                                                                  : 2;
       if (step == PS_UPDATE) {  // alpha
-        totals(2, 0, 1);
+        totals(2, 0);
         if (tid == 0) {
           if (cg.iter == 0) tot[0] = cg.pp;  // of the set-up's first direction
           cg.dpi_old = cg.dpi;
-          cg.dpi = tot[0] * dinvN + A.a_cn * tot[1] * dscale * dscale;
+          cg.dpi = tot[0] * invN + A.a_cn * tot[1] * invN * invN;
           cg.beta_old = cg.beta;
           cg.it = cg.iter + 1;
           if (cg.dpi == 0.0 || (cg.iter > 0 && cg.dpi * cg.dpi_old <= 0.0))
@@ -968,260 +706,121 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
         }
         __syncthreads();
         if (cg.status != 0) {  // x and r stay as they are
-          if (A.prog == PP_SOLVE_SPEC) break;
           step = PS_LEAVE;
           continue;
         }
       }
-      const R al = (R)cg.alpha, alN = (R)(cg.alpha * dinvN), bc = (R)cg.bcoef;
+      const double al = cg.alpha, alN = cg.alpha * invN, bc = cg.bcoef;
       for (int tile = blockIdx.x; tile < Geo_::XT; tile += gridDim.x) {
         // forward, first part: rows x = R2 a + b
-        for (int i0 = 0; i0 < (BOTH ? 1 : nin); i0++) {
-          for (int task = tid; task < (BOTH ? nin : 1) * T * R2; task += NT) {
-            const int c = task % T, ib = task / T, i = BOTH ? ib >= R2 : i0;
-            const int b = BOTH ? ib - i * R2 : ib, q = tile * T + c;
-            if (q >= PL) continue;
-            const C* src = Mp + i * S + q;
-            if constexpr (FX) {  // M_x, then i w_y M_y + M_z
-              fx_task1<R1, N>(fx(src + b * PL), fx(src + S + b * PL), R2 * PL,
-                              fx(buf + i * TILE + b * T + c), R2 * T, at_tw(b, twA + b), R2,
-                              i == 1 ? FX_FWD | FX_IC | FX_SUM : FX_FWD, wavenum(q / NH, N), 0);
-              continue;
-            } else {
-            C u[R1];
-            auto tw = [&](int k1) { return twA[k1 * R2 + b]; };
-            if (i == 1) {  // i w_y M_y + M_z
-              K::template dft_sum_tw<R1, -1>(
-                  u, [&](int a) { return src[(R2 * a + b) * PL]; },
-                  [&](int a) { return src[S + (R2 * a + b) * PL]; }, wavenum(q / NH, N), tw);
-            } else {
-#pragma unroll
-              for (int a = 0; a < R1; a++) u[a] = src[(R2 * a + b) * PL];
-              K::template dft_tw<R1, -1, true>(u, tw);
-            }
-#pragma unroll
-            for (int k1 = 0; k1 < R1; k1++) buf[i * TILE + (k1 * R2 + b) * T + c] = u[k1];
-            }
-          }
+        for (int task = tid; task < nin * T * R2; task += NT) {
+          const int c = task % T, ib = task / T, i = ib >= R2, b = ib - i * R2, q = tile * T + c;
+          if (q >= PL) continue;
+          const C* src = Mp + i * S + q;
+          // M_x, then i w_y M_y + M_z
+          fx_task1<R1, N>(fx(src + b * PL), fx(src + S + b * PL), R2 * PL,
+                          fx(buf + i * TILE + b * T + c), R2 * T, at_tw(b, twA + b), R2,
+                          i == 1 ? FX_FWD | FX_IC | FX_SUM : FX_FWD, wavenum(q / NH, N), 0);
         }
         if (nin) __syncthreads();
         for (int task = tid; task < T * R1; task += NT) {
           const int c = task % T, k1 = task / T, q = tile * T + c;
           if (q >= PL) continue;
-          const int ky = q / NH, kz = q - ky * NH;
-          const int wy = wavenum(ky, N), wz = wavenum(kz, N);
-          const R mult = (kz == 0 || kz == NQ) ? (R)1 : (R)2;
+          const int kz = q % NH;
+          const double mult = kz == 0 || kz == NQ ? 1.0 : 2.0;
           C* sl = buf + k1 * R2 * T + c;
           auto at = [&](int k2) { return (k1 + R1 * k2) * PL + q; };
-          auto pm = [&](int k2) {
-            if constexpr (FX)
-              return A.pf[at(k2)];
-            else
-              return pc_mult<R>(pcc, wavenum(k1 + R1 * k2, N), wy, wz);
-          };
-          // what a step does at one spectrum element: d = the forward x transform's result (the
-          // divergence for two inputs); returns the value that is transformed back
-          [[maybe_unused]] auto element = [&](int k2, C d) -> C {
+          auto pm = [&](int k2) { return A.pf[at(k2)]; };
+          // What a step does at one spectrum element: d = the forward x transform's result (the
+          // divergence for two inputs); returns the value that is transformed back. FP64 operations
+          // are what this costs: a task's sums are taken without the multiplicity, ||z||^2 and <z, r>
+          // of the set-up are those of its first direction, and the spectra sent to the planes keep
+          // their factor n^3 (a1 = a_cn / n^3).
+          double part[4] = {0, 0, 0, 0};
+          auto element = [&](int k2, C d) -> C {
             const int e = at(k2);
             switch (step) {
               case PS_SPEC:
               case PS_ENTER:
                 ch[e] = d;
-                return cmk<C>(d.x * invN, d.y * invN);
-              case PS_OPEN: {
-                const C c = ch[e];
-                return cmk<C>(c.x * invN, c.y * invN);
-              }
+                return d;
               case PS_SMOOTH:
                 return cmul2(d, A.mulk[e]);
               case PS_SETUP: {
-                const C av = ch[e];
-                const R br = av.x + a_cn * d.x, bi = av.y + a_cn * d.y;
-                const R rr = (R)2 * a_cn * d.x, ri = (R)2 * a_cn * d.y;
-                const R P = pm(k2), r2 = rr * rr + ri * ri;
-                acc[0].add(mult * P * P * (br * br + bi * bi));
-                acc[1].add(mult * P * P * r2);
-                acc[2].add(mult * P * r2);
+                const C c0 = ch[e];
+                const double P = pm(k2);
+                const double br = P * (c0.x + a1 * d.x), bi = P * (c0.y + a1 * d.y);
+                const C r = cmk<C>(2.0 * a1 * d.x, 2.0 * a1 * d.y);
+                const C p = cmk<C>(P * r.x, P * r.y);  // the first direction
+                part[0] = fma(br, br, fma(bi, bi, part[0]));
+                part[1] = fma(p.x, p.x, fma(p.y, p.y, part[1]));
+                part[2] = fma(p.x, r.x, fma(p.y, r.y, part[2]));
                 if (A.cx) {
                   const C xv = A.cx[e];
-                  acc[3].add(mult * (xv.x * d.x + xv.y * d.y));
+                  part[3] = fma(xv.x, d.x, fma(xv.y, d.y, part[3]));
                 }
-                xh[e] = cmk<C>(av.x * invN, av.y * invN);
-                rh[e] = cmk<C>(rr, ri);
-                const C p = cmk<C>(rr * P, ri * P);  // the first direction
+                xh[e] = cmk<C>(c0.x * invN, c0.y * invN);
+                rh[e] = r;
                 ph[e] = p;
-                acc[4].add(mult * (p.x * p.x + p.y * p.y));
-                return cmk<C>(p.x * invN, p.y * invN);
+                return p;
               }
               case PS_UPDATE: {
                 const C p = ph[e], xv = xh[e], rv = rh[e];
-                const R wr = p.x - a_cn * d.x, wi = p.y - a_cn * d.y;
-                const C rn = cmk<C>(rv.x - al * wr, rv.y - al * wi);
+                const double P = pm(k2);
+                const C r = cmk<C>(rv.x - al * (p.x - a1 * d.x), rv.y - al * (p.y - a1 * d.y));
                 xh[e] = cmk<C>(xv.x + alN * p.x, xv.y + alN * p.y);
-                rh[e] = rn;
-                const R P = pm(k2), m2 = mult * (rn.x * rn.x + rn.y * rn.y);
-                acc[0].add(P * P * m2);
-                acc[1].add(P * m2);
+                rh[e] = r;
+                const double t = P * (r.x * r.x + r.y * r.y);
+                part[0] = fma(P, t, part[0]);
+                part[1] += t;
                 return d;
               }
               case PS_DIR: {
                 const C rv = rh[e], po = ph[e];
-                const R P = pm(k2);
-                const C p = cmk<C>(rv.x * P + bc * po.x, rv.y * P + bc * po.y);
+                const double P = pm(k2);
+                const C p = cmk<C>(fma(P, rv.x, bc * po.x), fma(P, rv.y, bc * po.y));
                 ph[e] = p;
-                acc[0].add(mult * (p.x * p.x + p.y * p.y));
-                return cmk<C>(p.x * invN, p.y * invN);
+                part[0] = fma(p.x, p.x, fma(p.y, p.y, part[0]));
+                return p;
               }
               case PS_LEAVE:
                 return xh[e];
               case PS_APPLY:
-                return cmk<C>(d.x * invN, d.y * invN);
+                return cmk<C>(d.x * invN2, d.y * invN2);
               default: {  // PS_DOT
                 const C xv = A.cx[e];
-                acc[0].add(mult * (xv.x * d.x + xv.y * d.y));
+                part[0] = fma(xv.x, d.x, fma(xv.y, d.y, part[0]));
                 return d;
               }
             }
           };
-          if constexpr (FX) {
-            // The same in double. FP64 operations are what this costs: a task's sums are taken
-            // without the multiplicity, ||z||^2 and <z, r> of the set-up are those of its first direction,
-            // and the spectra sent to the planes keep their factor n^3 (a1 = a_cn / n^3).
-            double part[4] = {0, 0, 0, 0};
-            auto element_fx = [&](int k2, C d) -> C {
-              const int e = at(k2);
-              switch (step) {
-                case PS_SPEC:
-                case PS_ENTER:
-                  ch[e] = d;
-                  return d;
-                case PS_OPEN:
-                  return ch[e];
-                case PS_SMOOTH:
-                  return cmul2(d, A.mulk[e]);
-                case PS_SETUP: {
-                  const C c0 = ch[e];
-                  const R P = pm(k2);
-                  const R br = P * (c0.x + a1 * d.x), bi = P * (c0.y + a1 * d.y);
-                  const C r = cmk<C>((R)2 * a1 * d.x, (R)2 * a1 * d.y);
-                  const C p = cmk<C>(P * r.x, P * r.y);  // the first direction
-                  part[0] = fma(br, br, fma(bi, bi, part[0]));
-                  part[1] = fma(p.x, p.x, fma(p.y, p.y, part[1]));
-                  part[2] = fma(p.x, r.x, fma(p.y, r.y, part[2]));
-                  if (A.cx) {
-                    const C xv = A.cx[e];
-                    part[3] = fma(xv.x, d.x, fma(xv.y, d.y, part[3]));
-                  }
-                  xh[e] = cmk<C>(c0.x * invN, c0.y * invN);
-                  rh[e] = r;
-                  ph[e] = p;
-                  return p;
-                }
-                case PS_UPDATE: {
-                  const C p = ph[e], xv = xh[e], rv = rh[e];
-                  const R P = pm(k2);
-                  const C r = cmk<C>(rv.x - al * (p.x - a1 * d.x), rv.y - al * (p.y - a1 * d.y));
-                  xh[e] = cmk<C>(xv.x + alN * p.x, xv.y + alN * p.y);
-                  rh[e] = r;
-                  const R t = P * (r.x * r.x + r.y * r.y);
-                  part[0] = fma(P, t, part[0]);
-                  part[1] += t;
-                  return d;
-                }
-                case PS_DIR: {
-                  const C rv = rh[e], po = ph[e];
-                  const R P = pm(k2);
-                  const C p = cmk<C>(fma(P, rv.x, bc * po.x), fma(P, rv.y, bc * po.y));
-                  ph[e] = p;
-                  part[0] = fma(p.x, p.x, fma(p.y, p.y, part[0]));
-                  return p;
-                }
-                case PS_LEAVE:
-                  return xh[e];
-                case PS_APPLY:
-                  return cmk<C>(d.x * invN2, d.y * invN2);
-                default: {  // PS_DOT
-                  const C xv = A.cx[e];
-                  part[0] = fma(xv.x, d.x, fma(xv.y, d.y, part[0]));
-                  return d;
-                }
-              }
-            };
-            const Tw* tw = at_tw(k1, twA + k1 * R2);
-            if (nin) fx_leave2<R2>(fx(sl), sl, T, true);
-            if (nin == 2) fx_leave2<R2>(fx(sl + TILE), sl + TILE, T, true);
+          const Tw* tw = at_tw(k1, twA + k1 * R2);
+          if (nin) fx_leave2<R2>(fx(sl), sl, T, true);
+          if (nin == 2) fx_leave2<R2>(fx(sl + TILE), sl + TILE, T, true);
 #pragma unroll 2
-            for (int k2 = 0; k2 < R2; k2++) {
-              C d = sl[k2 * T];
-              if (nin == 2) d = cadd(cimul<C>(wtab[k1 + R1 * k2], d), sl[TILE + k2 * T]);
-              sl[k2 * T] = element_fx(k2, d);
-            }
-#pragma unroll
-            for (int q = 0; q < 4; q++) acc[q].s += mult * part[q];
-            if (nout == 2) fx_enter2<R2, N>(sl, fx(sl + TILE), T, tw, FX_IW, k1, R1);
-            if (nout) fx_enter2<R2, N>(sl, fx(sl), T, tw, 0, 0, 0);
-            continue;
-          } else {
-          C d[R2];
-          if (nin) {
-#pragma unroll
-            for (int b = 0; b < R2; b++) d[b] = sl[b * T];
-            K::template dft<R2, -1>(d);  // x wave number k1 + R1 k2
-          }
-          if (nin == 2) {
-#pragma unroll
-            for (int k2 = 0; k2 < R2; k2++) d[k2] = cimul<C>((R)wavenum(k1 + R1 * k2, N), d[k2]);
-            C y[R2];
-#pragma unroll
-            for (int b = 0; b < R2; b++) y[b] = sl[TILE + b * T];
-            K::template dft<R2, -1>(y);
-#pragma unroll
-            for (int k2 = 0; k2 < R2; k2++) d[k2] = cadd(d[k2], y[k2]);
+          for (int k2 = 0; k2 < R2; k2++) {
+            C d = sl[k2 * T];
+            if (nin == 2) d = cadd(cimul<C>(wtab[k1 + R1 * k2], d), sl[TILE + k2 * T]);
+            sl[k2 * T] = element(k2, d);
           }
 #pragma unroll
-          for (int k2 = 0; k2 < R2; k2++) d[k2] = element(k2, d[k2]);
-          if (nout == 2) {
-            C g[R2];
-#pragma unroll
-            for (int k2 = 0; k2 < R2; k2++) g[k2] = d[k2];
-            K::template dft_iw_tw<R2, +1>(
-                g, [&](int k2) { return wavenum(k1 + R1 * k2, N); },
-                [&](int b) { return twA[k1 * R2 + b]; });
-#pragma unroll
-            for (int b = 0; b < R2; b++) sl[TILE + b * T] = g[b];
-          }
-          if (nout) {
-            K::template dft_tw<R2, +1, false>(d, [&](int b) { return twA[k1 * R2 + b]; });
-#pragma unroll
-            for (int b = 0; b < R2; b++) sl[b * T] = d[b];
-          }
-          }
+          for (int q = 0; q < 4; q++) acc[q] += mult * part[q];
+          if (nout == 2) fx_enter2<R2, N>(sl, fx(sl + TILE), T, tw, FX_IW, k1, R1);
+          if (nout) fx_enter2<R2, N>(sl, fx(sl), T, tw, 0, 0, 0);
+          continue;
         }
         __syncthreads();
         // inverse, second part: rows x = b + R2 a
-        for (int i0 = 0; i0 < (BOTH ? 1 : nout); i0++) {
-          for (int task = tid; task < (BOTH ? nout : 1) * T * R2; task += NT) {
-            const int c = task % T, ib = task / T, i = BOTH ? ib >= R2 : i0;
-            const int b = BOTH ? ib - i * R2 : ib, q = tile * T + c;
-            if (q >= PL) continue;
-            C* dst = Gp + (1 - i) * S + q;  // i = 0: G_0, i = 1: G_x
-            if constexpr (FX) {
-              fx_task1<R1, N>(fx(buf + i * TILE + b * T + c), nullptr, R2 * T, fx(dst + b * PL),
-                              R2 * PL, nullptr, 0, 0, 0, 0);
-            } else {
-            C u[R1];
-#pragma unroll
-            for (int k1 = 0; k1 < R1; k1++) u[k1] = buf[i * TILE + (k1 * R2 + b) * T + c];
-            K::template dft<R1, +1>(u);
-#pragma unroll
-            for (int a = 0; a < R1; a++) dst[(b + R2 * a) * PL] = u[a];
-            }
-          }
+        for (int task = tid; task < nout * T * R2; task += NT) {
+          const int c = task % T, ib = task / T, i = ib >= R2, b = ib - i * R2, q = tile * T + c;
+          if (q >= PL) continue;
+          C* dst = Gp + (1 - i) * S + q;  // i = 0: G_0, i = 1: G_x
+          fx_task1<R1, N>(fx(buf + i * TILE + b * T + c), nullptr, R2 * T, fx(dst + b * PL),
+                          R2 * PL, nullptr, 0, 0, 0, 0);
         }
         if (nout) __syncthreads();
-        if (PI) sums(step, tile);
       }
-      if (!PI) sums(step, blockIdx.x);
+      sums(step);
     }
     if (step == PS_SPEC || (Geo_::SPLIT ? step == PS_LINE && kind == PS_BACK : step == PS_BACK))
       break;
@@ -1244,7 +843,6 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
         step = A.prog == PP_SPEC ? PS_SPEC : A.prog == PP_SMOOTH ? PS_SMOOTH : PS_ENTER;
         break;
       case PS_ENTER:
-      case PS_OPEN:
         step = PS_GRAD;
         break;
       case PS_GRAD:
@@ -1255,33 +853,33 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
         break;
       case PS_SETUP:
         started = true;
-        totals(5, 1, -1);
+        totals(4, 1);
         if (tid == 0) {
-          double snorm = tot[0] * dinvN;
-          cg.dp = tot[1] * dinvN;
+          double snorm = tot[0] * invN;
+          cg.dp = tot[1] * invN;
           if (snorm == 0.0) snorm = cg.dp;
           cg.rnorm0 = snorm;
           cg.ttol = fmax(A.rtol * A.rtol * snorm, A.abstol * A.abstol);
-          cg.beta = tot[2] * dinvN;
-          cg.pp = tot[4];
+          cg.beta = tot[2] * invN;
+          cg.pp = tot[1];
           cg.status = converged(cg.dp);
           if (cg.status == 0 && cg.beta == 0.0) {
             cg.status = 2;
             cg.it = 1;
           }
-          if (A.cx && blockIdx.x == 0) A.sc->acc[6] += A.kdot_weight * tot[3] * dinvN * dscale;
+          if (A.cx && blockIdx.x == 0) A.sc->acc[6] += A.kdot_weight * tot[3] * invN * invN;
           cg.step = cg.status == 0 ? PS_GRAD : PS_LEAVE;
         }
         __syncthreads();
         step = cg.step;
         break;
       case PS_UPDATE:
-        totals(2, 2, -1);
+        totals(2, 2);
         if (tid == 0) {
-          cg.dp = tot[0] * dinvN;
+          cg.dp = tot[0] * invN;
           cg.status = converged(cg.dp);
           if (cg.status == 0) {
-            const double bnew = tot[1] * dinvN;
+            const double bnew = tot[1] * invN;
             cg.beta = bnew;
             cg.bcoef = bnew / cg.beta_old;
             cg.iter++;
@@ -1301,14 +899,13 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
         step = PS_GRAD;
         break;
       case PS_DOT:
-        totals(1, 2, -1);
-        if (blockIdx.x == 0 && tid == 0) A.sc->acc[6] += A.kdot_weight * tot[0] * dinvN * dscale;
+        totals(1, 2);
+        if (blockIdx.x == 0 && tid == 0) A.sc->acc[6] += A.kdot_weight * tot[0] * invN * invN;
         bar.leave();
         return;
       default:  // PS_SMOOTH, PS_LEAVE, PS_APPLY
         step = PS_BACK;
     }
-    if (step == PS_LEAVE && A.prog == PP_SOLVE_SPEC) break;
     if constexpr (Geo_::SPLIT) {
       if (step <= PS_BACK) {
         kind = step;
@@ -1317,7 +914,7 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
     }
   }
   // outcome and sweep statistics
-  if ((A.prog == PP_SOLVE || A.prog == PP_SOLVE_SPEC) && blockIdx.x == 0 && tid == 0) {
+  if (A.prog == PP_SOLVE && blockIdx.x == 0 && tid == 0) {
     DevScalars* s = A.sc;
     s->it = cg.it;
     s->iter = cg.iter;
@@ -1335,11 +932,11 @@ __global__ void __launch_bounds__(PlaneGeo<R, NN>::NT, PlaneGeo<R, NN>::MINB)
   bar.leave();
 }
 
-template <typename R, int N>
+template <int N>
 PlaneKernel plane_entry() {
-  using P = PlaneGeo<R, N>;
-  return PlaneKernel{reinterpret_cast<const void*>(&k_plane<R, N>), P::NT, P::SMEM,
-                     P::ITEMS, P::SPLIT, P::PER_ITEM};
+  using P = PlaneGeo<N>;
+  return PlaneKernel{reinterpret_cast<const void*>(&k_plane<N>), P::NT, P::SMEM, P::ITEMS,
+                     P::SPLIT};
 }
 
 }  // namespace glia

@@ -1,5 +1,5 @@
-// plane.hpp — interface of the persistent plane kernels (plane.cuh), one instantiation per type and
-// grid size, compiled in translation units of their own.
+// plane.hpp — interface of the persistent plane kernels (plane.cuh), one instantiation per grid size,
+// compiled in translation units of their own.
 #pragma once
 
 #include "kernels.cuh"
@@ -8,29 +8,27 @@ namespace glia {
 
 enum PlaneProg {
   PP_SOLVE = 0,  // one Crank-Nicolson solve, in -> out
-  PP_SOLVE_SPEC, // the same on spectra: chat -> xhat (times 1/n^3)
   PP_APPLY,      // D in -> out
   PP_SMOOTH,     // in convolved with mulk -> out
   PP_SPEC,       // spectrum of in -> chat
   PP_DOT         // acc[6] += kdot_weight <cx, D in>
 };
 
-constexpr int kPlanePartials = 6;  // partial-sum slots
+constexpr int kPlanePartials = 5;  // partial-sum slots
 
-template <typename R>
 struct PlaneArgs {
-  using C = typename CT<R>::C;
+  using C = double2;
   int prog, which;
   // field transformed, and what acts on it as it is read: 0 nothing, 1 the logistic step (half
   // receives the field itself when not null), 2 its linearisation at lin
-  const R* in;
+  const double* in;
   int pre;
-  const R* rho;
-  const R* lin;
-  R* half;
-  R dt;
-  R* out;
-  const R* k;
+  const double* rho;
+  const double* lin;
+  double* half;
+  double dt;
+  double* out;
+  const double* k;
   C *chat, *xhat, *rhat, *phat;  // spectrum of in, PCG vectors
   C *G, *M;                      // scratch: [G_x, G_0], [M_x, M_y, M_z]
   C* W;                          // scratch of split kernels: line pairs per component
@@ -39,10 +37,10 @@ struct PlaneArgs {
   double a_cn, pc_c, rtol, abstol, divtol, kdot_weight;
   int maxit;
   DevScalars* sc;
-  double* part;    // kPlanePartials values per CTA or work item
+  double* part;    // kPlanePartials values per CTA
   unsigned* bar;   // two counters, zero between launches
-  const void* tw;  // exp(2 pi i j / n), j < n: float2, or FxTw for double
-  const R* pf;     // double: the preconditioner 1 / (1 + pc_c |w|^2) per spectrum element
+  const void* tw;  // exp(2 pi i j / n), j < n, as FxTw (fx.cuh)
+  const double* pf;  // the preconditioner 1 / (1 + pc_c |w|^2) per spectrum element
 };
 
 struct PlaneKernel {
@@ -50,21 +48,16 @@ struct PlaneKernel {
   int threads, smem;
   int items;       // most work items of a phase
   bool split;      // needs W
-  bool any_grid;   // the result does not depend on the number of CTAs
 };
 // One instantiation per grid size, in translation units by size: every multiple of 8 that factors
 // into R1 <= 16 and R2 = 4, 8 or 16 (plane.cuh). That leaves 136, 152, 168, 184, 200, 216, 232 and
-// 248 (a factor of 17 or more) on cuFFT's transforms and, in float, 240 (its plane does not fit).
-// Time of a solve, cuFFT's transforms / this kernel: double 2.2 to 5.7 at every size; float 1.7 to
-// 1.9 up to 88, 1.4 to 1.6 up to 120, above see plane_f32_large.cu.
-PlaneKernel plane_kernel_f32_small(int n);
-PlaneKernel plane_kernel_f32_large(int n);
+// 248 (a factor of 17 or more) on cuFFT's transforms. Time of a solve with cuFFT's transforms over
+// this kernel's: 2.2 to 5.7 at every size.
 PlaneKernel plane_kernel_f64_small(int n);
 PlaneKernel plane_kernel_f64_mid(int n);
 PlaneKernel plane_kernel_f64_large(int n);
-template <typename R>
-PlaneKernel plane_kernel(int n) {
-  if (sizeof(R) == 4) return n <= 128 ? plane_kernel_f32_small(n) : plane_kernel_f32_large(n);
+void plane_twiddles(int n, int4* out);  // exp(2 pi i j / n), j < n, as FxTw (fx.cuh)
+inline PlaneKernel plane_kernel(int n) {
   return n <= 96    ? plane_kernel_f64_small(n)
          : n <= 144 ? plane_kernel_f64_mid(n)
                     : plane_kernel_f64_large(n);

@@ -5,13 +5,13 @@
 namespace glia {
 PlaneKernel plane_kernel_f64_large(int n) {
   switch (n) {
-    case 160: return plane_entry<double, 160>();
-    case 176: return plane_entry<double, 176>();
-    case 192: return plane_entry<double, 192>();
-    case 208: return plane_entry<double, 208>();
-    case 224: return plane_entry<double, 224>();
-    case 240: return plane_entry<double, 240>();
-    case 256: return plane_entry<double, 256>();
+    case 160: return plane_entry<160>();
+    case 176: return plane_entry<176>();
+    case 192: return plane_entry<192>();
+    case 208: return plane_entry<208>();
+    case 224: return plane_entry<224>();
+    case 240: return plane_entry<240>();
+    case 256: return plane_entry<256>();
     default: return PlaneKernel{};
   }
 }

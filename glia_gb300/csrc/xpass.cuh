@@ -1,5 +1,5 @@
 // xpass.cuh — the x direction of the spectral D apply, fused into the kernels that already stream
-// the spectra (FP32; n = 256 by default, 64, 128 and 256 around 2-D cuFFT transforms).
+// the spectra (FP32, n = 64, 128, 256).
 //
 // A three-dimensional transform is a 2-D transform over (y, z) for every x plus a 1-D transform
 // along x. cuFFT does the (y, z) part as a contiguous batched 2-D transform; these kernels do the
@@ -17,7 +17,6 @@
 // CTA count), so every CTA walks the same number of tiles to within one.
 #pragma once
 
-#include "dft.cuh"
 #include "kernels.cuh"
 
 namespace glia {
@@ -36,6 +35,102 @@ template <>
 struct XDecomp<64> {
   static constexpr int N = 64, R1 = 8, R2 = 8, T = 64;
 };
+
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ float2 cmul2(float2 a, float2 b) {
+  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+
+// In-register DFTs, natural order in and out: X[k] = sum_j v[j] exp(S 2 pi i j k / R) for
+// R = 2, 4, 8, 16, built from radix-4 butterflies (the factors +-i and -1 are sign changes and
+// swaps, never multiplications).
+template <int S>
+__device__ __forceinline__ void dft4(float2& a0, float2& a1, float2& a2, float2& a3) {
+  const float2 t0 = cadd(a0, a2), t1 = csub(a0, a2), t2 = cadd(a1, a3), t3 = csub(a1, a3);
+  a0 = cadd(t0, t2);
+  a2 = csub(t0, t2);
+  a1 = make_float2(t1.x - S * t3.y, t1.y + S * t3.x);  // t1 + S i t3
+  a3 = make_float2(t1.x + S * t3.y, t1.y - S * t3.x);  // t1 - S i t3
+}
+
+// exp(S 2 pi i e / 16) times z for a compile-time e; e = 4 is S i (a swap)
+template <int S, int E>
+__device__ __forceinline__ float2 tw16(float2 z) {
+  constexpr int e = E & 15;
+  if constexpr (e == 0) {
+    return z;
+  } else if constexpr (e == 4) {
+    return make_float2(-S * z.y, S * z.x);
+  } else if constexpr (e == 8) {
+    return make_float2(-z.x, -z.y);
+  } else if constexpr (e == 12) {
+    return make_float2(S * z.y, -S * z.x);
+  } else {
+    constexpr float c[16] = {1.000000000f,  0.923879533f,  0.707106781f,  0.382683432f,
+                             0.000000000f,  -0.382683432f, -0.707106781f, -0.923879533f,
+                             -1.000000000f, -0.923879533f, -0.707106781f, -0.382683432f,
+                             0.000000000f,  0.382683432f,  0.707106781f,  0.923879533f};
+    const float wc = c[e], ws = S * c[(e + 12) & 15];  // sin(2 pi e / 16) = cos(2 pi (e - 4) / 16)
+    return make_float2(z.x * wc - z.y * ws, z.x * ws + z.y * wc);
+  }
+}
+
+template <int R, int S>
+__device__ __forceinline__ void reg_dft(float2 (&v)[R]) {
+  static_assert(R == 2 || R == 4 || R == 8 || R == 16, "register DFT sizes 2 ... 16");
+  if constexpr (R == 2) {
+    const float2 a = v[0];
+    v[0] = cadd(a, v[1]);
+    v[1] = csub(a, v[1]);
+  } else if constexpr (R == 4) {
+    dft4<S>(v[0], v[1], v[2], v[3]);
+  } else if constexpr (R == 8) {
+    // decimation in time: X[k] = E[k] + W^k O[k], X[k + 4] = E[k] - W^k O[k], W = w_16^2
+    float2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6];
+    float2 o0 = v[1], o1 = v[3], o2 = v[5], o3 = v[7];
+    dft4<S>(e0, e1, e2, e3);
+    dft4<S>(o0, o1, o2, o3);
+    o1 = tw16<S, 2>(o1);
+    o2 = tw16<S, 4>(o2);
+    o3 = tw16<S, 6>(o3);
+    v[0] = cadd(e0, o0);
+    v[4] = csub(e0, o0);
+    v[1] = cadd(e1, o1);
+    v[5] = csub(e1, o1);
+    v[2] = cadd(e2, o2);
+    v[6] = csub(e2, o2);
+    v[3] = cadd(e3, o3);
+    v[7] = csub(e3, o3);
+  } else {
+    // 4 x 4: j = 4 j1 + j2; DFT over j1, twiddle w_16^(j2 k1), DFT over j2; k = k1 + 4 k2
+    dft4<S>(v[0], v[4], v[8], v[12]);
+    dft4<S>(v[1], v[5], v[9], v[13]);
+    dft4<S>(v[2], v[6], v[10], v[14]);
+    dft4<S>(v[3], v[7], v[11], v[15]);
+    v[5] = tw16<S, 1>(v[5]);
+    v[6] = tw16<S, 2>(v[6]);
+    v[7] = tw16<S, 3>(v[7]);
+    v[9] = tw16<S, 2>(v[9]);
+    v[10] = tw16<S, 4>(v[10]);
+    v[11] = tw16<S, 6>(v[11]);
+    v[13] = tw16<S, 3>(v[13]);
+    v[14] = tw16<S, 6>(v[14]);
+    v[15] = tw16<S, 9>(v[15]);
+    dft4<S>(v[0], v[1], v[2], v[3]);
+    dft4<S>(v[4], v[5], v[6], v[7]);
+    dft4<S>(v[8], v[9], v[10], v[11]);
+    dft4<S>(v[12], v[13], v[14], v[15]);
+    // v[4 k1 + k2] holds X[k1 + 4 k2]: transpose to natural order
+    float2 t[16];
+#pragma unroll
+    for (int k1 = 0; k1 < 4; k1++)
+#pragma unroll
+      for (int k2 = 0; k2 < 4; k2++) t[k1 + 4 * k2] = v[4 * k1 + k2];
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = t[i];
+  }
+}
 
 // twiddle exp(S 2 pi i e / n) from the shared table W_256^j = exp(-2 pi i j / 256)
 template <int NN, int S>
@@ -152,12 +247,12 @@ __device__ __forceinline__ void xdft(float2* sm, const float2* twb, int c, int g
 // so two x transforms give the three components: G_x = F^-1(i w_x u) / N and
 // G_y, G_z = i w_y, i w_z F^-1(u) / N. The inputs of the CTA's next tile are staged into shared
 // memory (cp.async) while the current tile is transformed.
-// OUT2 (own y / z passes): two arrays out, [G_x, G_0] with G_0 = F^-1(u) / N, and in MODE 1 also
-// sum |p|^2 (DevScalars::pp); otherwise three, [G_x, G_y, G_z].
+// OUT2 (own y / z passes): two arrays out, [G_x, G_0] with G_0 = F^-1(u) / N; otherwise three,
+// [G_x, G_y, G_z].
 template <int NN, int MODE, bool OUT2>
 __global__ void __launch_bounds__(256, 2)
     k_xinv(Geo g, const float* __restrict__ src, float* __restrict__ pdir, float* __restrict__ G3,
-           DevScalars* __restrict__ sc, RedWs ws, const float2* __restrict__ tw_g) {
+           const DevScalars* __restrict__ sc, const float2* __restrict__ tw_g) {
   using D = XDecomp<NN>;
   constexpr int R1 = D::R1, R2 = D::R2, T = D::T, GR = 256 / T;
   constexpr int NB1 = R2 / GR;
@@ -186,13 +281,11 @@ __global__ void __launch_bounds__(256, 2)
     cp_async_commit();
   };
   stage(blockIdx.x);
-  Acc<float> pp;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     cp_async_wait<0>();
     __syncthreads();
     const XCol col = xcol(g, tile * T + c);
     float2 v[NB1][R1];
-    float pl = 0.f;  // the tile's few positive terms, then compensated
 #pragma unroll
     for (int m = 0; m < NB1; m++) {
       const int b = gi + GR * m;
@@ -210,12 +303,10 @@ __global__ void __launch_bounds__(256, 2)
             val.y += bc * po.y;
           }
           P[kx * plane + col.q] = val;
-          if (OUT2) pl = fmaf(val.x, val.x, fmaf(val.y, val.y, pl));
         }
         v[m][a] = val;
       }
     }
-    if (MODE == 1 && OUT2) pp.add(col.mult * pl);
     __syncthreads();  // slots read: stage the next tile behind the transforms
     stage(tile + gridDim.x);
     xdft<D, +1>(
@@ -244,10 +335,6 @@ __global__ void __launch_bounds__(256, 2)
     }
   }
   cp_async_wait<0>();
-  if constexpr (MODE == 1 && OUT2) {
-    double sums[1] = {pp.value()};
-    if (grid_sum_last<1>(sums, ws) && threadIdx.x == 0) sc->pp = sums[0];
-  }
 }
 
 // Epilogue of the forward x pass for one output element (k_spec_div semantics): d = the
@@ -285,14 +372,10 @@ __device__ __forceinline__ void xfwd_finish(Acc<float> (&acc)[4], Geo g, DevScal
     double sums[4] = {acc[0].value(), acc[1].value(), acc[2].value(), acc[3].value()};
     if (!grid_sum_last<4>(sums, ws)) return;
     if (threadIdx.x == 0) div_setup_finish(sums, sc, g.invN, has_cx);
-  } else if constexpr (EPI == EPI_CGU) {
-    double sums[2] = {acc[0].value(), acc[1].value()};
-    if (!grid_sum_last<2>(sums, ws)) return;
-    if (threadIdx.x == 0) cg_update_finish(sums, sc, g.invN);
   } else if constexpr (EPI == EPI_CGW) {
     double sums[1] = {acc[0].value()};
     if (!grid_sum_last<1>(sums, ws)) return;
-    if (threadIdx.x == 0) cg_alpha(sums[0] * g.invN, sc);
+    if (threadIdx.x == 0) div_cgw_finish(sums[0], sc, g.invN);
   }
 }
 
@@ -370,16 +453,10 @@ constexpr int xfwd_own_smem_bytes() {
 }
 
 // Forward x pass of the own-transform path: M = [M_x, M_r] in the half-spectrum layout,
-// divergence i w_x F_x M_x + F_x M_r, and the epilogue: EPI_APPLYD and EPI_SETUP as k_spec_div;
-// EPI_CGU the whole PCG update, w = p - a D p, x' += (alpha / N) p, r -= alpha w, ||z||^2 and
-// <z, r> (aux_in = p, cx = r in and aux_out = r out, out = x'). alpha is known here because the z
-// pass has summed k |grad p|^2 (k_zpass2): w is never stored, and the update needs no pass of its
-// own (7 spectra moved instead of 4 + 6). Measured at 256^3: 98 us instead of 64 + 67; the two sums
-// behind alpha cost the z pass 12 us and the x inverse 8 (one more grid-wide reduction in all, a few
-// microseconds of tail each); a gradient evaluation of 20 steps 196.5 -> 191.8 ms.
-// The CTA's inputs form a stream of items (M_x, M_r and the epilogue's spectra of its first tile,
-// then of the next, ...) through two shared-memory slots: item i sits in slot i % 2 and, once
-// consumed, its slot receives item i + 2 (cp.async). EPI_CGU reads x' straight from global memory.
+// divergence i w_x F_x M_x + F_x M_r, epilogue of k_spec_div. The CTA's inputs form a stream of
+// items (M_x, M_r and the epilogue's spectra of its first tile, then of the next, ...) through
+// two shared-memory slots: item i sits in slot i % 2 and, once consumed, its slot receives item
+// i + 2 (cp.async).
 template <int NN, int EPI>
 __global__ void __launch_bounds__(256, 2)
     k_xfwd_own(Geo g, const float* __restrict__ M2, const float* __restrict__ aux_in,
@@ -393,7 +470,7 @@ __global__ void __launch_bounds__(256, 2)
   float2* slots = reinterpret_cast<float2*>(xfwd_dyn);  // 2 x NN * T
   float2* sm = slots + 2 * NN * T;
   float2* tw = sm + NN * T;
-  if (EPI == EPI_CGU && sc->status != 0) return;
+  if (EPI == EPI_CGW && sc->status != 0) return;
   fill_twb<D, -1>(tw, tw_g);
   const int c = threadIdx.x % T, gi = threadIdx.x / T;
   const int plane = NN * g.nh, Ns = plane * NN;
@@ -401,15 +478,13 @@ __global__ void __launch_bounds__(256, 2)
   const float a = EPI == EPI_APPLYD ? 0.f : (float)sc->a_cn;
   const float pcc = (float)sc->pc_c;
   const float invN = (float)g.invN;
-  const float al = EPI == EPI_CGU ? (float)sc->alpha : 0.f;
-  const float alN = EPI == EPI_CGU ? (float)(sc->alpha * g.invN) : 0.f;
   const float2* Mx = reinterpret_cast<const float2*>(M2);
   const float2* Mr = Mx + Ns;
   const float2* AX = reinterpret_cast<const float2*>(aux_in);
   const float2* CX = reinterpret_cast<const float2*>(cx);
   float2* O = reinterpret_cast<float2*>(out);
   float2* AO = reinterpret_cast<float2*>(aux_out);
-  const int naux = EPI == EPI_APPLYD ? 0 : (EPI == EPI_CGU || (EPI == EPI_SETUP && CX) ? 2 : 1);
+  const int naux = EPI == EPI_APPLYD ? 0 : (EPI == EPI_SETUP && CX ? 2 : 1);
   const int NI = 2 + naux;
   const int mytiles =
       (int)blockIdx.x < ntiles ? (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x
@@ -466,30 +541,11 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
     for (int m2 = 0; m2 < NB2; m2++) {
       const int k1 = gi + GR * m2;
-      constexpr int XH = 8;  // x' values in flight per thread
-      float2 xo[XH];
 #pragma unroll
       for (int k2 = 0; k2 < R2; k2++) {
         const int kx = k1 + R1 * k2;
-        if (EPI == EPI_CGU && k2 % XH == 0) {
-#pragma unroll
-          for (int i = 0; i < XH; i++) xo[i] = O[(kx + R1 * i) * plane + col.q];
-        }
         const float2 av = naux ? SA[kx * T + c] : make_float2(0.f, 0.f);
         const float2 xv = naux == 2 ? SX[kx * T + c] : make_float2(0.f, 0.f);
-        if constexpr (EPI == EPI_CGU) {
-          const float2 d = dsum[m2][k2];
-          const int idx = kx * plane + col.q;
-          const float wr = av.x - a * d.x, wi = av.y - a * d.y;
-          const float2 r = make_float2(xv.x - al * wr, xv.y - al * wi);
-          const float pm = pc_mult<float>(pcc, wavenum(kx, NN), col.wy, col.wz);
-          const float mr2 = col.mult * (r.x * r.x + r.y * r.y);
-          acc[0].add(pm * pm * mr2);
-          acc[1].add(pm * mr2);
-          AO[idx] = r;
-          O[idx] = make_float2(xo[k2 % XH].x + alN * av.x, xo[k2 % XH].y + alN * av.y);
-          continue;
-        }
         xfwd_epilogue<NN, EPI>(dsum[m2][k2], kx, kx * plane + col.q, col, a, pcc, invN, scale, av,
                                xv, naux == 2, O, AO, acc);
       }

@@ -29,6 +29,14 @@ template <>
 struct Z2Decomp<256> {
   static constexpr int R1 = 16, R2 = 16;
 };
+template <>
+struct Z2Decomp<128> {
+  static constexpr int R1 = 16, R2 = 8;
+};
+template <>
+struct Z2Decomp<64> {
+  static constexpr int R1 = 8, R2 = 8;
+};
 
 template <int NN>
 struct Z2Geom {
@@ -152,13 +160,10 @@ __device__ __forceinline__ void pair_line(float2* E0, float2* E1, const float4* 
 // rev: blocks in descending order. The y-inverse pass writes the lines in ascending order and
 // the y-forward pass reads them in ascending order, so in descending order the z pass starts on
 // the lines still in L2 and ends on the ones the y-forward pass reads first.
-// DOT: sums k |grad p|^2 over the grid on the way and, with sum |p|^2 from k_xinv, sets alpha of
-// the PCG step: <p, A p> = sum p^2 + a sum k |grad p|^2, the derivatives being skew-symmetric.
-template <int NN, bool DOT>
+template <int NN>
 __global__ void __launch_bounds__(256, 2)
     k_zpass2(float* __restrict__ Hio, const float* __restrict__ kf,
-             const float2* __restrict__ tw_g, bool rev, DevScalars* __restrict__ sc, RedWs ws,
-             double invN) {
+             const float2* __restrict__ tw_g, bool rev) {
   using Z = Z2Geom<NN>;
   constexpr int R1 = Z::R1, R2 = Z::R2, KPT = Z::KPT, NQ = Z::NQ, LB = Z::LB, LS = Z::LS;
   constexpr int NP = NN * NN * NQ, PS = Z::PS;
@@ -194,7 +199,6 @@ __global__ void __launch_bounds__(256, 2)
   issue(0);
   issue(1);
   issue(2);
-  Acc<float> dot;
   float kv[2][KPT][R2];  // k of lines l0, l1 at t + R2 ii + R1 k2
   for (int b = 0; b < nblk; b++) {
     const int i0 = 4 * b, bi = (int)blockIdx.x + b * (int)gridDim.x;
@@ -239,15 +243,12 @@ __global__ void __launch_bounds__(256, 2)
         }
       }
       float2* OX = Hc + (size_t)(blk * LB + l) * NQ;
-      float dl = 0.f;  // this line's positive terms, then compensated
       float2* OY = OX + NP;
       pair_line<NN>(
           X + sh, Y + sh, twr, t, u,
           [&](int ii, int k2, float2 z) {
             const float kk = kv[j][ii][k2];
-            const float2 s = make_float2(z.x * kk, z.y * kk);
-            if (DOT) dl = fmaf(s.x, z.x, fmaf(s.y, z.y, dl));
-            return s;
+            return make_float2(z.x * kk, z.y * kk);
           },
           [&](int ii, int k2, float2 A, float2 B) {
             const int q = t + R2 * ii + R1 * k2;
@@ -261,7 +262,6 @@ __global__ void __launch_bounds__(256, 2)
             OX[q] = A;
             OY[q] = B;
           });
-      if (DOT) dot.add(dl);
     }
     __syncthreads();
     issue(i0 + 4);
@@ -292,13 +292,10 @@ __global__ void __launch_bounds__(256, 2)
       }
       float2* O0 = Hc + (size_t)2 * NP + (size_t)(blk * LB + l0) * NQ;
       float2* O1 = O0 + NQ;
-      float dl = 0.f;
       pair_line<NN>(
           P0 + sh, P1 + sh, twr, t, u,
           [&](int ii, int k2, float2 z) {
-            const float2 s = make_float2(z.x * kv[0][ii][k2], z.y * kv[1][ii][k2]);
-            if (DOT) dl = fmaf(s.x, z.x, fmaf(s.y, z.y, dl));
-            return s;
+            return make_float2(z.x * kv[0][ii][k2], z.y * kv[1][ii][k2]);
           },
           [&](int ii, int k2, float2 A, float2 B) {
             const int q = t + R2 * ii + R1 * k2;
@@ -306,17 +303,11 @@ __global__ void __launch_bounds__(256, 2)
             O0[q] = make_float2(-w * A.y, w * A.x);
             O1[q] = make_float2(-w * B.y, w * B.x);
           });
-      if (DOT) dot.add(dl);
     }
     __syncthreads();
     issue(i0 + 6);
   }
   cp_async_wait<0>();
-  if constexpr (DOT) {
-    double sums[1] = {dot.value()};
-    if (grid_sum_last<1>(sums, ws) && threadIdx.x == 0)
-      cg_alpha(sc->pp * invN + sc->a_cn * sums[0], sc);
-  }
 }
 
 }  // namespace glia
