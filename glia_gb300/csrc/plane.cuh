@@ -73,7 +73,7 @@ struct PlaneGeo {
   static constexpr int T = SPLIT ? 8 : N > 32 && T4 < 8 ? 8 : T4;
   static constexpr int XT = (PL + T - 1) / T;
   static constexpr int TILE = N * T;
-  static constexpr int RED = 5 * 512 * 8 / (int)sizeof(C);  // partial sums of a phase
+  static constexpr int RED = 4 * 512 * 8 / (int)sizeof(C);  // partial sums of a phase
   static constexpr int LINES = SPLIT ? 16 * PS2 : 0;  // one pair of lines per group of R2 lanes
   static constexpr int BUF0 = 2 * TILE > RED ? 2 * TILE : RED;
   static constexpr int BUF1 = PLANE > LINES ? PLANE : LINES, BUF = BUF0 > BUF1 ? BUF0 : BUF1;
@@ -340,25 +340,6 @@ __device__ __noinline__ double fx_middle2(fx2* row, const double* ka, const doub
   return sum;
 }
 
-enum PlaneStep {
-  PS_FWD = 0,   // planes: real field -> y, z forward
-  PS_GRAD,      // planes: G -> gradient, times k, -> M
-  PS_BACK,      // planes: G_0 -> real field
-  PS_YINV,      // SPLIT: columns of planes, y inverse, G -> W (Z pairs)
-  PS_LINE,      // SPLIT: line pairs in W, z inverse, k, z forward (GRAD; FWD: z forward only;
-                //        BACK: z inverse only)
-  PS_YFWD,      // SPLIT: columns of planes, y forward, W -> M
-  PS_SPEC,      // columns: M_0 -> spectrum (stored)
-  PS_ENTER,     // columns: M_0 -> spectrum (stored) -> G_x, G_0
-  PS_SMOOTH,    // columns: M_0 -> spectrum times mulk -> G_0
-  PS_SETUP,     // columns: M -> D c, solve set-up, first direction -> G_x, G_0
-  PS_UPDATE,    // columns: M -> D p, x and r
-  PS_DIR,       // columns: next direction -> G_x, G_0
-  PS_LEAVE,     // columns: x -> G_0
-  PS_APPLY,     // columns: M -> D u -> G_0
-  PS_DOT        // columns: M -> <cx, D u>
-};
-
 template <int NN>
 __global__ void __launch_bounds__(PlaneGeo<NN>::NT, PlaneGeo<NN>::MINB)
     k_plane(const __grid_constant__ PlaneArgs A) {
@@ -410,27 +391,27 @@ __global__ void __launch_bounds__(PlaneGeo<NN>::NT, PlaneGeo<NN>::MINB)
   C* __restrict__ const ch = A.chat;
   const double* __restrict__ const kf = A.k;
 
-  // partial sums per CTA of slots s0 ... s0 + Q - 1, and their totals after the next barrier
-  // (few FP64 operations: all threads' values go to shared memory and one warp adds each sum)
-  auto partials = [&](const double* v, int q_n, int s0) {
+  // partial sums per CTA, and their totals after the next barrier (plane_steps.hpp; few FP64
+  // operations: all threads' values go to shared memory and one warp adds each sum)
+  auto partials = [&](const double* v, PlaneSlots s) {
     double* all = reinterpret_cast<double*>(buf);
     __syncthreads();
-    for (int q = 0; q < q_n; q++) all[q * NT + tid] = v[q];
+    for (int q = 0; q < s.count; q++) all[q * NT + tid] = v[q];
     __syncthreads();
-    for (int q = warp; q < q_n; q += Geo_::NW) {
+    for (int q = warp; q < s.count; q += Geo_::NW) {
       double x = 0;
 #pragma unroll
       for (int w = 0; w < Geo_::NW; w++) x += all[q * NT + 32 * w + lane];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-      if (lane == 0) A.part[(s0 + q) * (int)gridDim.x + blockIdx.x] = x;
+      if (lane == 0) A.part[(s.first + q) * (int)gridDim.x + blockIdx.x] = x;
     }
   };
-  auto totals = [&](int q_n, int s0) {
-    for (int q = warp; q < q_n; q += Geo_::NW) {
+  auto totals = [&](PlaneSlots s) {
+    for (int q = warp; q < s.count; q += Geo_::NW) {
       double x = 0;
       for (int b = lane; b < (int)gridDim.x; b += 32)
-        x += __ldcg(&A.part[(s0 + q) * (int)gridDim.x + b]);
+        x += __ldcg(&A.part[(s.first + q) * (int)gridDim.x + b]);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
       if (lane == 0) tot[q] = x;
@@ -466,14 +447,14 @@ __global__ void __launch_bounds__(PlaneGeo<NN>::NT, PlaneGeo<NN>::MINB)
   auto at_tw = [](int i, const Tw* tw) { return i ? tw : nullptr; };
   double acc[4];
   auto sums = [&](int kind) {
-    if (kind == PS_GRAD)
-      partials(acc, 1, 1);
-    else if (kind == PS_SETUP)
-      partials(acc, 4, 1);
-    else if (kind == PS_UPDATE || kind == PS_DOT)
-      partials(acc, 2, 2);
-    else if (kind == PS_DIR)
-      partials(acc, 1, 0);
+    switch (kind) {
+      case PS_GRAD: partials(acc, plane_sums(PS_GRAD)); break;
+      case PS_SETUP: partials(acc, plane_sums(PS_SETUP)); break;
+      case PS_UPDATE: partials(acc, plane_sums(PS_UPDATE)); break;
+      case PS_DIR: partials(acc, plane_sums(PS_DIR)); break;
+      case PS_DOT: partials(acc, plane_sums(PS_DOT)); break;
+      default: break;
+    }
   };
   // Row k1 of a line pair in real space (places k2, z = k1 + R1 k2 of lines l0 and l1)
   auto line_middle = [&](int kind, C* row, int64_t l0, int64_t l1, int k1) {
@@ -690,7 +671,7 @@ __global__ void __launch_bounds__(PlaneGeo<NN>::NT, PlaneGeo<NN>::MINB)
                        : step == PS_SPEC || step == PS_UPDATE || step == PS_DOT  ? 0
                                                                                  : 2;
       if (step == PS_UPDATE) {  // alpha
-        totals(2, 0);
+        totals(kPlaneAlphaSums);
         if (tid == 0) {
           if (cg.iter == 0) tot[0] = cg.pp;  // of the set-up's first direction
           cg.dpi_old = cg.dpi;
@@ -853,7 +834,7 @@ __global__ void __launch_bounds__(PlaneGeo<NN>::NT, PlaneGeo<NN>::MINB)
         break;
       case PS_SETUP:
         started = true;
-        totals(4, 1);
+        totals(plane_sums(PS_SETUP));
         if (tid == 0) {
           double snorm = tot[0] * invN;
           cg.dp = tot[1] * invN;
@@ -874,7 +855,7 @@ __global__ void __launch_bounds__(PlaneGeo<NN>::NT, PlaneGeo<NN>::MINB)
         step = cg.step;
         break;
       case PS_UPDATE:
-        totals(2, 2);
+        totals(plane_sums(PS_UPDATE));
         if (tid == 0) {
           cg.dp = tot[0] * invN;
           cg.status = converged(cg.dp);
@@ -899,7 +880,7 @@ __global__ void __launch_bounds__(PlaneGeo<NN>::NT, PlaneGeo<NN>::MINB)
         step = PS_GRAD;
         break;
       case PS_DOT:
-        totals(1, 2);
+        totals(plane_sums(PS_DOT));
         if (blockIdx.x == 0 && tid == 0) A.sc->acc[6] += A.kdot_weight * tot[0] * invN * invN;
         bar.leave();
         return;

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "kernels.cuh"
+#include "plane_steps.hpp"
 
 namespace glia {
 
@@ -13,8 +14,6 @@ enum PlaneProg {
   PP_SPEC,       // spectrum of in -> chat
   PP_DOT         // acc[6] += kdot_weight <cx, D in>
 };
-
-constexpr int kPlanePartials = 5;  // partial-sum slots
 
 struct PlaneArgs {
   using C = double2;
