@@ -440,6 +440,7 @@ int glia_batch_launch(glia_batch* b, void* stream) {
   return batch_guarded(b, [&] {
     if (!b->exec) throw glia::Error(GLIA_ERR_STATE, "no captured batch graph");
     BATCH_CUDA(cudaGraphLaunch(b->exec, stream ? static_cast<cudaStream_t>(stream) : b->root));
+    for (glia_ctx* c : b->ctxs) c->eng->eval_launched();
   });
 }
 

@@ -55,6 +55,7 @@ class EngineBase {
   // graph has run.
   virtual void eval_prepare(const double* x, int nx, const void* d1) = 0;
   virtual void eval_capture() = 0;
+  virtual void eval_launched() = 0;  // the captured graph has been launched (once more)
   virtual void eval_finish(double* J, double* dJ) = 0;
   virtual void* stream() const = 0;
   virtual glia_stats stats() const = 0;

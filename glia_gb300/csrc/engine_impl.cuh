@@ -2123,6 +2123,7 @@ class Engine final : public EngineBase {
     const glia_stats saved = st_;  // capturing runs nothing: the counts come with eval_finish
     capture_ = true;
     cap_solves_ = 0;
+    plane_pc_ = kNoField;  // the graph fills the field itself, whatever solves before a launch do
     try {
       k_solve_stats_reset<<<1, 1, 0, stream_>>>(sc_);
       GLIA_LAUNCH_CHECK();
@@ -2141,10 +2142,12 @@ class Engine final : public EngineBase {
       }
     } catch (...) {
       capture_ = false;
+      plane_pc_ = kNoField;
       st_ = saved;
       throw;
     }
     capture_ = false;
+    plane_pc_ = kNoField;  // recorded, not filled
     cap_total_solves_ = st_.total_diffusion_solves - saved.total_diffusion_solves;
     st_ = saved;
     // nothing has run yet: the history is valid only once a launch of the graph has been read
@@ -2152,6 +2155,7 @@ class Engine final : public EngineBase {
     cap_adjoint_done_ = adjoint_done_;
     state_done_ = adjoint_done_ = false;
   }
+  void eval_launched() override { plane_pc_ = kNoField; }
   void eval_finish(double* J, double* dJ) override {
     if (!cap_ready_) throw Error(GLIA_ERR_STATE, "eval_finish needs a captured evaluation");
     std::vector<double> pp(std::max(phi_np_, 1));
@@ -2610,8 +2614,9 @@ class Engine final : public EngineBase {
   double* plane_part_ = nullptr;
   unsigned* plane_bar_ = nullptr;
   int4* plane_tw_ = nullptr;
-  R* plane_pf_ = nullptr;  // preconditioner field for pc_c = plane_pc_
-  double plane_pc_ = -1;
+  static constexpr double kNoField = -1;
+  R* plane_pf_ = nullptr;        // preconditioner field for pc_c = plane_pc_
+  double plane_pc_ = kNoField;   // a launched graph fills the field for its own
   float2* tw_ = nullptr;
   char* fft_ws_ = nullptr;
   char* batch_ws_ = nullptr;
