@@ -77,23 +77,6 @@ def test_solve_state_and_gradient_match_the_cufft_path(prec, n, monkeypatch):
         assert rel_l2(a, b) < (1e-12 if prec == FP64 else 1e-5)
 
 
-@pytest.mark.parametrize("n", [n for n in SIZES[MIXED] if n <= 128])
-def test_result_does_not_depend_on_the_grid(n):
-    """Float solves keep their sums per work item: the same bits on one or two CTAs per SM
-    and on their share beside the other branches of a captured batch."""
-    out = []
-    for geometry in ((8, 4), (2, 1)):
-        g = gpu(n, MIXED)
-        g.set_launch_geometry(*geometry)
-        g.set_tissue(field(n, 5))
-        g.set_coefficients(k=0.05, rho=1.0)
-        c = field(n, 6)
-        out.append((g.diffusion_solve(c, 0.01), c))
-        g.close()
-    assert out[0][0] == out[1][0]
-    assert np.array_equal(out[0][1], out[1][1])
-
-
 @pytest.mark.parametrize("prec", [FP64, MIXED])
 def test_non_finite_fields_are_reported(prec):
     """A NaN or an infinity in the field stops the solve with an error, as on the other paths."""
