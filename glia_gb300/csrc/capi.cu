@@ -254,6 +254,9 @@ int glia_solve_adjoint(glia_ctx* ctx, int linearized, const void* pt, void* a0) 
 int glia_selftest_bounded_wait(glia_ctx* ctx) {
   return guarded(ctx, [&](glia::EngineBase& e) { e.selftest_bounded_wait(); });
 }
+int glia_selftest_wait_limit(glia_ctx* ctx, int64_t clocks) {
+  return guarded(ctx, [&](glia::EngineBase& e) { e.selftest_wait_limit(clocks); });
+}
 int glia_hessian_matvec(glia_ctx* ctx, const double* x, int nx, double* y) {
   if (!x || !y) return GLIA_ERR_INVALID;
   return guarded(ctx, [&](glia::EngineBase& e) { e.hessian_matvec(x, nx, y); });

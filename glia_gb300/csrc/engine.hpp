@@ -60,6 +60,7 @@ class EngineBase {
   virtual void* stream() const = 0;
   virtual glia_stats stats() const = 0;
   virtual void selftest_bounded_wait() = 0;
+  virtual void selftest_wait_limit(int64_t clocks) = 0;
   virtual void reset_stats() = 0;
   virtual void set_timing(bool on) = 0;
   virtual int timing(int slot, const char** name, int64_t* launches, double* ms,

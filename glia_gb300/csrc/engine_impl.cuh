@@ -367,6 +367,7 @@ class Engine final : public EngineBase {
     a.sc = sc_;
     a.part = plane_part_;
     a.bar = plane_bar_;
+    a.wait = plane_wait_;
     a.tw = plane_tw_;
     a.pf = plane_pf_;
     return a;
@@ -808,6 +809,10 @@ class Engine final : public EngineBase {
       GLIA_CUDA(cudaStreamSynchronize(stream_));
     }
   }
+  void selftest_wait_limit(int64_t clocks) override {
+    if (!plane()) throw Error(GLIA_ERR_INVALID, "selftest_wait_limit: no plane kernel");
+    plane_wait_ = clocks ? clocks : kPlaneWait;
+  }
   // a kernel's bounded wait ran out (its CTA stopped early): the results are invalid
   [[noreturn]] void raise_device_fault() {
     GLIA_CUDA(cudaMemsetAsync(&sc_->dev_fault, 0, sizeof(int), stream_));
@@ -1093,6 +1098,7 @@ class Engine final : public EngineBase {
   void smooth(void* out, const void* in, double sigma) override {
     import_field(in, tmp_);
     smooth_into(tmp_, tmp_, sigma);
+    if (plane()) check_device_fault();
     export_field(tmp_, out);
   }
 
@@ -1930,6 +1936,7 @@ class Engine final : public EngineBase {
         }
         GLIA_CUDA(cudaMemcpyAsync(hsc_, sc_, sizeof(DevScalars), cudaMemcpyDeviceToHost, stream_));
         GLIA_CUDA(cudaStreamSynchronize(stream_));
+        if (hsc_->dev_fault) raise_device_fault();
         std::memcpy(acc, hsc_->acc, sizeof(acc));
       }
       rows[0] = rows[1] = rows[2] = 0.0;
@@ -2613,6 +2620,11 @@ class Engine final : public EngineBase {
   int plane_res_ = 0;
   double* plane_part_ = nullptr;
   unsigned* plane_bar_ = nullptr;
+  // Some 8 s: much longer than a barrier takes (1 us) or the CTAs of a launch differ (a phase, 2 ms
+  // at 256^3), so that other streams' kernels or time slices of other processes, which can hold
+  // some of the CTAs up, are no fault
+  static constexpr long long kPlaneWait = 1LL << 34;
+  long long plane_wait_ = kPlaneWait;
   int4* plane_tw_ = nullptr;
   static constexpr double kNoField = -1;
   R* plane_pf_ = nullptr;        // preconditioner field for pc_c = plane_pc_

@@ -89,10 +89,13 @@ struct PlaneGeo {
 };
 
 // Barrier of all CTAs of a cooperative launch: cnt counts arrivals and is set back to zero by the
-// last CTA that leaves the kernel. The wait is bounded by the SM clock (about one second).
+// last CTA that leaves the kernel. The wait is bounded by the SM clock. A launch whose wait ran out
+// leaves the counters as they are until the host has read the fault and cleared both; launches until
+// then return at once.
 struct GridBarrier {
   unsigned* cnt;
   unsigned target;
+  long long limit;
   __device__ __forceinline__ bool sync(int* fault) {
     __syncthreads();
     bool late = false;
@@ -104,7 +107,7 @@ struct GridBarrier {
       for (;;) {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(cnt) : "memory");
         if ((int)(v - target) >= 0) break;
-        if (clock64() - t0 > (1LL << 31)) {
+        if (clock64() - t0 > limit) {
           late = true;
           atomicExch(fault, 2);
           break;
@@ -363,6 +366,7 @@ __global__ void __launch_bounds__(PlaneGeo<NN>::NT, PlaneGeo<NN>::MINB)
   double* wtab = reinterpret_cast<double*>(zin + N);  // wave numbers
   __shared__ double tot[4];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (__syncthreads_or(tid == 0 && A.sc->dev_fault)) return;  // the counters are not zero
   for (int i = tid; i < N; i += NT) {
     const int k1 = i / R2, b = i - k1 * R2;
     twA[i] = reinterpret_cast<const Tw*>(A.tw)[b * k1];  // b k1 < N
@@ -372,7 +376,7 @@ __global__ void __launch_bounds__(PlaneGeo<NN>::NT, PlaneGeo<NN>::MINB)
   const double invN = 1.0 / ((double)N * N * N);
   // the spectra sent to the planes keep their factor n^3
   const double a1 = A.a_cn * invN, invN2 = invN * invN;
-  GridBarrier bar{A.bar, 0};
+  GridBarrier bar{A.bar, 0, A.wait};
   // PCG scalars, the same in every CTA (thread 0 updates them)
   __shared__ struct {
     double beta, beta_old, dpi, dpi_old, alpha, bcoef;

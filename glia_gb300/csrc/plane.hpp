@@ -38,6 +38,7 @@ struct PlaneArgs {
   DevScalars* sc;
   double* part;    // kPlanePartials values per CTA
   unsigned* bar;   // two counters, zero between launches
+  long long wait;  // longest wait at a grid barrier, in SM clocks
   const void* tw;  // exp(2 pi i j / n), j < n, as FxTw (fx.cuh)
   const double* pf;  // the preconditioner 1 / (1 + pc_c |w|^2) per spectrum element
 };

@@ -309,6 +309,12 @@ int glia_mismatch_f32_noalloc(const float* c, const float* obs, const float* d, 
  * context still runs kernels afterwards, GLIA_ERR_CUDA otherwise. FP32 contexts only. */
 int glia_selftest_bounded_wait(glia_ctx* ctx);
 
+/* Diagnostic (extension; no counterpart in the reference): sets the time limit of the grid barriers
+ * inside a context's FP64 solve kernels, in SM cycles (0: the default, 2^34). With a negative limit
+ * every wait runs out at once and the context's calls return GLIA_ERR_CUDA; after the default is
+ * set again they give right results. FP64 contexts whose grid size has such a kernel only. */
+int glia_selftest_wait_limit(glia_ctx* ctx, int64_t clocks);
+
 #ifdef __cplusplus
 }
 #endif

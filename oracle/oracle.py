@@ -39,6 +39,7 @@ def load() -> _abi.Bound:
         _api = _abi.Bound(lib, "oracle_glia_", optional=("set_timing", "get_timing", "mismatch_f32_noalloc",
                                                        "set_launch_geometry",
                                                        "selftest_bounded_wait",
+                                                       "selftest_wait_limit",
                                                        *_abi.BATCH_NAMES))
         for name, res, args in (
             ("oracle_fft_r2c", ctypes.c_int, [ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]),
