@@ -275,6 +275,11 @@ class Engine final : public EngineBase {
     k_assemble<R><<<red_blocks_, kThreads, 0, stream_>>>(N_, rho_, wm_, gm_, csf_, dwm, dgm,
                                                           dglm, sc_, 1, ws_);
     GLIA_LAUNCH_CHECK();
+    if (plane()) {
+      k_max<R><<<red_blocks_, kThreads, 0, stream_>>>(N_, rho_, ws_.partials, 1, sc_, ws_.counter);
+      GLIA_LAUNCH_CHECK();
+      rho_max_ = read_red(1);
+    }
   }
   void set_coefficients(double k, double kgm, double kglm, double rho, double rgm,
                         double rglm) override {
@@ -349,6 +354,12 @@ class Engine final : public EngineBase {
   // Arguments and launch of the grid's plane kernel (plane.cuh), all CTAs resident at once.
   static constexpr bool kPlane = std::is_same<R, double>::value;
   bool plane() const { return plane_.fn != nullptr; }
+  // Whether this context's work takes the plane kernel. Rounding in tumour-free tissue grows like
+  // exp(rho T) over a simulation, and its gradient feels it most: against cuFFT's transforms the
+  // plane kernel moves FP64 gradients by 2e-13 of their norm at rho T = 5, 3e-11 at 10, 2e-10 at 10.5,
+  // 4e-9 at 12 and 3e-8 at 14 (largest of 28 to 56 problems each, 16^3 to 96^3, 32^3 mostly; states by
+  // a hundredth of that). FP64 results may move by 1e-9, so cuFFT's transforms stay beyond 10.5.
+  bool plane_now() const { return plane() && rho_max_ * dt_ * nt_ <= kPlaneGrowth; }
   static double2* cx2(R* p) { return reinterpret_cast<double2*>(p); }
   static const double2* cx2(const R* p) { return reinterpret_cast<const double2*>(p); }
   PlaneArgs plane_args(int prog, const R* in, R* out, R* chat) {
@@ -382,7 +393,7 @@ class Engine final : public EngineBase {
   // spectrum of a real field
   void spectrum(const R* in, R* out) {
     if constexpr (kPlane) {
-      if (plane()) {
+      if (plane_now()) {
         PlaneArgs a = plane_args(PP_SPEC, in, nullptr, out);
         plane_launch(a, FB() + SB());
         st_.total_fft_execs += 1;
@@ -419,7 +430,7 @@ class Engine final : public EngineBase {
 
   void fused_solve(R* c, double dts, R* chat, const R* cx, double kdot_w, int which, Pre pre) {
     if constexpr (kPlane) {
-      if (plane()) {
+      if (plane_now()) {
         plane_solve(c, dts, chat, cx, kdot_w, which, pre);
         return;
       }
@@ -1006,7 +1017,7 @@ class Engine final : public EngineBase {
       return;
     }
     if constexpr (kPlane) {
-      if (plane()) {
+      if (plane_now()) {
         PlaneArgs a = plane_args(PP_APPLY, c, dc, chat_);
         plane_launch(a, 3 * FB());
         st_.total_fft_execs += 2;
@@ -1082,7 +1093,7 @@ class Engine final : public EngineBase {
     }
     const R* K = smoother_kernel(sigma);
     if constexpr (kPlane) {
-      if (plane()) {
+      if (plane_now()) {
         PlaneArgs a = plane_args(PP_SMOOTH, in, out, chat_);
         a.mulk = cx2(K);
         plane_launch(a, 2 * FB() + SB());
@@ -1552,7 +1563,7 @@ class Engine final : public EngineBase {
   // half; 2: linearised at lin): a plane kernel takes it as it reads the field of the next solve,
   // otherwise it runs here.
   Pre react(R* c, int mode, const R* lin, R* half) {
-    if (plane() && k_scale_ != 0) return Pre{mode, lin, half};
+    if (plane_now() && k_scale_ != 0) return Pre{mode, lin, half};
     if (mode == 1)
       reaction(c, half);
     else
@@ -1826,7 +1837,7 @@ class Engine final : public EngineBase {
   // acc[6] += w <c_0, D alpha_0>: a D apply on alpha_0 whose spectral epilogue takes the dot
   void kappa_dot_at(const R* chat0, double w) {
     if constexpr (kPlane) {
-      if (plane()) {
+      if (plane_now()) {
         PlaneArgs a = plane_args(PP_DOT, p0_, nullptr, xhat_);
         a.cx = cx2(chat0);
         a.kdot_weight = w;
@@ -2626,6 +2637,8 @@ class Engine final : public EngineBase {
   static constexpr long long kPlaneWait = 1LL << 34;
   long long plane_wait_ = kPlaneWait;
   int4* plane_tw_ = nullptr;
+  static constexpr double kPlaneGrowth = 10.5;
+  double rho_max_ = 0;
   static constexpr double kNoField = -1;
   R* plane_pf_ = nullptr;        // preconditioner field for pc_c = plane_pc_
   double plane_pc_ = kNoField;   // a launched graph fills the field for its own
