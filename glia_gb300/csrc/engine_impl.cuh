@@ -425,7 +425,7 @@ class Engine final : public EngineBase {
     a.kdot_weight = kdot_w;
     plane_launch(a, 3 * FB());  // c in and out, k
     graph_solves_ = true;
-    st_.total_fft_execs += 2;
+    st_.total_fft_execs += 8;  // there, the set-up's D apply, back
   }
 
   void fused_solve(R* c, double dts, R* chat, const R* cx, double kdot_w, int which, Pre pre) {
@@ -1020,7 +1020,7 @@ class Engine final : public EngineBase {
       if (plane_now()) {
         PlaneArgs a = plane_args(PP_APPLY, c, dc, chat_);
         plane_launch(a, 3 * FB());
-        st_.total_fft_execs += 2;
+        st_.total_fft_execs += 8;
         return;
       }
     }
@@ -1842,7 +1842,7 @@ class Engine final : public EngineBase {
         a.cx = cx2(chat0);
         a.kdot_weight = w;
         plane_launch(a, 2 * FB() + SB());
-        st_.total_fft_execs += 1;
+        st_.total_fft_execs += 7;
         return;
       }
     }
