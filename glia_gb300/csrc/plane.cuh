@@ -22,8 +22,8 @@
 // FP64 only. Arithmetic is the bound there, see fx.cuh; a barrier costs 1.0 us. As separate launches
 // a solve took 7 kernels and a conditional graph node an iteration, and cuFFT's transforms ran at the
 // FP64 units' rate. Measured on GB300, before -> after:
-//   forward   64^3, 100 steps   150 -> 45 ms      gradient 128^3, 6 steps   164 -> 32 ms
-//   adjoint  120^3, 2 steps    48.7 -> 10.5 ms    solve    256^3           46 -> 10.3 ms
+//   forward   64^3, 100 steps   151 -> 45.1 ms    gradient 128^3, 6 steps   164 -> 32.3 ms
+//   adjoint  120^3, 2 steps    48.7 -> 10.5 ms    solve    256^3           53.0 -> 11.4 ms
 //
 // N = R1 R2 (R2 a power of two, so that a group of R2 threads is part of a warp). Inverse
 // transforms read index R2 a + b (R1-point DFTs over a, twiddle w^(b k1), R2-point DFTs over b) and

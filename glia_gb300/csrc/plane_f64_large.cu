@@ -1,5 +1,5 @@
 // Plane kernels of the FP64 engine above 144^3: split, no plane fits in shared memory. A solve at 256^3
-// takes 10.3 ms against 45 with cuFFT transforms, which run at the FP64 units' rate.
+// takes 11.4 ms against 53 with cuFFT transforms, which run at the FP64 units' rate.
 #include "plane.cuh"
 
 namespace glia {
