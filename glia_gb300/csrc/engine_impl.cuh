@@ -7,6 +7,7 @@
 //    half spectra; z = P r is never formed; the operator apply is 6 transforms
 //    (1 batched C2R of the three gradient spectra, 1 batched R2C of k * grad) plus 4 fused
 //    passes; the set-up reuses one D apply for both the right-hand side and r0.
+//    FP64 grids with a plane kernel (plane.cuh) run all of a solve as one launch.
 //  - reference-structured (GLIA_ENGINE_REFERENCE): a restatement of the reference's GPU
 //    structure with our own kernels: real-space PCG, 10 transforms per D apply, one kernel per
 //    PETSc vector operation and a host round trip per inner product. It is the plain baseline.
@@ -1086,6 +1087,11 @@ class Engine final : public EngineBase {
     wkern_sigma_ = sigma;
     return wkern_;
   }
+  // The smoother by the plane kernel: from 64^3. It is one launch, but the call then has to look for
+  // a timed-out barrier, which waits for it, so small calls no longer follow each other without a
+  // gap. us a call, cuFFT / plane: 16^3 56 / 55, 32^3 76 / 68, 56^3 79 / 93 (one small case among
+  // others 41 / 69), 64^3 109 / 80, 96^3 242 / 130, 256^3 3693 / 1061.
+  bool plane_smooth() const { return plane_now() && g_.n >= 64; }
   void smooth_into(R* out, const R* in, double sigma) {
     if (sigma == 0) {
       if (out != in) vcopy(out, in);
@@ -1093,7 +1099,7 @@ class Engine final : public EngineBase {
     }
     const R* K = smoother_kernel(sigma);
     if constexpr (kPlane) {
-      if (plane_now()) {
+      if (plane_smooth()) {
         PlaneArgs a = plane_args(PP_SMOOTH, in, out, chat_);
         a.mulk = cx2(K);
         plane_launch(a, 2 * FB() + SB());
@@ -1109,7 +1115,7 @@ class Engine final : public EngineBase {
   void smooth(void* out, const void* in, double sigma) override {
     import_field(in, tmp_);
     smooth_into(tmp_, tmp_, sigma);
-    if (plane()) check_device_fault();
+    if (plane_smooth()) check_device_fault();
     export_field(tmp_, out);
   }
 

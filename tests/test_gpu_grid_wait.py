@@ -13,7 +13,7 @@ from tests.helpers import reference_test_field
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [32, 160])  # planes in shared memory, y and z phases of their own
+@pytest.mark.parametrize("n", [64, 160])  # planes in shared memory, y and z phases of their own
 def test_a_wait_that_runs_out_is_reported_by_every_call(n):
     wl, tissue, centers = small_problem(n, 2, n_gauss=4)
     g = gpu(n, FP64)
