@@ -28,3 +28,12 @@ def test_solve_and_smoother(n, monkeypatch):
         g.close()
     assert out[0][0] == out[1][0]
     assert rel_l2(out[0][1], out[1][1]) < 1e-12 and rel_l2(out[0][2], out[1][2]) < 1e-12
+
+
+@pytest.mark.parametrize("n,plane", [(56, 0), (64, 1), (256, 1)])
+def test_smoother_runs_on_the_plane_kernel_from_64(n, plane):
+    g = gpu(n, FP64)
+    g.set_timing(True)
+    g.smooth(np.random.default_rng(n).random(n ** 3), 0.3)
+    assert g.timing().get("k_plane", (0,))[0] == plane
+    g.close()
